@@ -968,12 +968,14 @@ private:
         // boundary (the PCISPH boundary model moves predicted positions after
         // the prediction), indices below 2^27
         cands_ = (d.simulation_method == SPH_PCISPH || d.simulation_method == SPH_WCSPH) && d.neighbor_list_max > 0 &&
-                 G_ == 1 && !bh_ && n < (size_t)kCandIdxMask;
+                 G_ == 1 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask;
         if (cands_) {
             ckmax_ = (uint32_t)d.neighbor_list_max;
             SPH_CUDA(cand_.alloc((size_t)ckmax_ * n));
             SPH_CUDA(candn_.alloc(n));
+            SPH_CUDA(candb_.alloc(n));
             SPH_CUDA(cudaMemsetAsync(candn_.p, 0, n * sizeof(uint32_t), st_));
+            SPH_CUDA(cudaMemsetAsync(candb_.p, 0, n * sizeof(uint32_t), st_));
         }
         SPH_CUDA(pairs_.alloc(lists_ ? (size_t)kmax_ * n : 1));
         SPH_CUDA(lcount_.alloc(lists_ ? n : 1));
@@ -1091,8 +1093,10 @@ private:
     {
         Fluid<R> f = F();
         const R reach = c_.h + cand_margin();
+        // never below the passes' own cull, which has some slack over h
+        const R reach2 = std::max(reach * reach, c_.cull2);
         run("k_density_cand", [&] { k_density_cand<R, EOS><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(
-            f, bd_[1].pos, gv_, starts_.p, bstarts_.p, c_, akinci_, reach * reach, cand_.p, candn_.p, ckmax_); });
+            f, bd_[1].pos, gv_, starts_.p, bstarts_.p, c_, akinci_, reach2, cand_.p, candn_.p, candb_.p, ckmax_); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1675,13 +1679,14 @@ private:
     uint32_t kmax_ = 0;
     bool cands_ = false;            // PCISPH candidate lists (CandLists)
     uint32_t ckmax_ = 0;
-    DevBuf<uint32_t> cand_, candn_;
+    DevBuf<uint32_t> cand_, candn_, candb_;
     CandLists CL() const
     {
-        return cands_ ? CandLists{cand_.p, candn_.p, ckmax_, &sc_.p->status} : CandLists{nullptr, nullptr, 0u, nullptr};
+        return cands_ ? CandLists{cand_.p, candn_.p, candb_.p, ckmax_, nb_, &sc_.p->status} : CandLists{};
     }
     // the lists' reach beyond h: predicted displacements up to half of it keep them exact
-    R cand_margin() const { return (R)0.1 * c_.h; }
+    // (WCSPH visits them at the current positions only)
+    R cand_margin() const { return d.simulation_method == SPH_PCISPH ? (R)0.1 * c_.h : (R)0; }
     DevBuf<DevScalars> sc_;
 };
 
