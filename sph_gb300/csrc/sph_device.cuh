@@ -436,7 +436,9 @@ template <typename R> __device__ __forceinline__ R adhesion_W(const Consts<R>& c
 }
 
 // ---------------------------------------------------------------------------
-// Block reductions in FP64 with a deterministic last-block finish.
+// Block reductions with a deterministic last-block finish: sums in FP64, maxima
+// in the type of their values (exact either way; this part has two FP64 lanes
+// per SM).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -444,27 +446,35 @@ __device__ __forceinline__ double warp_sum(double v)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_max(double v)
+template <typename T> __device__ __forceinline__ T max_of(T a, T b)
+{
+    if constexpr (sizeof(T) == 8) return fmax(a, b);
+    else return fmaxf(a, b);
+}
+template <typename T> __device__ __forceinline__ T warp_max(T v)
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
+    for (int o = 16; o > 0; o >>= 1) v = max_of(v, (T)__shfl_down_sync(0xffffffffu, v, o));
     return v;
 }
+template <typename T> __device__ __forceinline__ T max_identity() { return sizeof(T) == 8 ? (T)-1.0e300 : (T)-1.0e38f; }
 
-// Sum (or max) of v over the block; the result is valid in thread 0.
-template <bool MAX> __device__ __forceinline__ double block_reduce(double v, double* sh)
+// Sum (or max) of v over the block; the result is valid in every thread.
+template <bool MAX, typename T> __device__ __forceinline__ T block_reduce(T v, T* sh)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    v = MAX ? warp_max(v) : warp_sum(v);
+    if constexpr (MAX) v = warp_max(v);
+    else v = warp_sum(v);
     if (lane == 0) sh[wid] = v;
     __syncthreads();
     if (wid == 0) {
-        double t = lane < nw ? sh[lane] : (MAX ? -1.0e300 : 0.0);
-        t = MAX ? warp_max(t) : warp_sum(t);
+        T t = lane < nw ? sh[lane] : (MAX ? max_identity<T>() : (T)0);
+        if constexpr (MAX) t = warp_max(t);
+        else t = warp_sum(t);
         if (lane == 0) sh[0] = t;
     }
     __syncthreads();
-    const double r = sh[0];
+    const T r = sh[0];
     __syncthreads();
     return r;
 }
@@ -473,14 +483,14 @@ template <bool MAX> __device__ __forceinline__ double block_reduce(double v, dou
 // last to finish), in which every thread sees the total in *total_out.  The
 // total is summed in block-index order, so the result does not depend on
 // which block finished last.
-template <bool MAX>
-__device__ __forceinline__ bool finish_reduction(double v, double* partials, unsigned* counter, double* sh,
-                                                 double* total_out)
+template <bool MAX, typename T>
+__device__ __forceinline__ bool finish_reduction(T v, double* partials, unsigned* counter, T* sh, T* total_out)
 {
-    const double b = block_reduce<MAX>(v, sh);
+    static_assert(MAX || sizeof(T) == 8, "sums in FP64");
+    const T b = block_reduce<MAX>(v, sh);
     __shared__ bool is_last;
     if (threadIdx.x == 0) {
-        partials[blockIdx.x] = b;
+        partials[blockIdx.x] = (double)b;
         __threadfence();
         const unsigned done = atomicAdd(counter, 1u);
         is_last = (done == gridDim.x - 1);
@@ -488,12 +498,13 @@ __device__ __forceinline__ bool finish_reduction(double v, double* partials, uns
     __syncthreads();
     if (!is_last) return false;
     __threadfence();
-    double t = MAX ? -1.0e300 : 0.0;
+    T t = MAX ? max_identity<T>() : (T)0;
     for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
-        const double p = *((volatile double*)(partials + i));
-        t = MAX ? fmax(t, p) : t + p;
+        const T p = (T) * ((volatile double*)(partials + i));
+        if constexpr (MAX) t = max_of(t, p);
+        else t = t + p;
     }
-    const double tot = block_reduce<MAX>(t, sh);
+    const T tot = block_reduce<MAX>(t, sh);
     if (threadIdx.x == 0) *counter = 0u;
     *total_out = tot;
     return true;

@@ -14,6 +14,8 @@
 
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 namespace sph {
 
 template <typename R> struct Fluid {
@@ -557,15 +559,24 @@ __device__ __forceinline__ void walk_reach(const GridView& g, const uint32_t* __
 // left a pass waiting for two dependent loads per candidate.  81k PCISPH drop:
 // predicted-density pass 31 -> 19 us, pressure accelerations 29 -> 16 us.
 // nj: length of the array j indexes.
+//
+// `shift` (FP32, shared memory): the offset of each cell offset code, so that
+// s costs one 16-byte load and three subtractions instead of decoding the
+// code (x - 0, x - h, x + h are each one rounding either way).
 template <typename R> constexpr int kListBatch = sizeof(R) == 4 ? 4 : 2;
+constexpr int kShiftCodes = 27;
+__device__ __forceinline__ void fill_shift_table(float4* t, float h)
+{
+    for (int c = threadIdx.x; c < kShiftCodes; c += blockDim.x)
+        t[c] = make_float4((float)(c / 9 - 1) * h, (float)((c / 3) % 3 - 1) * h, (float)(c % 3 - 1) * h, 0.f);
+    __syncthreads();
+}
 
-template <typename R, typename Load, typename Eval>
+template <typename R, int B, typename Load, typename Eval>
 __device__ __forceinline__ void list_visit(const CandLists& L, uint32_t n, uint32_t i, uint32_t first, uint32_t cnt,
-                                           uint32_t nj, V3<R> xi, R h, Load&& load, Eval&& eval)
+                                           uint32_t nj, V3<R> xi, const float4* shift, Load&& load, Eval&& eval)
 {
     constexpr bool REL = sizeof(R) == 4;
-    constexpr int B = kListBatch<R>;
-    const R szm = xi.z + h, sz0 = xi.z, szp = xi.z - h;
     const uint32_t* __restrict__ p = L.idx + (size_t)first * n + i;
 #pragma unroll 1
     for (uint32_t k = 0; k < cnt; k += B) {
@@ -588,33 +599,56 @@ __device__ __forceinline__ void list_visit(const CandLists& L, uint32_t n, uint3
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             if (!ok[b]) continue;
-            const uint32_t code = e[b] >> kCandIdxBits;
-            const int dx = (int)(code / 9) - 1, dy = (int)((code / 3) % 3) - 1, dz = (int)(code % 3) - 1;
-            const V3<R> s = REL ? V3<R>{xi.x - (R)dx * h, xi.y - (R)dy * h, dz < 0 ? szm : (dz == 0 ? sz0 : szp)} : xi;
-            eval(q[b], s, e[b] & kCandIdxMask);
+            V3<R> s = xi;
+            if constexpr (REL) {
+                const float4 d = shift[e[b] >> kCandIdxBits];
+                s = V3<R>{xi.x - d.x, xi.y - d.y, xi.z - d.z};
+            }
+            eval(q[b], s);
         }
     }
 }
 
-// Fluid candidates of particle i at lane LANE of G: the list (G = 1 and a
-// stored list) or the cell walk.
-template <typename R, int G, bool TRIM = true, typename Load, typename Eval>
+// The cell walk of a particle that has no list, out of line and one column at
+// a time: its registers are not carried by the list loop (64 -> 48 in the
+// predicted-density pass; 490k drop: 108 -> 89 us with the shift table).
+template <typename R, bool TRIM, typename Acc, typename Load, typename Eval>
+__device__ __noinline__ Acc walk_out_of_line(const GridView& g, const uint32_t* __restrict__ starts, uint32_t pc, V3<R> xi,
+                                             R h, Acc acc, Load load, Eval eval)
+{
+    walk<R, 1, TRIM, true>(g, starts, pc, xi, h, 0, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
+    return acc;
+}
+
+// Fluid candidates of particle i at lane LANE of G, summed into acc by
+// eval(acc, load(j), s): LISTS (G = 1): the stored list, or the walk out of
+// line where it did not fit; else the cell walk.
+template <typename R, int G, bool LISTS, int B, bool TRIM = true, typename Acc, typename Load, typename Eval>
 __device__ __forceinline__ void fluid_visit(const CandLists& L, uint32_t n, uint32_t i, const GridView& g,
                                             const uint32_t* __restrict__ cs, uint32_t pc, V3<R> xi, R h, int lane,
-                                            Load&& load, Eval&& eval)
+                                            const float4* shift, Acc& acc, Load load, Eval eval)
 {
-    if (G == 1 && L.has(i)) list_visit<R>(L, n, i, 0u, L.cnt[i], n, xi, h, load, eval);
-    else walk<R, G, TRIM>(g, cs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(load(j), s, j); });
+    if constexpr (LISTS) {
+        if (L.has(i)) list_visit<R, B>(L, n, i, 0u, L.cnt[i], n, xi, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
+        else acc = walk_out_of_line<R, TRIM>(g, cs, pc, xi, h, acc, load, eval);
+    } else {
+        walk<R, G, TRIM>(g, cs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
+    }
 }
 
 // Boundary candidates likewise: listed after the fluid ones, or the walk.
-template <typename R, int G, typename Load, typename Eval>
+template <typename R, int G, bool LISTS, int B, typename Acc, typename Load, typename Eval>
 __device__ __forceinline__ void boundary_visit(const CandLists& L, uint32_t n, uint32_t i, const GridView& g,
                                                const uint32_t* __restrict__ bs, uint32_t pc, V3<R> xi, R h, int lane,
-                                               Load&& load, Eval&& eval)
+                                               const float4* shift, Acc& acc, Load load, Eval eval)
 {
-    if (G == 1 && L.has_boundary(i)) list_visit<R>(L, n, i, L.cnt[i], L.bcnt[i], L.nb, xi, h, load, eval);
-    else walk<R, G>(g, bs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(load(j), s, j); });
+    if constexpr (LISTS) {
+        if (L.has_boundary(i))
+            list_visit<R, B>(L, n, i, L.cnt[i], L.bcnt[i], L.nb, xi, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
+        else acc = walk_out_of_line<R, true>(g, bs, pc, xi, h, acc, load, eval);
+    } else {
+        walk<R, G>(g, bs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
+    }
 }
 
 // Densities (SPHSolver::computeFluidDensities SPHSolver.cpp:44-91, as
@@ -738,13 +772,22 @@ __global__ void __launch_bounds__(kBlock) k_density(Fluid<R> f, const P4<R>* __r
     }
 }
 
+// A boundary candidate's loads in the pressure walks: the point with its
+// weight, and (PCISPH boundary model) p_b / rho_b^2.
+template <typename R> struct BoundaryLoad {
+    P4<R> p;
+    R dp;
+};
+
 // WCSPHSolver::computePressureForce WCSPHSolver.cpp:132-188 (xk.w = p/rho^2)
-template <typename R, int G>
+template <typename R, int G, bool LISTS>
 __global__ void __launch_bounds__(kBlock) k_wcsph_pressure_force(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                  Consts<R> c, int akinci, const R* __restrict__ bdp,
-                                                                 CandLists L = CandLists{})
+                                                                 CandLists L)
 {
+    __shared__ float4 shift[LISTS ? kShiftCodes : 1];
+    if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
@@ -755,23 +798,25 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_pressure_force(Fluid<R> f, con
         const V3<R> xi = xyz(pi);
         const R dpi = pi.w;
         const uint32_t pc = f.cell[i];
-        fluid_visit<R, G>(
-            L, f.n, i, g, cs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(f.xk + j); },
-            [&](const P4<R>& pj, V3<R> s, uint32_t) {
+        fluid_visit<R, G, LISTS, kListBatch<R>>(
+            L, f.n, i, g, cs, pc, xi, c.h, lane, shift, sum, [=](uint32_t j) { return ldg4(f.xk + j); },
+            [=](V3<R>& a, const P4<R>& pj, V3<R> s) {
                 const V3<R> r = s - xyz(pj);
                 const R r2 = dot3(r, r);
-                if (r2 <= c.cull2) sum = sum - (c.mass * (dpi + pj.w)) * cubic_gradW(c, r, r2);
+                if (r2 <= c.cull2) a = a - (c.mass * (dpi + pj.w)) * cubic_gradW(c, r, r2);
             });
         if (akinci)
-            boundary_visit<R, G>(L, f.n, i, g, bs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(bpos + j); },
-                                 [&](const P4<R>& pb, V3<R> s, uint32_t j) {
-                const V3<R> r = s - xyz(pb);
-                const R r2 = dot3(r, r);
+            boundary_visit<R, G, LISTS, kListBatch<R>>(
+                L, f.n, i, g, bs, pc, xi, c.h, lane, shift, sum,
                 // Akinci: rho0 psi_b (p_i / rho_i^2); PCISPH model: m_b (p_i / rho_i^2 + p_b / rho_b^2)
                 // (WCSPHSolver.cpp:162-186)
-                const R q = bdp ? dpi + bdp[j] : dpi * (R)1;
-                if (r2 <= c.cull2) sum = sum - (pb.w * q) * cubic_gradW(c, r, r2);
-            });
+                [=](uint32_t j) { return BoundaryLoad<R>{ldg4(bpos + j), bdp ? bdp[j] : (R)0}; },
+                [=](V3<R>& a, const BoundaryLoad<R>& b, V3<R> s) {
+                    const V3<R> r = s - xyz(b.p);
+                    const R r2 = dot3(r, r);
+                    const R q = bdp ? dpi + b.dp : dpi * (R)1;
+                    if (r2 <= c.cull2) a = a - (b.p.w * q) * cubic_gradW(c, r, r2);
+                });
     }
     if (G > 1) sum = group_sum3<G>(sum);
     if (!valid || lane != 0) return;
@@ -782,36 +827,47 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_pressure_force(Fluid<R> f, con
 
 // SurfaceTensionAkinci::step, normal pass SurfaceTensionAkinci.h:43-61: this
 // lane's part of particle i's sum (the caller adds the lanes and scales by h).
-template <typename R, int G>
+template <typename R> struct PosDens {
+    P4<R> x;
+    R rho;
+    uint32_t j;
+};
+
+template <typename R, int G, bool LISTS = false>
 __device__ __forceinline__ V3<R> st_normal_sum(uint32_t i, int lane, const Fluid<R>& f, const GridView& g,
                                                const uint32_t* __restrict__ cs, const Consts<R>& c,
-                                               const CandLists& L = CandLists{})
+                                               const CandLists& L = CandLists{}, const float4* shift = nullptr)
 {
     V3<R> ni = {0, 0, 0};
     const V3<R> xi = xyz(f.pos[i]);
-    fluid_visit<R, G>(
-        L, f.n, i, g, cs, f.cell[i], xi, c.h, lane, [&](uint32_t j) { return ldg4(f.pos + j); },
-        [&](const P4<R>& pj, V3<R> s, uint32_t j) {
-            const V3<R> r = s - xyz(pj);
+    const P4<R>*pos = f.pos, *vel = f.vel;
+    // (a walk visits many candidates beyond h: their densities are not loaded)
+    fluid_visit<R, G, LISTS, kListBatch<R>>(
+        L, f.n, i, g, cs, f.cell[i], xi, c.h, lane, shift, ni,
+        [=](uint32_t j) { return PosDens<R>{ldg4(pos + j), LISTS ? ldg1(&vel[j].w) : (R)0, j}; },
+        [=](V3<R>& a, const PosDens<R>& q, V3<R> s) {
+            const V3<R> r = s - xyz(q.x);
             const R r2 = dot3(r, r);
             if (r2 <= c.cull2) {
-                const R vol = c.mass / ldg4(f.vel + j).w;
-                ni = ni + vol * cubic_gradW(c, r, r2);
+                const R vol = c.mass / (LISTS ? q.rho : ldg4(vel + q.j).w);
+                a = a + vol * cubic_gradW(c, r, r2);
             }
         });
     return ni;
 }
 
-template <typename R, int G>
+template <typename R, int G, bool LISTS>
 __global__ void __launch_bounds__(kBlock) k_st_normals(Fluid<R> f, GridView g, const uint32_t* __restrict__ cs, Consts<R> c,
-                                                       CandLists L = CandLists{})
+                                                       CandLists L)
 {
+    __shared__ float4 shift[LISTS ? kShiftCodes : 1];
+    if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
     const bool valid = i < f.count();
     V3<R> ni = {0, 0, 0};
-    if (valid) ni = st_normal_sum<R, G>(i, lane, f, g, cs, c, L);
+    if (valid) ni = st_normal_sum<R, G, LISTS>(i, lane, f, g, cs, c, L, shift);
     if (G > 1) ni = group_sum3<G>(ni);
     if (!valid || lane != 0) return;
     ni = ni * ((R)1 * c.h);
@@ -829,16 +885,23 @@ __global__ void __launch_bounds__(kBlock) k_st_normals(Fluid<R> f, GridView g, c
 template <typename R> struct NPForces {
     V3<R> av, avb, ast, aad;
 };
+template <typename R> struct PosVelIdx {
+    P4<R> x, v;
+    uint32_t j;
+};
+template <typename R> struct NPFluid { V3<R> av, ast; };
+template <typename R> struct NPBoundary { V3<R> avb, aad; };
 
-template <typename R, int G>
+template <typename R, int G, bool LISTS = false>
 __device__ __forceinline__ NPForces<R> npforce_sums(uint32_t i, int lane, const Fluid<R>& f,
                                                     const P4<R>* __restrict__ bpos, const GridView& g,
                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                     const Consts<R>& c, int akinci, R dt,
-                                                    const CandLists& L = CandLists{})
+                                                    const CandLists& L = CandLists{}, const float4* shift = nullptr)
 {
     const int fl = c.force_flags;
-    V3<R> av = {0, 0, 0}, avb = {0, 0, 0}, ast = {0, 0, 0}, aad = {0, 0, 0};
+    NPFluid<R> sf = {{0, 0, 0}, {0, 0, 0}};
+    NPBoundary<R> sb = {{0, 0, 0}, {0, 0, 0}};
     const V3<R> xi = xyz(f.pos[i]);
     const P4<R> vi4 = f.vel[i];
     const V3<R> vi = xyz(vi4);
@@ -847,61 +910,65 @@ __device__ __forceinline__ NPForces<R> npforce_sums(uint32_t i, int lane, const 
     if (fl & F_SURFACE_TENSION) ni = xyz(f.normal[i]);
     const uint32_t pc = f.cell[i];
     const R h2 = c.h * c.h;
+    const P4<R>*pos = f.pos, *vel = f.vel, *normal = f.normal;
     if (fl & (F_XSPH | F_STD_VISC | F_ART_VISC | F_SURFACE_TENSION))
-        fluid_visit<R, G>(L, f.n, i, g, cs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(f.pos + j); },
-                          [&](const P4<R>& pj, V3<R> s, uint32_t j) {
-            const V3<R> r = s - xyz(pj);
+        fluid_visit<R, G, LISTS, kListBatch<R>>(
+            L, f.n, i, g, cs, pc, xi, c.h, lane, shift, sf,
+            [=](uint32_t j) { return PosVelIdx<R>{ldg4(pos + j), LISTS ? ldg4(vel + j) : P4<R>{0, 0, 0, 0}, j}; },
+            [=](NPFluid<R>& a, const PosVelIdx<R>& q, V3<R> s) {
+            const V3<R> r = s - xyz(q.x);
             const R r2 = dot3(r, r);
             if (!(r2 <= c.cull2)) return;
-            const P4<R> vj4 = ldg4(f.vel + j);
+            const P4<R> vj4 = LISTS ? q.v : ldg4(vel + q.j);
             const V3<R> vj = xyz(vj4);
             const R rho_j = vj4.w;
             const R rl = sqrt(r2);
             if (fl & F_XSPH)
-                av = av + (((c.visc * (c.mass / rho_j)) * (vj - vi)) * cubic_W(c, rl)) / dt;
+                a.av = a.av + (((c.visc * (c.mass / rho_j)) * (vj - vi)) * cubic_W(c, rl)) / dt;
             if (fl & F_STD_VISC)
-                av = av + ((c.mass * (vj - vi)) / rho_j) * visc_laplW(c, r2);
+                a.av = a.av + ((c.mass * (vj - vi)) / rho_j) * visc_laplW(c, r2);
             if (fl & F_ART_VISC) {
                 const R dotProd = dot3(vi - vj, r);
                 const R sqDist = rl * rl;
                 const R kij = (R)2 * c.density0 / (rho_i + rho_j);
-                av = av + (kij * (R)10 * (R)0.1 * c.visc * (c.mass / rho_j) * dotProd / (sqDist + (R)0.01 * h2)) *
-                              cubic_gradW(c, r, r2);
+                a.av = a.av + (kij * (R)10 * (R)0.1 * c.visc * (c.mass / rho_j) * dotProd / (sqDist + (R)0.01 * h2)) *
+                                  cubic_gradW(c, r, r2);
             }
             if (fl & F_SURFACE_TENSION) {
                 if (rl > (R)0 && rl <= c.h) {
-                    const V3<R> nj = xyz(ldg4(f.normal + j));
+                    const V3<R> nj = xyz(ldg4(normal + q.j));
                     const R kij = (R)2 * c.density0 / (rho_i + rho_j);
                     const V3<R> coh = ((-c.mass * cohesion_W(c, rl)) * r) / rl;
                     const V3<R> curv = (R)-1 * (ni - nj);
-                    ast = ast + (c.st * kij) * (coh + curv);
+                    a.ast = a.ast + (c.st * kij) * (coh + curv);
                 }
             }
         });
     const bool bvisc = (fl & F_BVISC) && akinci;
     if ((fl & F_ADHESION) || bvisc)
-        boundary_visit<R, G>(L, f.n, i, g, bs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(bpos + j); },
-                             [&](const P4<R>& pb, V3<R> s, uint32_t) {
+        boundary_visit<R, G, LISTS, kListBatch<R>>(
+            L, f.n, i, g, bs, pc, xi, c.h, lane, shift, sb, [=](uint32_t j) { return ldg4(bpos + j); },
+            [=](NPBoundary<R>& a, const P4<R>& pb, V3<R> s) {
             const V3<R> r = s - xyz(pb);
             const R r2 = dot3(r, r);
             if (!(r2 <= c.cull2)) return;
             const R rl = sqrt(r2);
             if (bvisc) {
                 if (fl & F_XSPH)
-                    avb = avb + (((c.bvisc * (pb.w / rho_i)) * (-vi)) * cubic_W(c, rl)) / dt;
+                    a.avb = a.avb + (((c.bvisc * (pb.w / rho_i)) * (-vi)) * cubic_W(c, rl)) / dt;
                 if (fl & F_STD_VISC)
-                    avb = avb + ((pb.w * (-vi)) / rho_i) * visc_laplW(c, r2);
+                    a.avb = a.avb + ((pb.w * (-vi)) / rho_i) * visc_laplW(c, r2);
                 if (fl & F_ART_VISC) {
                     const R dotProd = dot3(vi, r);
                     const R sqDist = rl * rl;
-                    avb = avb + ((R)10 * (R)0.1 * c.bvisc * (pb.w / rho_i) * dotProd / (sqDist + (R)0.01 * h2)) *
-                                    cubic_gradW(c, r, r2);
+                    a.avb = a.avb + ((R)10 * (R)0.1 * c.bvisc * (pb.w / rho_i) * dotProd / (sqDist + (R)0.01 * h2)) *
+                                        cubic_gradW(c, r, r2);
                 }
             }
             if ((fl & F_ADHESION) && rl > (R)0)
-                aad = aad - ((c.adh * pb.w * adhesion_W(c, rl)) * r) / rl;
+                a.aad = a.aad - ((c.adh * pb.w * adhesion_W(c, rl)) * r) / rl;
         });
-    return NPForces<R>{av, avb, ast, aad};
+    return NPForces<R>{sf.av, sb.avb, sf.ast, sb.aad};
 }
 
 // The forces added to particle i's acceleration in the reference's plugin
@@ -925,18 +992,20 @@ __device__ __forceinline__ void npforce_apply(uint32_t i, const Fluid<R>& f, con
 }
 
 // Non-pressure forces in one walk (npforce_sums), lanes added, then applied.
-template <typename R, int G>
+template <typename R, int G, bool LISTS>
 __global__ void __launch_bounds__(kBlock) k_npforce(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                     Consts<R> c, int akinci, const DevScalars* __restrict__ scr,
-                                                    CandLists L = CandLists{})
+                                                    CandLists L)
 {
+    __shared__ float4 shift[LISTS ? kShiftCodes : 1];
+    if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
     const bool valid = i < f.count();
     NPForces<R> s = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    if (valid) s = npforce_sums<R, G>(i, lane, f, bpos, g, cs, bs, c, akinci, (R)scr->dt, L);
+    if (valid) s = npforce_sums<R, G, LISTS>(i, lane, f, bpos, g, cs, bs, c, akinci, (R)scr->dt, L, shift);
     if (G > 1) {
         s.av = group_sum3<G>(s.av); s.avb = group_sum3<G>(s.avb); s.ast = group_sum3<G>(s.ast); s.aad = group_sum3<G>(s.aad);
     }
@@ -955,18 +1024,18 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_dfsph_cfl(Fluid<R> f, Consts<R> c, DevScalars* sc, LoopLimits lim,
                                                    double* partials)
 {
-    __shared__ double sh[33];
+    __shared__ R sh[33];
     const uint32_t i = gtid();
     const R dt = (R)sc->dt;
-    double m = 0.1;
+    R m = 0;
     if (i < f.count()) {
         const P4<R> v = f.vel[i], a = f.acc[i];
         const V3<R> cur = {v.x + (a.x + c.gx) * dt, v.y + (a.y + c.gy) * dt, v.z + (a.z + c.gz) * dt};
-        m = fmax(m, (double)sqrt(sqrt(dot3(cur, cur))));
+        m = max_of(m, (R)sqrt(sqrt(dot3(cur, cur))));
     }
-    double maxVel;
-    if (finish_reduction<true>(m, partials, &sc->block_counter, sh, &maxVel) && threadIdx.x == 0) {
-        maxVel = fmax(maxVel, 0.1);
+    R mr;
+    if (finish_reduction<true>(m, partials, &sc->block_counter, sh, &mr) && threadIdx.x == 0) {
+        const double maxVel = fmax((double)mr, 0.1);
         const double ts = sc->dt;
         const double cflTs = lim.cflFactor * 0.4 * 2.0 * lim.particleRadius / maxVel;
         double newTs;
@@ -1338,44 +1407,45 @@ __global__ void k_pcisph_predict(Fluid<R> f, Consts<R> c, DevScalars* __restrict
 // positions, cells of the current positions) fused with
 // PCISPHSolver::updatePressure PCISPHSolver.cpp:249-295 (max reduction) and
 // the p/rho^2 hand-off to the pressure-acceleration walk.
-template <typename R, int G>
+template <typename R, int G, bool LISTS>
 __global__ void __launch_bounds__(kBlock) k_pcisph_density_pressure(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                     Consts<R> c, int akinci, DevScalars* sc, LoopLimits lim,
-                                                                    double* partials,
-                                                                    CandLists L = CandLists{},
-                                                                    float margin = 0.f)
+                                                                    double* partials, CandLists L, float margin)
 {
-    __shared__ double sh[33];
+    __shared__ R sh[33];
+    __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (!sc->active) return;
+    if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
     const bool valid = i < f.count();
     // the lists hold every candidate that can come within h while each
     // predicted displacement stays below margin / 2 (10 % slack for rounding)
-    if (L.idx && !(2.f * __uint_as_float(sc->disp_bits) <= 0.9f * margin)) L.idx = nullptr;
+    if (LISTS && !(2.f * __uint_as_float(sc->disp_bits) <= 0.9f * margin)) L.idx = nullptr;
     R density = 0;
     if (valid) {
         const V3<R> xi = xyz(f.predR[i]);
         const uint32_t pc = f.cell[i];
-        fluid_visit<R, G, false>(
-            L, f.n, i, g, cs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(f.predR + j); },
-            [&](const P4<R>& pj, V3<R> s, uint32_t) {
+        fluid_visit<R, G, LISTS, kListBatch<R>, false>(
+            L, f.n, i, g, cs, pc, xi, c.h, lane, shift, density, [=](uint32_t j) { return ldg4(f.predR + j); },
+            [=](R& a, const P4<R>& pj, V3<R> s) {
                 const V3<R> r = s - xyz(pj);
                 const R r2 = dot3(r, r);
-                if (r2 <= c.cull2) density += c.mass * cubic_W(c, sqrt(r2));
+                if (r2 <= c.cull2) a += c.mass * cubic_W(c, sqrt(r2));
             });
         if (akinci)
-            boundary_visit<R, G>(L, f.n, i, g, bs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(bpos + j); },
-                                 [&](const P4<R>& pb, V3<R> s, uint32_t) {
-                const V3<R> r = s - xyz(pb);
-                const R r2 = dot3(r, r);
-                if (r2 <= c.cull2) density += pb.w * cubic_W(c, sqrt(r2));
-            });
+            boundary_visit<R, G, LISTS, kListBatch<R>>(
+                L, f.n, i, g, bs, pc, xi, c.h, lane, shift, density, [=](uint32_t j) { return ldg4(bpos + j); },
+                [=](R& a, const P4<R>& pb, V3<R> s) {
+                    const V3<R> r = s - xyz(pb);
+                    const R r2 = dot3(r, r);
+                    if (r2 <= c.cull2) a += pb.w * cubic_W(c, sqrt(r2));
+                });
     }
     if (G > 1) density = group_sum<G>(density);
-    double err = 0.0;
+    R err = 0;
     if (valid && lane == 0) {
         f.rho[i] = density;
         f.vel[i].w = density;
@@ -1384,11 +1454,12 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_density_pressure(Fluid<R> f, 
         f.press[i] = p;
         const P4<R> x = f.pos[i];
         f.xk[i] = P4<R>{x.x, x.y, x.z, p / (density * density)};
-        err = (double)(e / c.density0);
+        err = e / c.density0;
     }
-    double mx;
-    if (finish_reduction<true>(err, partials, &sc->block_counter, sh, &mx) && threadIdx.x == 0) {
-        mx = fmax(mx, 0.0);
+    // a maximum of FP32 values needs no FP64 (2 FP64 lanes per SM and cycle)
+    R mr;
+    if (finish_reduction<true>(err, partials, &sc->block_counter, sh, &mr) && threadIdx.x == 0) {
+        const double mx = fmax((double)mr, 0.0);
         sc->maxDensityError = mx;
         if (!isfinite(mx)) sc->status |= ST_NONFINITE;
         const unsigned it = sc->iterations + 1;
@@ -1398,14 +1469,15 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_density_pressure(Fluid<R> f, 
 
 // PCISPHSolver::computePressureAcc PCISPHSolver.cpp:297-358 (Spiky gradient,
 // current positions; xk.w = p/rho^2)
-template <typename R, int G>
+template <typename R, int G, bool LISTS>
 __global__ void __launch_bounds__(kBlock) k_pcisph_pressure_acc(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                 const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                 Consts<R> c, int akinci, const DevScalars* __restrict__ sc,
-                                                                const R* __restrict__ bdp,
-                                                                CandLists L = CandLists{})
+                                                                const R* __restrict__ bdp, CandLists L)
 {
+    __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (!sc->active) return;
+    if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
@@ -1416,22 +1488,24 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_pressure_acc(Fluid<R> f, cons
         const V3<R> xi = xyz(pi);
         const R dpi = pi.w;
         const uint32_t pc = f.cell[i];
-        fluid_visit<R, G>(
-            L, f.n, i, g, cs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(f.xk + j); },
-            [&](const P4<R>& pj, V3<R> s, uint32_t) {
+        fluid_visit<R, G, LISTS, kListBatch<R>>(
+            L, f.n, i, g, cs, pc, xi, c.h, lane, shift, pacc, [=](uint32_t j) { return ldg4(f.xk + j); },
+            [=](V3<R>& a, const P4<R>& pj, V3<R> s) {
                 const V3<R> r = s - xyz(pj);
                 const R r2 = dot3(r, r);
-                if (r2 <= c.cull2) pacc = pacc - (c.mass * (dpi + pj.w)) * spiky_gradW(c, r, r2);
+                if (r2 <= c.cull2) a = a - (c.mass * (dpi + pj.w)) * spiky_gradW(c, r, r2);
             });
         if (akinci)
-            boundary_visit<R, G>(L, f.n, i, g, bs, pc, xi, c.h, lane, [&](uint32_t j) { return ldg4(bpos + j); },
-                                 [&](const P4<R>& pb, V3<R> s, uint32_t j) {
-                const V3<R> r = s - xyz(pb);
-                const R r2 = dot3(r, r);
+            boundary_visit<R, G, LISTS, kListBatch<R>>(
+                L, f.n, i, g, bs, pc, xi, c.h, lane, shift, pacc,
                 // PCISPHSolver.cpp:332-356, as the WCSPH force
-                const R q = bdp ? dpi + bdp[j] : dpi;
-                if (r2 <= c.cull2) pacc = pacc - (pb.w * q) * spiky_gradW(c, r, r2);
-            });
+                [=](uint32_t j) { return BoundaryLoad<R>{ldg4(bpos + j), bdp ? bdp[j] : (R)0}; },
+                [=](V3<R>& a, const BoundaryLoad<R>& b, V3<R> s) {
+                    const V3<R> r = s - xyz(b.p);
+                    const R r2 = dot3(r, r);
+                    const R q = bdp ? dpi + b.dp : dpi;
+                    if (r2 <= c.cull2) a = a - (b.p.w * q) * spiky_gradW(c, r, r2);
+                });
     }
     if (G > 1) pacc = group_sum3<G>(pacc);
     if (!valid || lane != 0) return;

@@ -1069,6 +1069,12 @@ private:
             default: fn(std::integral_constant<int, 1>{}); break;
         }
     }
+    // the same for the passes that can visit candidate lists (one lane): fn(G, lists)
+    template <typename Fn> void withGL(Fn&& fn)
+    {
+        if (cands_) fn(std::integral_constant<int, 1>{}, std::true_type{});
+        else withG([&](auto gt) { fn(gt, std::false_type{}); });
+    }
     unsigned wblocks() const { return blocks((size_t)n_ * G_, kBlock); }
 
     int launch_density(bool alpha, bool eos)
@@ -1297,12 +1303,13 @@ private:
         if (!c_.force_flags) return SPH_OK;
         Fluid<R> f = F();
         const P4<R>* bp = bd_[1].pos;
-        withG([&](auto gt) {
+        withGL([&](auto gt, auto lt) {
             constexpr int G = decltype(gt)::value;
+            constexpr bool LISTS = decltype(lt)::value;
             const CandLists L = CL();
             if (c_.force_flags & F_SURFACE_TENSION)
-                run("k_st_normals", [&] { k_st_normals<R, G><<<wblocks(), kBlock, 0, ls_>>>(f, gv_, starts_.p, c_, L); });
-            run("k_npforce", [&] { k_npforce<R, G><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
+                run("k_st_normals", [&] { k_st_normals<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, gv_, starts_.p, c_, L); });
+            run("k_npforce", [&] { k_npforce<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
         });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1490,9 +1497,10 @@ private:
         const R* dp = bdp();
         {
             auto ph = phase("Pressure force");
-            withG([&](auto gt) {
+            withGL([&](auto gt, auto lt) {
                 constexpr int G = decltype(gt)::value;
-                run("k_wcsph_pressure_force", [&] { k_wcsph_pressure_force<R, G><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, dp, CL()); });
+                constexpr bool LISTS = decltype(lt)::value;
+                run("k_wcsph_pressure_force", [&] { k_wcsph_pressure_force<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, dp, CL()); });
             });
             SPH_CUDA(cudaGetLastError());
         }
@@ -1557,14 +1565,15 @@ private:
                     if (bh_)  // correctPredPositions PCISPHSolver.cpp:367-377
                         run("k_bh_collide", [&] { k_bh_collide<R, 2><<<blocks(n_, 128), 128, 0, ls_>>>(f, B(1), gv_, bstarts_.p, c_, sc_.p,
                                                                                                   cell_epoch_.p); });
-                    withG([&](auto gt) {
+                    withGL([&](auto gt, auto lt) {
                         constexpr int G = decltype(gt)::value;
+                        constexpr bool LISTS = decltype(lt)::value;
                         const CandLists L = CL();
                         const float margin = (float)cand_margin();
-                        run("k_pcisph_density_pressure", [&] { k_pcisph_density_pressure<R, G><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_,
+                        run("k_pcisph_density_pressure", [&] { k_pcisph_density_pressure<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_,
                                                                                        hasb_, sc_.p, lim_, partials_.p, L, margin); });
                         launch_bh_boundary(2);
-                        run("k_pcisph_pressure_acc", [&] { k_pcisph_pressure_acc<R, G><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
+                        run("k_pcisph_pressure_acc", [&] { k_pcisph_pressure_acc<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
                                                                                    sc_.p, dp, L); });
                     });
                     run("k_pcisph_loop_next", [&] { k_pcisph_loop_next<<<1, 1, 0, ls_>>>(sc_.p, lim_, h); });
