@@ -409,16 +409,45 @@ __device__ __forceinline__ uint32_t final_slot(uint32_t p, const uint32_t* __res
     return s + rank;
 }
 
+// Half-precision copy of cell-relative positions, two points (2k, 2k+1) per
+// 16-byte word: {x pair, y pair, z pair, unused} as half2, z in the cell's
+// modulo-3 frame.
+__device__ __forceinline__ void store_half(uint4* __restrict__ posh, uint32_t d, float x, float y, float zf)
+{
+    __half* ph = reinterpret_cast<__half*>(posh) + (size_t)(d >> 1) * 8 + (d & 1);
+    ph[0] = __float2half_rn(x);
+    ph[2] = __float2half_rn(y);
+    ph[4] = __float2half_rn(zf);
+}
+// the same from a stored point (FP32: cell-relative; FP64: absolute)
+template <typename R>
+__device__ __forceinline__ void store_half_abs(uint4* __restrict__ posh, uint32_t d, const P4<R>& p, uint32_t c,
+                                               const GridView& g, double h)
+{
+    V3<float> o = {(float)p.x, (float)p.y, (float)p.z};
+    if constexpr (sizeof(R) == 8)
+        o = {(float)(p.x - (double)(cell_x(c) + g.ox) * h), (float)(p.y - (double)(cell_y(c) + g.oy) * h),
+             (float)(p.z - (double)(cell_z(c) + g.oz) * h)};
+    store_half(posh, d, o.x, o.y, zframe3(o.z, cell_z(c), (float)h));
+}
+
+// The boundary points' half-precision copy (they do not move: written once
+// per grid box).
+template <typename R>
+__global__ void k_boundary_half(Boundary<R> b, GridView g, double h, uint4* __restrict__ posh)
+{
+    const uint32_t d = gtid();
+    if (d < b.n) store_half_abs(posh, d, b.pos[d], b.cell[d], g, h);
+}
+
 // Gather of the state that survives a re-sort (x, v, DFSPH k, kv and the
 // last predicted density; the other fields are recomputed after every build).
-// posh (FP32, optional): also the half-precision copy of the positions the
-// list build culls with, two particles (2k, 2k+1) per 16-byte word:
-// {x pair, y pair, z pair, unused} as half2, z in the cell's modulo-3 frame
-// (position.w, written by the cell update).
+// posh (optional): also the half-precision copy of the positions the list
+// build culls with.
 template <typename R>
 __global__ void k_gather_fluid(uint32_t n, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ key,
                                const uint32_t* __restrict__ starts, Fluid<R> src, Fluid<R> dst,
-                               uint4* __restrict__ posh = nullptr)
+                               uint4* __restrict__ posh = nullptr, GridView g = GridView{}, double h = 0.0)
 {
     const uint32_t p = gtid();
     if (p >= src.count()) return;
@@ -426,13 +455,10 @@ __global__ void k_gather_fluid(uint32_t n, const uint32_t* __restrict__ tmp, con
     const uint32_t d = final_slot(p, tmp, key, src.id, starts, &i);
     const P4<R> x = src.pos[i];
     dst.pos[d] = x;
-    if constexpr (sizeof(R) == 4) {
-        if (posh) {
-            __half* ph = reinterpret_cast<__half*>(posh) + (size_t)(d >> 1) * 8 + (d & 1);
-            ph[0] = __float2half_rn(x.x);
-            ph[2] = __float2half_rn(x.y);
-            ph[4] = __float2half_rn(x.w);
-        }
+    if (posh) {
+        // (FP32: the cell update left z in the modulo-3 frame in w)
+        if constexpr (sizeof(R) == 4) store_half(posh, d, x.x, x.y, x.w);
+        else store_half_abs(posh, d, x, src.cell[i], g, h);
     }
     dst.vel[d] = src.vel[i];
     dst.kappa[d] = src.kappa[i];

@@ -36,8 +36,8 @@ template <typename R> struct Lists {
     P4<R>* bgrad;       // xyz: sum_b rho0 psi_b gradW_ib
     R* kbuf;            // k (or kv) of the pass in progress
     uint32_t kmax;
-    // FP32 form: a half-precision copy of the cell-relative positions for
-    // the build's cull, two particles per 16-byte word ({x, y, z, unused}
+    // A half-precision copy of the cell-relative positions for the build's
+    // cull, two particles per 16-byte word ({x, y, z, unused}
     // half2 pairs, z in the cell's modulo-3 frame), or nullptr
     const uint4* posh;
     unsigned* fault;    // status word of the bounds-checked build (SPH_INDEX_OK)
@@ -47,7 +47,7 @@ template <typename R> struct Lists {
     const uint32_t* bcell;
 };
 
-// Phase 1 of the FP32 list build from the half-precision positions: the
+// Phase 1 of the list build from the half-precision positions: the
 // nine columns of the 27-cell neighbourhood (trimmed as walk() trims them),
 // two candidates per half2 operation, accepted indices queued in walk order.
 // The caller guarantees that the particle's cell is at least two cells from
@@ -214,6 +214,15 @@ __device__ __noinline__ BuildSums<R> build_walk_all(uint32_t i, const Fluid<R>& 
     return b;
 }
 
+// The dot product of the velocity divergence terms with its rounding written
+// out (FP32: the contraction the compiler chose for the pass over the lists
+// first), so that the sum the build forms and the passes' agree bit for bit.
+template <typename R> __device__ __forceinline__ R dot3_div(V3<R> a, V3<R> b)
+{
+    if constexpr (sizeof(R) == 8) return dot3(a, b);
+    else return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+
 // Forward declarations: the list build's DIV0 form ends with the velocity
 // divergence the first divergence-error pass would compute from the lists.
 template <typename R> struct DivSum;
@@ -231,17 +240,21 @@ __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint3
         const P4<R> pr = L.pairs[(size_t)k * n + i];
         const uint32_t j = as_idx(pr.w);
         if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-        dv += dot3(vi - xyz(f.vel[j]), xyz(pr));
+        dv += dot3_div(vi - xyz(f.vel[j]), xyz(pr));
     }
     return dv;
 }
 
+// EB: queued candidates evaluated per round, their loads in flight together.
+// The one-scene build has one wave of blocks or less up to ~130k particles and
+// waits for its loads (EB = 4); the pool's is bound by issue slots (EB = 1).
+//
 // DIV0: also sum m (v_i - v_j) . gradW_ij over the pairs as they are listed,
 // plus v_i . (boundary gradient): the value velocity_div_one would read from
 // the finished lists (same terms, same order), into *div0, with the count of
 // neighbours into *nn0 (a particle whose list or queue overflowed takes the
 // same list or cell walk as velocity_div_one).
-template <typename R, bool FAST = false, bool DIV0 = false>
+template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1>
 __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                                 const GridView& g, const uint32_t* __restrict__ cs,
                                                 const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
@@ -276,21 +289,25 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             }
             if (cnt < L.kmax) L.pairs[(size_t)cnt * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j)};
             ++cnt;
-            if constexpr (DIV0) dv += dot3(vi - vj, mg);
+            if constexpr (DIV0) dv += dot3_div(vi - vj, mg);
         }
     };
     // phase 1: cull.  The half-precision cull needs all 27 cells inside the
     // grid box and clear of its border cells (where particles that left the
     // box are kept, with unbounded offsets), and in-cell offsets; elsewhere
-    // the cull runs in FP32.
+    // the cull runs in R.
     uint32_t nq = 0;
     bool half_cull = false;
-    if constexpr (FAST && sizeof(R) == 4) {
-        const R hh = (R)0.5 * c.h;
+    V3<float> xr;  // the position in its cell's frame
+    {
         const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
+        if constexpr (sizeof(R) == 4) xr = xi;
+        else xr = V3<float>{(float)(xi.x - (R)(cx + g.ox) * c.h), (float)(xi.y - (R)(cy + g.oy) * c.h),
+                            (float)(xi.z - (R)(cz + g.oz) * c.h)};
+        const float hf = (float)c.h, hh = 0.5f * hf;
         half_cull = L.posh && cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
-                    fabsf(xi.x - hh) <= c.h && fabsf(xi.y - hh) <= c.h && fabsf(xi.z - hh) <= c.h;
-        if (half_cull) nq = cull_half(g, cs, pc, xi, c.h, c.cull2, L.posh, q, qstride, qcap);
+                    fabsf(xr.x - hh) <= hf && fabsf(xr.y - hh) <= hf && fabsf(xr.z - hh) <= hf;
+        if (half_cull) nq = cull_half(g, cs, pc, xr, hf, (float)c.cull2, L.posh, q, qstride, qcap);
     }
     if (!half_cull)
         walk<R, 1, true, FAST>(g, cs, pc, xi, c.h, 0, [&](uint32_t j, V3<R> s) {
@@ -302,13 +319,26 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
         });
     if (nq <= qcap) {
         // phase 2: evaluate the queued candidates in walk order
-        for (uint32_t k = 0; k < nq; ++k) {
-            const uint32_t j = q[k * qstride + threadIdx.x];
-            // (a plain load for the velocity: other threads write its w here)
-            V3<R> vj = {0, 0, 0};
-            if constexpr (DIV0) vj = xyz(f.vel[j]);
-            const V3<R> r = pair_vec(xi, pc, ldg4(f.pos + j), __ldg(f.cell + j), c.h);
-            accept(j, r, dot3(r, r), vj);
+        for (uint32_t k = 0; k < nq; k += EB) {
+            uint32_t j[EB], cj[EB];
+            P4<R> pj[EB];
+            V3<R> vj[EB];
+#pragma unroll
+            for (int b = 0; b < EB; ++b) {
+                // (past the end: the last candidate once more, not evaluated)
+                j[b] = q[(EB == 1 || k + b < nq ? k + b : nq - 1) * qstride + threadIdx.x];
+                // (a plain load for the velocity: other threads write its w here)
+                vj[b] = V3<R>{0, 0, 0};
+                if constexpr (DIV0) vj[b] = xyz(f.vel[j[b]]);
+                pj[b] = ldg4(f.pos + j[b]);
+                cj[b] = sizeof(R) == 4 ? __ldg(f.cell + j[b]) : 0u;
+            }
+#pragma unroll
+            for (int b = 0; b < EB; ++b) {
+                if (EB > 1 && k + b >= nq) break;
+                const V3<R> r = pair_vec(xi, pc, pj[b], cj[b], c.h);
+                accept(j[b], r, dot3(r, r), vj[b]);
+            }
         }
     } else {
         const BuildSums<R> b = build_walk_all<R, FAST>(i, f, g, cs, c, L, xi, pc);
@@ -334,14 +364,22 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
         // the same order as the walk, the gradient sum compiled apart from
         // the walk's, so its last bit may differ); or the walk itself.
         uint32_t nb = qcap + 1u;
-        if constexpr (FAST && sizeof(R) == 4) {
-            if (half_cull && L.bposh) nb = cull_half(g, bs, pc, xi, c.h, c.cull2, L.bposh, q, qstride, qcap);
-        }
+        if (half_cull && L.bposh) nb = cull_half(g, bs, pc, xr, (float)c.h, (float)c.cull2, L.bposh, q, qstride, qcap);
         if (nb <= qcap) {
-            for (uint32_t k = 0; k < nb; ++k) {
-                const uint32_t j = q[k * qstride + threadIdx.x];
-                const P4<R> pb = ldg4(bpos + j);
-                bterm(pb, pair_vec(xi, pc, pb, __ldg(L.bcell + j), c.h));
+            for (uint32_t k = 0; k < nb; k += EB) {
+                P4<R> pb[EB];
+                uint32_t cb[EB];
+#pragma unroll
+                for (int b = 0; b < EB; ++b) {
+                    const uint32_t j = q[(EB == 1 || k + b < nb ? k + b : nb - 1) * qstride + threadIdx.x];
+                    pb[b] = ldg4(bpos + j);
+                    cb[b] = sizeof(R) == 4 ? __ldg(L.bcell + j) : 0u;
+                }
+#pragma unroll
+                for (int b = 0; b < EB; ++b) {
+                    if (EB > 1 && k + b >= nb) break;
+                    bterm(pb[b], pair_vec(xi, pc, pb[b], cb[b], c.h));
+                }
             }
         } else {
             walk<R, 1>(g, bs, pc, xi, c.h, 0, [&](uint32_t j, V3<R> s) {
@@ -370,22 +408,81 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             *nn0 = d.nn;
         } else {
             if (nq > qcap) dv = reread_div<R>(f, L, i, vi, cnt);
-            if (akinci) dv += dot3(vi, bg);
+            if (akinci) dv += dot3_div(vi, bg);
             *div0 = dv;
             *nn0 = cnt;
         }
     }
 }
 
+// A particle's first divergence error from its velocity divergence
+// (computeDivergenceError's clamps and k; DFSPHSolver.cpp:468-486).
 template <typename R>
+__device__ __forceinline__ double divergence_error(uint32_t i, const Fluid<R>& f, const Lists<R>& L, const Consts<R>& c, R dt,
+                                                   R dv, uint32_t nn)
+{
+    dv = nn < 20u ? (R)0 : (dv < (R)0 ? (R)0 : dv);
+    f.div[i] = dv;
+    L.kbuf[i] = dv * f.alpha[i] / (dt * f.rho[i]);
+    return rel_error(c, (double)dv);
+}
+
+// The divergence solve's loop control after an error pass (INITIAL: before the
+// first iteration; DFSPHSolver.cpp:505-585).  One thread.
+template <bool INITIAL>
+__device__ __forceinline__ void divergence_control(DevScalars* sc, const LoopLimits& lim, double total, uint32_t n,
+                                                   cudaGraphConditionalHandle cond)
+{
+    const double avg = total / (double)n;
+    const double lim_v = lim.maxErrorV / sc->dt;
+    if (!isfinite(avg)) sc->status |= ST_NONFINITE;
+    if (INITIAL) {
+        sc->iterationsV = 0;
+        sc->avgDivError = avg;
+        sc->active = (lim.minItV > 0u) && (lim.maxIt > 0u);
+        if (!sc->active) sc->avgDivError = 0.0;
+    } else {
+        const unsigned it = ++sc->iterationsV;
+        sc->avgDivError = avg;
+        const unsigned act = ((avg > lim_v) || (it < lim.minItV)) && (it < lim.maxIt);
+        sc->active = act;
+        if (!act) {
+            sc->sumIterationsV += it;
+            if (it >= lim.maxIt && avg > lim_v) sc->status |= ST_ITER_CAP_V;
+        }
+    }
+    if (cond) cudaGraphSetConditional(cond, sc->active);
+}
+
+// DIV0: the build of a step, which also forms the divergence solve's first
+// error pass (its sums, its reduction and the first loop test): one pass over
+// the lists and one launch less (13k dam break 164 -> 150 us/step, 125k 275 ->
+// 265).  The half-precision cull serves FP64 too, whose distance test alone
+// (9 FP64 operations on each of ~150 candidates, at two FP64 lanes per SM)
+// was a third of the build: 125k particles 1454 -> 1003 us with the boundary's
+// cull and the fused error pass.
+template <typename R, bool DIV0>
 __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                            const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
-                                                           Consts<R> c, int akinci, Lists<R> L)
+                                                           Consts<R> c, int akinci, Lists<R> L, DevScalars* sc,
+                                                           LoopLimits lim, double* partials, cudaGraphConditionalHandle cond)
 {
     __shared__ uint32_t q[kQueue * kBlock];
     const uint32_t i = gtid();
-    if (i >= f.count()) return;
-    build_lists_one<R, sizeof(R) == 4>(i, f, bpos, g, cs, bs, c, akinci, L, q);
+    constexpr int EB = sizeof(R) == 4 ? 4 : 2;
+    double err = 0.0;
+    if (i < f.count()) {
+        R dv = 0;
+        uint32_t nn = 0;
+        build_lists_one<R, sizeof(R) == 4, DIV0, EB>(i, f, bpos, g, cs, bs, c, akinci, L, q, kBlock, kQueue, &dv, &nn);
+        if (DIV0) err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
+    }
+    if constexpr (DIV0) {
+        __shared__ double sh[33];
+        double total;
+        if (finish_reduction<false>(err, partials, &sc->block_counter, sh, &total) && threadIdx.x == 0)
+            divergence_control<true>(sc, lim, total, f.count(), cond);
+    }
 }
 
 // ---- cell-walk fallbacks for particles whose list overflowed -------------
@@ -522,9 +619,9 @@ __device__ __forceinline__ R velocity_div_list(const Fluid<R>& f, const Lists<R>
         const P4<R> q = ldcs4(p + (size_t)k * n);
         const uint32_t j = as_idx(q.w);
         if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-        d += dot3(vi - xyz(ldg4(f.vel + j)), xyz(q));
+        d += dot3_div(vi - xyz(ldg4(f.vel + j)), xyz(q));
     }
-    if (akinci) d += dot3(vi, xyz(L.bgrad[i]));
+    if (akinci) d += dot3_div(vi, xyz(L.bgrad[i]));
     return d;
 }
 
@@ -594,8 +691,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_predict_density_list(Fluid<
     }
 }
 
-// DFSPHSolver::computeDivergenceError over the lists (+ loop control).
-template <typename R, bool INITIAL>
+// DFSPHSolver::computeDivergenceError over the lists (+ loop control); the
+// step's first one is formed by the list build.
+template <typename R>
 __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                   Consts<R> c, int akinci, DevScalars* sc, LoopLimits lim,
@@ -603,41 +701,18 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f,
                                                                   Lists<R> L)
 {
     __shared__ double sh[33];
-    if (!INITIAL && !sc->active) return;
+    if (!sc->active) return;
     const uint32_t i = gtid();
     double err = 0.0;
     if (i < f.count()) {
         const V3<R> vi = xyz(f.vel[i]);
         uint32_t nn;
-        R dv = velocity_div_one(i, f, bpos, g, cs, bs, c, akinci, L, vi, &nn);
-        const R dt = (R)sc->dt;
-        dv = nn < 20u ? (R)0 : (dv < (R)0 ? (R)0 : dv);
-        f.div[i] = dv;
-        L.kbuf[i] = dv * f.alpha[i] / (dt * f.rho[i]);
-        err = rel_error(c, (double)dv);
+        const R dv = velocity_div_one(i, f, bpos, g, cs, bs, c, akinci, L, vi, &nn);
+        err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
     }
     double total;
-    if (finish_reduction<false>(err, partials, &sc->block_counter, sh, &total) && threadIdx.x == 0) {
-        const double avg = total / (double)f.count();
-        const double lim_v = lim.maxErrorV / sc->dt;
-        if (!isfinite(avg)) sc->status |= ST_NONFINITE;
-        if (INITIAL) {
-            sc->iterationsV = 0;
-            sc->avgDivError = avg;
-            sc->active = (lim.minItV > 0u) && (lim.maxIt > 0u);
-            if (!sc->active) sc->avgDivError = 0.0;
-        } else {
-            const unsigned it = ++sc->iterationsV;
-            sc->avgDivError = avg;
-            const unsigned act = ((avg > lim_v) || (it < lim.minItV)) && (it < lim.maxIt);
-            sc->active = act;
-            if (!act) {
-                sc->sumIterationsV += it;
-                if (it >= lim.maxIt && avg > lim_v) sc->status |= ST_ITER_CAP_V;
-            }
-        }
-        if (cond) cudaGraphSetConditional(cond, sc->active);
-    }
+    if (finish_reduction<false>(err, partials, &sc->block_counter, sh, &total) && threadIdx.x == 0)
+        divergence_control<false>(sc, lim, total, f.count(), cond);
 }
 
 // The stored lists of the n particles at [base, base + n) of a layout whose

@@ -249,10 +249,7 @@ __global__ void k_pool_boundary_half(uint32_t N, Boundary<float> b, const uint32
     if (d >= N) return;
     const float h = T[bsid[d]].c.h;
     const P4<float> x = b.pos[d];
-    __half* ph = reinterpret_cast<__half*>(posh) + (size_t)(d >> 1) * 8 + (d & 1);
-    ph[0] = __float2half_rn(x.x);
-    ph[2] = __float2half_rn(x.y);
-    ph[4] = __float2half_rn(zframe3(x.z, cell_z(b.cell[d]), h));
+    store_half(posh, d, x.x, x.y, zframe3(x.z, cell_z(b.cell[d]), h));
 }
 
 // AkinciBoundaryModel::computeVolume (AkinciBoundayModel.cpp:11-40) per scene.

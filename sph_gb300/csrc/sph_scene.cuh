@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <optional>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -352,6 +353,7 @@ public:
             k_gather_boundary<R><<<blocks(nb_, 256), 256, 0, st_>>>(nb_, tmp_.p, key_.p, bstarts_.p, B(0), B(1));
             SPH_CUDA(cudaGetLastError());
             if (akinci_) k_boundary_psi<R><<<blocks(nb_, 128), 128, 0, st_>>>(B(1), gv_, bstarts_.p, c_);
+            if (lists_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
             SPH_CUDA(cudaGetLastError());
             SPH_CUDA(cudaStreamSynchronize(st_));
         } else {
@@ -476,6 +478,7 @@ public:
             k_gather_boundary<R><<<blocks(nb_, 256), 256, 0, st_>>>(nb_, tmp_.p, key_.p, bstarts_.p, B(1), B(0));
             std::swap(bd_[0], bd_[1]);
             if (akinci_) k_boundary_psi<R><<<blocks(nb_, 128), 128, 0, st_>>>(B(1), gv_, bstarts_.p, c_);
+            if (lists_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
             SPH_CUDA(cudaGetLastError());
         } else {
             SPH_CUDA(cudaMemsetAsync(bstarts_.p, 0, (nkeys_ + 1) * sizeof(uint32_t), st_));
@@ -851,7 +854,8 @@ private:
     Fluid<R> F() const { return fl_[cur_]; }
     Lists<R> LS() const
     {
-        return Lists<R>{pairs_.p, lcount_.p, bgrad_.p, kbuf_.p, kmax_, posh_.p, &sc_.p->status, nullptr, nullptr};
+        return Lists<R>{pairs_.p, lcount_.p, bgrad_.p, kbuf_.p, kmax_, posh_.p, &sc_.p->status,
+                        nb_ ? bposh_.p : nullptr, bd_[1].cell};
     }
     Boundary<R> B(int k) const { return bd_[k]; }
 
@@ -981,11 +985,14 @@ private:
         SPH_CUDA(lcount_.alloc(lists_ ? n : 1));
         SPH_CUDA(bgrad_.alloc(lists_ ? n : 1));
         SPH_CUDA(kbuf_.alloc(n));
-        // FP32 pair lists: half-precision positions for the build's cull
-        // (particle pairs, the last one whole); written by every gather
-        if (lists_ && sizeof(R) == 4) {
-            SPH_CUDA(posh_.alloc(n / 2 + 2));  // a spare word past the last pair for the cull
+        // pair lists: half-precision positions for the build's cull (pairs of
+        // points, the last one whole, and a spare word for the cull), the
+        // fluid's written by every gather, the boundary's once per grid box
+        if (lists_) {
+            SPH_CUDA(posh_.alloc(n / 2 + 2));
             SPH_CUDA(cudaMemsetAsync(posh_.p, 0, (n / 2 + 2) * sizeof(uint4), st_));
+            SPH_CUDA(bposh_.alloc(nb / 2 + 2));
+            SPH_CUDA(cudaMemsetAsync(bposh_.p, 0, (nb / 2 + 2) * sizeof(uint4), st_));
         }
         SPH_CUDA(cudaMemsetAsync(lcount_.p, 0, lcount_.n * sizeof(uint32_t), st_));
         SPH_CUDA(cudaMemsetAsync(kbuf_.p, 0, n * sizeof(R), st_));
@@ -1054,7 +1061,7 @@ private:
         if (rc) return rc;
         run("k_scatter", [&] { k_scatter<<<blocks(n_, 256), 256, 0, ls_>>>(n_, key_.p, slot_.p, starts_.p, tmp_.p, a.na); });
         run("k_gather_fluid", [&] { k_gather_fluid<R><<<blocks(n_, 256), 256, 0, ls_>>>(n_, tmp_.p, key_.p, starts_.p, fl_[cur_], fl_[1 - cur_],
-                                                                                  posh_.p); });
+                                                                                  posh_.p, gv_, hd_); });
         SPH_CUDA(cudaGetLastError());
         cur_ = 1 - cur_;
         return SPH_OK;
@@ -1107,13 +1114,15 @@ private:
         return SPH_OK;
     }
 
-    // Densities, alpha and the DFSPH pair lists after a grid build.
-    int launch_build_lists()
+    // Densities, alpha and the DFSPH pair lists after a grid build (DIV0: and
+    // the divergence solve's first error pass, with its loop test into h).
+    template <bool DIV0 = false> int launch_build_lists(cudaGraphConditionalHandle h = 0)
     {
         Fluid<R> f = F();
         const P4<R>* bp = bd_[1].pos;
         Lists<R> L = LS();
-        run("k_build_lists", [&] { k_build_lists<R><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L); });
+        run("k_build_lists", [&] { k_build_lists<R, DIV0><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(
+            f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1263,25 +1272,24 @@ private:
         rc = dfsph_move_and_build();  // updatePositions + fill grid + neighbour search
         if (rc) return rc;
         {
-            auto ph = phase("Neigh search+Densities+Alpha factor");
-            rc = launch_build_lists();  // computeDensities + computeAlpha + pair lists
-            if (rc) return rc;
-            launch_bh_boundary(0);
-        }
-        {
             Fluid<R> f = F();
             const P4<R>* bp = bd_[1].pos;
             Lists<R> L = LS();
-            // correctDivergenceError DFSPHSolver.cpp:494-590
-            auto ph = phase("Divergence solver");
+            std::optional<Phase> solver;  // opened once the build is launched
             rc = solve_loop(2,
                 [&](cudaGraphConditionalHandle h) {
-                    run("k_dfsph_divergence_list", [&] { k_dfsph_divergence_list<R, true><<<nb, kBlock, 0, ls_>>>(
-                        f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
+                    {
+                        // computeDensities + computeAlpha + pair lists + the first divergence error
+                        auto ph = phase("Neigh search+Densities+Alpha factor");
+                        launch_build_lists<true>(h);
+                        launch_bh_boundary(0);
+                    }
+                    // correctDivergenceError DFSPHSolver.cpp:494-590
+                    solver.emplace(phases_, "Divergence solver", ls_, capturing_, prof_);
                 },
                 [&](cudaGraphConditionalHandle h) {
                     run("k_dfsph_correct_list", [&] { k_dfsph_correct_list<R, 2><<<nb, kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
-                    run("k_dfsph_divergence_list", [&] { k_dfsph_divergence_list<R, false><<<nb, kBlock, 0, ls_>>>(
+                    run("k_dfsph_divergence_list", [&] { k_dfsph_divergence_list<R><<<nb, kBlock, 0, ls_>>>(
                         f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
                 },
                 lim_.minItV, lim_.maxIt);
@@ -1642,7 +1650,7 @@ private:
     DevBuf<EmitterDev> em_;
     DevBuf<double> egroup_;
     DevBuf<double> cap_x_, cap_v_;  // staging of asynchronous frame captures
-    DevBuf<uint4> posh_;            // FP32 pair lists: half-precision positions (build cull, particle pairs)
+    DevBuf<uint4> posh_, bposh_;    // pair lists: half-precision positions, fluid and boundary (build cull)
     int akinci_ = 0;   // Akinci boundary model: boundary terms in the forces too
     int bh_ = 0;       // PCISPH boundary model
     int hasb_ = 0;     // boundary particles take part in the solver sums

@@ -2,10 +2,13 @@
 
 * Candidate lists whose fluid candidates fit but whose boundary candidates do not (those are then walked): the
   passes must still give the cell walks' results bit for bit.
+* The DFSPH list build that also forms the divergence solve's first error pass, at block edges.
 """
 import numpy as np
 import pytest
 
+import sph_gb300
+from scenes import jitter, lattice
 from test_pcisph_lists import drop, run
 
 pytestmark = pytest.mark.gpu
@@ -17,3 +20,42 @@ def test_boundary_candidates_beyond_the_list(gpu_lib, case, precision, lists):
     a, w = (run(x, v, b, p, precision, n, 12, True) for n in (lists, 0))
     for f in ("x", "v", "rho"):
         assert np.array_equal(a.get(f), w.get(f)), f
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("n", [127, 128, 129, 700])
+def test_first_divergence_error_formed_by_the_build(gpu_lib, precision, n):
+    """The list build's half-precision cull and the divergence error it forms, over one block, one particle less or
+    more, and a part of a block: FP64 against walks of every cell (neighbor_list_max = 0), FP32 against the same scene
+    in a pool (a walk's kernel values round differently there, and a pair at the support radius may count for one
+    of them and not for the other, which decides the solver's rule of 20 neighbours)."""
+    r = 0.02
+    x = jitter(lattice(r, (2 * r, 2 * r, 2 * r), (0.45, 0.45, 0.45)), r, 3)[:n]
+    v = np.random.default_rng(n).uniform(-0.2, 0.2, x.shape)
+    p = dict(method=2, boundary=2, radius=r, precision=precision, eta=0.001, eta_v=0.001, max_it_v=0, min_it_v=0)
+    b = sph_gb300.sample_box(4 * r, (0, 0, 0), (0.6, 0.6, 0.6))
+
+    def alone(lists):
+        s = sph_gb300.Scene(neighbor_list_max=lists, threads_per_particle=1, **p)
+        s.set_fluid(x, v)
+        s.add_boundary_points(b)
+        s.init()
+        s.step(1)
+        return s.get("rho"), s.get("alpha"), s.get("div"), s.stats()["iterations"]
+
+    def pooled():
+        P = sph_gb300.Pool(max_particles=n, max_boundary=len(b), max_keys=100_000, max_scenes=2)
+        P.set_autotune(0)
+        k = P.add_scene(x, v=v, boundary_points=b, steps=2, **p)
+        P.step(1)
+        return P.get(k, "rho"), P.get(k, "alpha"), P.get(k, "div"), P.query(k)[0]["iterations"]
+
+    rho, alpha, div, it = alone(64)
+    rho0, alpha0, div0, it0 = pooled() if precision == "f32" else alone(0)
+    # sums of up to ~60 terms, the boundary's pre-added in the lists: 60 roundings of the largest value
+    tol = 60 * (2.0**-24 if precision == "f32" else 2.0**-53)
+    assert it == it0
+    for a, e, scale in ((rho, rho0, 1.0), (alpha, alpha0, 4.0)):
+        assert np.abs(a - e).max() <= scale * tol * np.abs(e).max()
+    # a divergence sums terms of either sign: bound by the sum of their sizes, |v_i - v_j| |m grad W| <= 0.7 * 60 * 500
+    assert np.abs(div - div0).max() <= tol * 0.7 * 60 * 500
