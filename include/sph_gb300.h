@@ -272,7 +272,9 @@ int sph_ctx_num_particles(const sph_ctx* ctx, unsigned* num_fluid, unsigned* num
 /* The descriptor the context was created with (for a loaded scene file:
  * the settings read from it). */
 int sph_ctx_get_desc(const sph_ctx* ctx, sph_scene_desc* out);
-/* Copy a field to host memory in original particle order (FP64). */
+/* Copy a field to host memory in original particle order (FP64).  The
+ * context keeps the device staging buffer of its largest download (8 bytes a
+ * value) until it is destroyed. */
 int sph_ctx_download(sph_ctx* ctx, int field, double* out);
 /* Same result as sph_ctx_download, without allocating device memory.  It has
  * no counterpart in the reference (which keeps its fields in host vectors).
@@ -280,8 +282,8 @@ int sph_ctx_download(sph_ctx* ctx, int field, double* out);
  * long-running serving process whose device memory is fully reserved for
  * resident scenes, or a real-time driver that must not call cudaFree (it
  * waits for the whole device).  sph_ctx_download allocates a staging buffer
- * per call; this variant stages through one fixed 4 MiB device array inside
- * the library instead.
+ * for the largest field read so far; this variant stages through one fixed
+ * 4 MiB device array inside the library instead.
  *   - Limit: a field of at most 524,288 values (174,762 particles for
  *     3-component fields); larger fields return SPH_ERR_CAPACITY.
  *   - The array is held by every GPU that loads the library until exit.

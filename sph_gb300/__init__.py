@@ -529,7 +529,7 @@ class Scene:
     def get(self, field):
         fid, width = FIELDS[field]
         count = self.nb if field in ("bx", "psi", "bdens", "bpress") else self.n
-        out = np.zeros((count, 3) if width == 3 else count)
+        out = np.empty((count, 3) if width == 3 else count)  # every value is written
         if count:
             self._check(lib().sph_ctx_download(self._h, fid, _d(out)), f"sph_ctx_download({field})")
         return out

@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <optional>
 #include <string>
 #include <type_traits>
@@ -639,8 +640,11 @@ public:
                          field == SPH_FIELD_BOUNDARY_POSITION;
         const size_t count = (size_t)n * (vec ? 3 : 1);
         if (count == 0) return SPH_OK;
-        DevBuf<double> o;
-        SPH_CUDA(o.alloc(count));
+        // a staging buffer kept between downloads (grow-only): no allocation,
+        // and no cudaFree, which waits for the whole device, per call.  Held
+        // for the whole call: several threads may read one scene.
+        std::lock_guard<std::mutex> hold(dl_mu_);
+        if (dl_.n < count) SPH_CUDA(dl_.alloc(count));
         Fluid<R> f = F();
         Boundary<R> b = B(1);
         const P4<R>* v4 = nullptr;
@@ -666,9 +670,9 @@ public:
             default: fail("unknown field"); return SPH_ERR_INVALID;
         }
         k_download<R><<<blocks(n, 256), 256, 0, st_>>>(n, v4, s, bnd ? b.id : f.id, bnd ? b.cell : f.cell, gv_, hd_, kind,
-                                                      o.p);
+                                                      dl_.p);
         SPH_CUDA(cudaGetLastError());
-        SPH_CUDA(cudaMemcpyAsync(out, o.p, count * 8, cudaMemcpyDeviceToHost, st_));
+        SPH_CUDA(cudaMemcpyAsync(out, dl_.p, count * 8, cudaMemcpyDeviceToHost, st_));
         SPH_CUDA(cudaStreamSynchronize(st_));
         return SPH_OK;
     }
@@ -1649,6 +1653,8 @@ private:
     int nem_ = 0;               // emitters
     DevBuf<EmitterDev> em_;
     DevBuf<double> egroup_;
+    DevBuf<double> dl_;             // staging of downloads (original order, FP64)
+    std::mutex dl_mu_;
     DevBuf<double> cap_x_, cap_v_;  // staging of asynchronous frame captures
     DevBuf<uint4> posh_, bposh_;    // pair lists: half-precision positions, fluid and boundary (build cull)
     int akinci_ = 0;   // Akinci boundary model: boundary terms in the forces too
