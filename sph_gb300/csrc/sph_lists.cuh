@@ -485,6 +485,345 @@ __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<
     }
 }
 
+// ---- the list build with W lanes per particle --------------------------------
+//
+// A scene of a few thousand particles has fewer warps than the chip has
+// schedulers, so one lane's build is one long chain of dependent loads (38 us
+// for 2,000 particles as for 24,000; 14 us and 31 us here).  Here W lanes share a particle: each
+// looks up its columns' ranges, tests its words of a column's candidates, and
+// evaluates its part of the accepted ones; the values go to shared memory and
+// are then summed one after another, each of the sums by a lane of its own,
+// in the list's order and with the rounding of build_lists_one (written out
+// below), so the results are bit-identical to it.
+
+// a * b + c as build_lists_one rounds it: fused in FP32, two roundings in the
+// FP64 parity form (compiled without contraction)
+__device__ __forceinline__ float mul_add(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+
+// |a|^2 as build_lists_one rounds it for the sum of the gradients
+__device__ __forceinline__ float sum_sq(V3<float> a) { return __fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))); }
+__device__ __forceinline__ double sum_sq(V3<double> a) { return dot3(a, a); }
+
+constexpr uint32_t kWideBlock = 128, kWideChunk = 32;
+
+// The candidate ranges of cull_half's nine columns, lane gl of W holding
+// columns gl, gl + W, ...: in b[], e[] (empty where trimmed, or with !on).
+template <int W> struct WideRanges {
+    static constexpr int C = (9 + W - 1) / W;
+    uint32_t b[C], e[C];
+};
+template <int W>
+__device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const GridView& g, const uint32_t* __restrict__ starts,
+                                                     uint32_t pc, V3<float> xi, float h)
+{
+    const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
+    const float ofx = xi.x, ofy = xi.y, ofz = xi.z;
+    const float gxm = ofx > 0.f ? ofx * ofx : 0.f, gxp = h - ofx > 0.f ? (h - ofx) * (h - ofx) : 0.f;
+    const float gym = ofy > 0.f ? ofy * ofy : 0.f, gyp = h - ofy > 0.f ? (h - ofy) * (h - ofy) : 0.f;
+    const float gzm = ofz > 0.f ? ofz * ofz : 0.f, gzp = h - ofz > 0.f ? (h - ofz) * (h - ofz) : 0.f;
+    const float lim = h * h * (float)(1.0 + 1e-5);
+    WideRanges<W> r;
+#pragma unroll
+    for (int t = 0; t < WideRanges<W>::C; ++t) {
+        const int c = gl + t * W;
+        r.b[t] = r.e[t] = 0u;
+        if (on && c < 9) {
+            const int dx = c / 3 - 1, dy = c % 3 - 1;
+            const float gxy = (dx < 0 ? gxm : (dx > 0 ? gxp : 0.f)) + (dy < 0 ? gym : (dy > 0 ? gyp : 0.f));
+            if (gxy <= lim) {
+                const uint32_t base = (__ldg(g.mortx + cx + dx) | __ldg(g.morty + cy + dy)) * (uint32_t)g.nz;
+                r.b[t] = __ldg(starts + base + (gxy + gzm <= lim ? cz - 1 : cz));
+                r.e[t] = __ldg(starts + base + (gxy + gzp <= lim ? cz + 2 : cz + 1));
+            }
+        }
+    }
+    return r;
+}
+
+// cull_half by W lanes: accepted candidates in walk order into the group's
+// queue; every lane returns their number.  gl = lane in the group; all lanes
+// of the warp call it.
+template <int W>
+__device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W>& rg, int cz, V3<float> xi, float h, float cull2,
+                                                   const uint4* __restrict__ posh, uint32_t* q, uint32_t qcap)
+{
+    const __half2 thr = __float2half2_rn(cull2 * 1.03f);
+    const __half2 zq = __float2half2_rn(zframe3(xi.z, cz, h));
+    const __half2 h3 = __float2half2_rn(3.f * h);
+    const int g0 = (int)(threadIdx.x & 31) & ~(W - 1);
+    // the first round of every column's words, all in flight together
+    uint4 w0[9];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        const uint32_t bb = __shfl_sync(0xffffffffu, rg.b[c / W], c % W, W), ee = __shfl_sync(0xffffffffu, rg.e[c / W], c % W, W);
+        const uint32_t word = (bb >> 1) + gl;
+        w0[c] = make_uint4(0u, 0u, 0u, 0u);
+        if (2 * word < ee) w0[c] = __ldg(posh + word);
+    }
+    uint32_t nq = 0;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        const int dx = c / 3 - 1, dy = c % 3 - 1;
+        const uint32_t bb = __shfl_sync(0xffffffffu, rg.b[c / W], c % W, W), ee = __shfl_sync(0xffffffffu, rg.e[c / W], c % W, W);
+        const __half2 sx = __float2half2_rn(xi.x - (float)dx * h), sy = __float2half2_rn(xi.y - (float)dy * h);
+        uint32_t word = (bb >> 1) + gl;
+        uint4 w = w0[c];
+        // rounds of W words; the warp runs the longest of its groups' columns
+        while (__any_sync(0xffffffffu, 2 * (word - gl) < ee)) {
+            const __half2 ddx = __hsub2(sx, as_half2(w.x)), ddy = __hsub2(sy, as_half2(w.y));
+            const __half2 dz = __habs2(__hsub2(zq, as_half2(w.z)));
+            const __half2 ddz = __hmin2(dz, __hsub2(h3, dz));
+            const __half2 r2 = __hfma2(ddz, ddz, __hfma2(ddy, ddy, __hmul2(ddx, ddx)));
+            const unsigned m = __hle2_mask(r2, thr);
+            const uint32_t j = 2 * word;
+            const bool a0 = (m & 1u) && j >= bb && j < ee;
+            const bool a1 = (m & 0x10000u) && j + 1 < ee;
+            const uint32_t b0 = (__ballot_sync(0xffffffffu, a0) >> g0) & ((1u << W) - 1u);
+            const uint32_t b1 = (__ballot_sync(0xffffffffu, a1) >> g0) & ((1u << W) - 1u);
+            const uint32_t below = (1u << gl) - 1u;
+            uint32_t at = nq + __popc(b0 & below) + __popc(b1 & below);
+            if (a0) {
+                if (at < qcap) q[at] = j;
+                ++at;
+            }
+            if (a1 && at < qcap) q[at] = j + 1;
+            nq += __popc(b0) + __popc(b1);
+            word += W;
+            if (2 * word < ee) w = __ldg(posh + word);
+        }
+    }
+    return nq;
+}
+
+template <typename R, int W, bool DIV0>
+__global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
+                                                                 const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
+                                                                 Consts<R> c, int akinci, Lists<R> L, DevScalars* sc,
+                                                                 LoopLimits lim, double* partials, cudaGraphConditionalHandle cond)
+{
+    static_assert(W == 8 || W == 4, "a lane per sum, or two sums a lane");
+    constexpr bool FAST = sizeof(R) == 4;
+    constexpr uint32_t GROUPS = kWideBlock / W;
+    __shared__ uint32_t queue[GROUPS][kQueue], bqueue[GROUPS][kQueue];
+    // per entry: W, m grad W, |m grad W|^2 and the divergence term (fluid), or W, grad W and the weight (boundary)
+    // of kWideChunk entries at a time (five blocks per SM at W = 4)
+    __shared__ R val[GROUPS][kWideChunk][6];
+    const int gl = (int)(threadIdx.x % W), grp = (int)(threadIdx.x / W);
+    const int lane = threadIdx.x & 31, g0 = lane & ~(W - 1);
+    const uint32_t i = (blockIdx.x * kWideBlock + threadIdx.x) / W;
+    const uint32_t n = f.n;
+    const bool valid = i < f.count();
+    uint32_t* q = queue[grp];
+    R(*v)[6] = val[grp];
+    const uint32_t qcap = L.kmax < kQueue ? L.kmax : kQueue;
+    V3<R> xi = {0, 0, 0}, vi = {0, 0, 0};
+    uint32_t pc = 0;
+    V3<float> xr = {0, 0, 0};
+    bool half = false;
+    const float hf = (float)c.h;
+    if (valid) {
+        xi = xyz(f.pos[i]);
+        pc = f.cell[i];
+        if constexpr (DIV0) vi = xyz(f.vel[i]);
+        const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
+        if constexpr (sizeof(R) == 4) xr = xi;
+        else xr = V3<float>{(float)(xi.x - (R)(cx + g.ox) * c.h), (float)(xi.y - (R)(cy + g.oy) * c.h),
+                            (float)(xi.z - (R)(cz + g.oz) * c.h)};
+        const float hh = 0.5f * hf;
+        half = cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
+               fabsf(xr.x - hh) <= hf && fabsf(xr.y - hh) <= hf && fabsf(xr.z - hh) <= hf;
+    }
+    const bool bhalf = half && akinci && L.bposh;
+    const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf), rb = wide_ranges<W>(bhalf, gl, g, bs, pc, xr, hf);
+    uint32_t nq = cull_half_wide<W>(gl, rf, cell_z(pc), xr, hf, (float)c.cull2, L.posh, q, qcap);
+    uint32_t nb = __any_sync(0xffffffffu, bhalf)
+                      ? cull_half_wide<W>(gl, rb, cell_z(pc), xr, hf, (float)c.cull2, L.bposh, bqueue[grp], qcap) : 0u;
+    if (valid && !half) {
+        // near the grid box's border: one lane culls in R
+        if (gl == 0)
+            walk<R, 1, true, true>(g, cs, pc, xi, c.h, 0, [&](uint32_t j, V3<R> s) {
+                const V3<R> r = s - xyz(ldg4(f.pos + j));
+                if (dot3(r, r) <= c.cull2) {
+                    if (nq < qcap) q[nq] = j;
+                    ++nq;
+                }
+            });
+    }
+    nq = __shfl_sync(0xffffffffu, nq, 0, W);
+    __syncwarp();
+    const bool over = nq > qcap;
+    // the sums in list order: sum s by lane s (W = 8), or s and s + 4 (W = 4)
+    R acc[8 / W];
+#pragma unroll
+    for (int t = 0; t < 8 / W; ++t) acc[t] = 0;
+    uint32_t cnt = 0;
+    const uint32_t ne = over ? 0u : nq;
+    for (uint32_t k0 = 0; __any_sync(0xffffffffu, k0 < ne); k0 += kWideChunk) {
+        const uint32_t m = k0 < ne ? (ne - k0 < kWideChunk ? ne - k0 : kWideChunk) : 0u;  // this chunk's entries
+        // evaluation, 2 W entries a round (both loads in flight); records in list order
+        for (uint32_t k = 0; __any_sync(0xffffffffu, k < m); k += 2 * W) {
+            uint32_t j[2], cj[2];
+            P4<R> pj[2];
+            V3<R> vj[2];
+            bool in[2];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const uint32_t e = k + t * W + gl;
+                in[t] = e < m;
+                if (in[t]) {
+                    j[t] = q[k0 + e];
+                    pj[t] = ldg4(f.pos + j[t]);
+                    cj[t] = sizeof(R) == 4 ? __ldg(f.cell + j[t]) : 0u;
+                    // (a plain load: other threads write its w here)
+                    if constexpr (DIV0) vj[t] = xyz(f.vel[j[t]]);
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                bool listed = false;
+                V3<R> mg = {0, 0, 0};
+                if (in[t]) {
+                    const V3<R> r = pair_vec(xi, pc, pj[t], cj[t], c.h);
+                    R w;
+                    V3<R> gw;
+                    cubic_W_gradW<FAST>(c, r, dot3(r, r), &w, &gw);
+                    mg = c.mass * gw;
+                    const R mg2 = dot3_div(mg, mg);
+                    listed = mg2 > (R)0;
+                    R sq = mg2;
+                    if constexpr (sizeof(R) == 8) {
+                        const R m1 = sqrt(mg2);
+                        sq = m1 * m1;
+                    }
+                    R* o = v[k + t * W + gl];
+                    o[0] = w;
+                    // an unlisted pair adds zeros (it would be left out: the same sums)
+                    o[1] = listed ? mg.x : (R)0; o[2] = listed ? mg.y : (R)0; o[3] = listed ? mg.z : (R)0;
+                    o[4] = listed ? sq : (R)0;
+                    if constexpr (DIV0) o[5] = listed ? dot3_div(vi - vj[t], mg) : (R)0;
+                }
+                const uint32_t b = (__ballot_sync(0xffffffffu, listed) >> g0) & ((1u << W) - 1u);
+                if (listed) {
+                    const uint32_t at = cnt + __popc(b & ((1u << gl) - 1u));
+                    if (at < L.kmax) L.pairs[(size_t)at * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j[t])};
+                }
+                cnt += __popc(b);
+            }
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (uint32_t k = 0; k < m; ++k) {
+#pragma unroll
+            for (int t = 0; t < 8 / W; ++t) {
+                const int s = gl + t * W;
+                if (s < (DIV0 ? 6 : 5)) {
+                    const R x = v[k][s];
+                    acc[t] = s == 0 ? mul_add(c.mass, x, acc[t]) : acc[t] + x;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (over && gl == 0) {
+        const BuildSums<R> b = build_walk_all<R, FAST>(i, f, g, cs, c, L, xi, pc);
+        v[0][0] = b.density; v[0][1] = b.sumGrad.x; v[0][2] = b.sumGrad.y; v[0][3] = b.sumGrad.z; v[0][4] = b.sumSq;
+        cnt = b.cnt;
+    }
+    __syncwarp();
+    cnt = __shfl_sync(0xffffffffu, cnt, 0, W);
+    if (over) {
+#pragma unroll
+        for (int t = 0; t < 8 / W; ++t) acc[t] = gl + t * W < 5 ? v[0][gl + t * W] : (R)0;
+    }
+    __syncwarp();
+    // boundary: W, grad W and weight per entry, then density and gradient sums
+    R bacc = 0;  // lanes 1..3: the boundary gradient's components
+    const bool bwalk = valid && akinci && (!bhalf || nb > qcap);
+    if (bwalk) nb = 0;
+    for (uint32_t k0 = 0; __any_sync(0xffffffffu, k0 < nb); k0 += kWideChunk) {
+        const uint32_t m = k0 < nb ? (nb - k0 < kWideChunk ? nb - k0 : kWideChunk) : 0u;
+        for (uint32_t e = gl; e < m; e += W) {
+            const uint32_t j = bqueue[grp][k0 + e];
+            const P4<R> pb = ldg4(bpos + j);
+            const V3<R> r = pair_vec(xi, pc, pb, sizeof(R) == 4 ? __ldg(L.bcell + j) : 0u, c.h);
+            const R r2 = dot3(r, r);
+            R w;
+            V3<R> gw;
+            cubic_W_gradW<FAST>(c, r, r2, &w, &gw);
+            const bool in = r2 <= c.cull2;
+            v[e][0] = in ? w : (R)0;
+            v[e][1] = in ? gw.x : (R)0; v[e][2] = in ? gw.y : (R)0; v[e][3] = in ? gw.z : (R)0;
+            v[e][4] = pb.w;
+        }
+        __syncwarp();
+        if (gl == 0)
+            for (uint32_t k = 0; k < m; ++k) acc[0] = mul_add(v[k][4], v[k][0], acc[0]);
+        else if (gl < 4)
+            for (uint32_t k = 0; k < m; ++k) bacc = mul_add(v[k][4], v[k][gl], bacc);
+        __syncwarp();
+    }
+    if (bwalk && gl == 0) {
+        V3<R> bg = {0, 0, 0};
+        R density = acc[0];
+        walk<R, 1, true, true>(g, bs, pc, xi, c.h, 0, [&](uint32_t j, V3<R> s) {
+            const P4<R> pb = ldg4(bpos + j);
+            const V3<R> r = s - xyz(pb);
+            const R r2 = dot3(r, r);
+            if (!(r2 <= c.cull2)) return;
+            R w;
+            V3<R> gw;
+            cubic_W_gradW<FAST>(c, r, r2, &w, &gw);
+            density = mul_add(pb.w, w, density);
+            bg = V3<R>{mul_add(pb.w, gw.x, bg.x), mul_add(pb.w, gw.y, bg.y), mul_add(pb.w, gw.z, bg.z)};
+        });
+        acc[0] = density;
+        v[0][1] = bg.x; v[0][2] = bg.y; v[0][3] = bg.z;
+    }
+    __syncwarp();
+    if (bwalk && gl > 0 && gl < 4) bacc = v[0][gl];
+    // everything to the group's first lane
+    const R density = acc[0];
+    const R sg = acc[0] + bacc;  // lanes 1..3: sum of the gradients
+    const V3<R> sumGrad = {__shfl_sync(0xffffffffu, sg, 1, W), __shfl_sync(0xffffffffu, sg, 2, W), __shfl_sync(0xffffffffu, sg, 3, W)};
+    const V3<R> bg = {__shfl_sync(0xffffffffu, bacc, 1, W), __shfl_sync(0xffffffffu, bacc, 2, W), __shfl_sync(0xffffffffu, bacc, 3, W)};
+    const R sumSq = __shfl_sync(0xffffffffu, acc[W == 8 ? 0 : 4 / W % (8 / W)], W == 8 ? 4 : 0, W);
+    R dv = __shfl_sync(0xffffffffu, acc[W == 8 ? 0 : 4 / W % (8 / W)], W == 8 ? 5 : 1, W);
+    double err = 0.0;
+    if (valid && gl == 0) {
+        f.rho[i] = density;
+        f.vel[i].w = density;
+        R den;
+        if constexpr (sizeof(R) == 8) {
+            const R m = sqrt(dot3(sumGrad, sumGrad));
+            den = m * m + sumSq;
+        } else {
+            den = sum_sq(sumGrad) + sumSq;
+        }
+        f.alpha[i] = (fabs(den) > c.eps) ? density / den : (R)0;
+        L.count[i] = cnt;
+        L.bgrad[i] = P4<R>{bg.x, bg.y, bg.z, 0};
+        if constexpr (DIV0) {
+            uint32_t nn = cnt;
+            if (cnt > L.kmax) {
+                const DivSum<R> d = velocity_div_cells(f, bpos, g, cs, bs, c, akinci, i, vi);
+                dv = d.dv;
+                nn = d.nn;
+            } else {
+                if (over) dv = reread_div<R>(f, L, i, vi, cnt);
+                if (akinci) dv += dot3_div(vi, bg);
+            }
+            err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
+        }
+    }
+    if constexpr (DIV0) {
+        __shared__ double sh[33];
+        double total;
+        if (finish_reduction<false>(err, partials, &sc->block_counter, sh, &total) && threadIdx.x == 0)
+            divergence_control<true>(sc, lim, total, f.count(), cond);
+    }
+}
+
 // ---- cell-walk fallbacks for particles whose list overflowed -------------
 
 template <typename R, int MODE>

@@ -276,6 +276,7 @@ public:
         }
         G_ = (G == 2 || G == 4 || G == 8) ? G : 1;
         SPH_CUDA(cudaGetDevice(&device_));
+        SPH_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_));
         SPH_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
         SPH_CUDA(cudaStreamCreateWithFlags(&st2_, cudaStreamNonBlocking));
         ls_ = st_;
@@ -1118,6 +1119,22 @@ private:
         return SPH_OK;
     }
 
+    // Lanes per particle of the list build (results do not depend on it).
+    // Several lanes shorten the chain of dependent loads but execute two to
+    // three times the instructions, so they pay while their blocks are all
+    // resident at once: 8 lanes at 4 blocks of 16 particles per SM, 4 lanes at
+    // 5 blocks of 32.  Build in us (1 / 4 / 8 lanes, FP32, with the ~5 us of an
+    // event pair): 2,000 particles 42.6 / 22.3 / 18.4; 8,000 45.2 / 24.5 / 21.8;
+    // 13,000 44.3 / 26.5 / 30.4; 24,000 46.0 / 35.7 / 39.4; 30,000 47.7 / 49.8 /
+    // 46.6; 40,000 50.1 / 53.6 / 59.2.  FP64: 2,000 177 / 63 / 43; 13,000 195 /
+    // 140 / 161; 30,000 309 / 304 / 316.
+    int build_lanes() const
+    {
+        if ((size_t)n_ <= (size_t)sms_ * 4 * (kWideBlock / 8)) return 8;
+        if ((size_t)n_ <= (size_t)sms_ * 5 * (kWideBlock / 4)) return 4;
+        return 1;
+    }
+
     // Densities, alpha and the DFSPH pair lists after a grid build (DIV0: and
     // the divergence solve's first error pass, with its loop test into h).
     template <bool DIV0 = false> int launch_build_lists(cudaGraphConditionalHandle h = 0)
@@ -1125,8 +1142,17 @@ private:
         Fluid<R> f = F();
         const P4<R>* bp = bd_[1].pos;
         Lists<R> L = LS();
-        run("k_build_lists", [&] { k_build_lists<R, DIV0><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(
-            f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
+        auto wide = [&](auto wt) {
+            constexpr int W = decltype(wt)::value;
+            run("k_build_lists", [&] { k_build_lists_wide<R, W, DIV0><<<blocks((size_t)n_ * W, kWideBlock), kWideBlock, 0, ls_>>>(
+                f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
+        };
+        const int W = build_lanes();
+        if (W == 8) wide(std::integral_constant<int, 8>{});
+        else if (W == 4) wide(std::integral_constant<int, 4>{});
+        else
+            run("k_build_lists", [&] { k_build_lists<R, DIV0><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(
+                f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1660,7 +1686,7 @@ private:
     int akinci_ = 0;   // Akinci boundary model: boundary terms in the forces too
     int bh_ = 0;       // PCISPH boundary model
     int hasb_ = 0;     // boundary particles take part in the solver sums
-    int device_ = 0;
+    int device_ = 0, sms_ = 1;
     int G_ = 1;
     uint32_t nkeys_ = 0;
     int cur_ = 0;

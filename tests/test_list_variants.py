@@ -3,6 +3,8 @@
 * Candidate lists whose fluid candidates fit but whose boundary candidates do not (those are then walked): the
   passes must still give the cell walks' results bit for bit.
 * The DFSPH list build that also forms the divergence solve's first error pass, at block edges.
+* The list build with 8, 4 and 1 lanes per particle (chosen by scene size), with lists that hold every neighbour and
+  lists that overflow.
 """
 import numpy as np
 import pytest
@@ -59,3 +61,36 @@ def test_first_divergence_error_formed_by_the_build(gpu_lib, precision, n):
         assert np.abs(a - e).max() <= scale * tol * np.abs(e).max()
     # a divergence sums terms of either sign: bound by the sum of their sizes, |v_i - v_j| |m grad W| <= 0.7 * 60 * 500
     assert np.abs(div - div0).max() <= tol * 0.7 * 60 * 500
+
+
+@pytest.mark.parametrize("lists", [64, 24])
+@pytest.mark.parametrize("side", [(1, 1, 1), (5, 3, 3), (21, 21, 22), (22, 21, 21), (23, 23, 23), (29, 29, 29), (30, 29, 29)])
+def test_build_lanes_match_the_pool(gpu_lib, side, lists):
+    """One scene (lanes by size: the sides around 9.7k and 24k particles change them) against the same scene in a pool
+    (one lane): the same neighbours in the same order, the same sums up to their rounding."""
+    r = 0.01
+    d = 2 * r
+    x = lattice(r, (d, d, d), tuple(d + d * k + 1e-9 for k in side))
+    assert x.shape[0] == side[0] * side[1] * side[2]
+    rng = np.random.default_rng(7)
+    # jittered enough that no pair lies at the support radius to rounding
+    x = x + rng.uniform(-0.2 * r, 0.2 * r, x.shape)
+    v = rng.uniform(-0.2, 0.2, x.shape)
+    p = dict(method=2, boundary=2, radius=r, precision="f32", eta=0.001, eta_v=0.001)
+    b = sph_gb300.sample_box(4 * r, (0, 0, 0), (0.8, 0.8, 0.8))
+    s = sph_gb300.Scene(neighbor_list_max=lists, **p)
+    s.set_fluid(x, v)
+    s.add_boundary_points(b)
+    s.init()
+    s.step(1)
+    P = sph_gb300.Pool(max_particles=len(x), max_boundary=len(b), max_keys=200_000, max_scenes=2, neighbor_list_max=lists)
+    P.set_autotune(0)
+    k = P.add_scene(x, v=v, boundary_points=b, steps=2, **p)
+    P.step(1)
+    a, e = s.pair_lists(), P.pair_lists(k)
+    for f in ("count", "off", "nbr"):
+        assert np.array_equal(a[f], e[f]), f
+    # the one-scene / pool bounds of the smoke test
+    for f, tol in (("x", 1e-6), ("rho", 1e-5), ("alpha", 4e-5)):
+        g, w = s.get(f), P.get(k, f)
+        assert np.abs(g - w).max() <= tol * np.abs(w).max(), f
