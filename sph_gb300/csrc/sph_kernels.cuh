@@ -114,6 +114,7 @@ __device__ __forceinline__ void store_particle(const Fluid<R>& f, uint32_t i, do
 static __global__ void k_shift_cells(uint32_t n, const uint32_t* __restrict__ na, uint32_t* __restrict__ cell, int sx,
                                      int sy, int sz)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= (na ? *na : n)) return;
     const uint32_t c = cell[i];
@@ -125,6 +126,7 @@ template <typename R>
 __global__ void k_upload_fluid(const double* __restrict__ x, const double* __restrict__ v, uint32_t n,
                                uint32_t first, Fluid<R> f, GridView g, double h, DevScalars* sc)
 {
+    grid_wait();
     const uint32_t t = gtid();
     if (t >= n) return;
     store_particle(f, first + t, x[3 * t], x[3 * t + 1], x[3 * t + 2], v[3 * t], v[3 * t + 1], v[3 * t + 2], g, h, sc);
@@ -134,6 +136,7 @@ template <typename R>
 __global__ void k_upload_boundary(const double* __restrict__ x, uint32_t n, Boundary<R> b, GridView g, double h,
                                   DevScalars* sc)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= n) return;
     const double px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
@@ -167,6 +170,7 @@ template <typename R>
 __global__ void k_download(uint32_t n, const P4<R>* __restrict__ v4, const R* __restrict__ s, const uint32_t* __restrict__ id,
                            const uint32_t* __restrict__ cell, GridView g, double h, int kind, double* __restrict__ out)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= n) return;
     const uint32_t o = id[i];
@@ -201,6 +205,7 @@ __global__ void k_cell_update(uint32_t n, P4<R>* __restrict__ pos, const P4<R>* 
                               GridView g, R h, double hd, DevScalars* sc, uint32_t* __restrict__ cell_epoch = nullptr,
                               P4<R>* __restrict__ carry = nullptr, const uint32_t* __restrict__ na = nullptr)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= (na ? *na : n)) return;
     P4<R> p = pos[i];
@@ -253,6 +258,7 @@ __global__ void k_cell_update(uint32_t n, P4<R>* __restrict__ pos, const P4<R>* 
 static __global__ void k_cell_count(uint32_t n, const uint32_t* __restrict__ cell, uint32_t* __restrict__ key,
                              uint32_t* __restrict__ slot, uint32_t* __restrict__ count, GridView g)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= n) return;
     const uint32_t c = cell[i];
@@ -305,6 +311,7 @@ template <unsigned PER = kScanPer>
 static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t nkeys, uint32_t* __restrict__ count,
                                                              uint32_t* __restrict__ starts, uint32_t* __restrict__ tile_sums)
 {
+    grid_wait();
     static_assert(PER % 4 == 0, "whole uint4 per thread");
     __shared__ uint32_t sh[33];
     const uint32_t base = blockIdx.x * (kScanThreads * PER) + threadIdx.x * PER;
@@ -352,6 +359,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t nke
 static __global__ void __launch_bounds__(1024) k_scan_tile_sums(uint32_t ntiles, uint32_t* __restrict__ tile_sums,
                                                          uint32_t* __restrict__ starts, uint32_t nkeys)
 {
+    grid_wait();
     __shared__ uint32_t sh[33];
     uint32_t carry = 0;
     for (uint32_t b = 0; b < ntiles; b += blockDim.x) {
@@ -369,6 +377,7 @@ template <unsigned PER = kScanPer>
 static __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t nkeys, const uint32_t* __restrict__ tile_sums,
                                                            uint32_t* __restrict__ starts)
 {
+    grid_wait();
     const uint32_t add = tile_sums[blockIdx.x];
     const uint32_t base = blockIdx.x * (kScanThreads * PER) + threadIdx.x * PER;
     if (base + PER <= nkeys) {
@@ -388,6 +397,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t nkeys
 static __global__ void k_scatter(uint32_t n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ slot,
                           const uint32_t* __restrict__ starts, uint32_t* __restrict__ tmp, const uint32_t* __restrict__ na = nullptr)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= (na ? *na : n)) return;
     tmp[starts[key[i]] + slot[i]] = i;
@@ -436,6 +446,7 @@ __device__ __forceinline__ void store_half_abs(uint4* __restrict__ posh, uint32_
 template <typename R>
 __global__ void k_boundary_half(Boundary<R> b, GridView g, double h, uint4* __restrict__ posh)
 {
+    grid_wait();
     const uint32_t d = gtid();
     if (d < b.n) store_half_abs(posh, d, b.pos[d], b.cell[d], g, h);
 }
@@ -449,6 +460,7 @@ __global__ void k_gather_fluid(uint32_t n, const uint32_t* __restrict__ tmp, con
                                const uint32_t* __restrict__ starts, Fluid<R> src, Fluid<R> dst,
                                uint4* __restrict__ posh = nullptr, GridView g = GridView{}, double h = 0.0)
 {
+    grid_wait();
     const uint32_t p = gtid();
     if (p >= src.count()) return;
     uint32_t i;
@@ -475,6 +487,7 @@ template <typename R>
 __global__ void k_gather_boundary(uint32_t n, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ key,
                                   const uint32_t* __restrict__ starts, Boundary<R> src, Boundary<R> dst)
 {
+    grid_wait();
     const uint32_t p = gtid();
     if (p >= n) return;
     uint32_t i;
@@ -494,6 +507,7 @@ __global__ void k_gather_boundary(uint32_t n, const uint32_t* __restrict__ tmp, 
 template <typename R>
 __global__ void k_boundary_psi(Boundary<R> b, GridView g, const uint32_t* __restrict__ bstarts, Consts<R> c)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= b.n) return;
     const P4<R> pi = b.pos[i];
@@ -687,6 +701,7 @@ __global__ void __launch_bounds__(kBlock) k_density_cand(Fluid<R> f, const P4<R>
                                                          uint32_t* __restrict__ cnt, uint32_t* __restrict__ bcnt,
                                                          uint32_t kmax)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     const uint32_t n = f.n;
@@ -735,6 +750,7 @@ __global__ void __launch_bounds__(kBlock) k_density(Fluid<R> f, const P4<R>* __r
                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                     Consts<R> c, int akinci)
 {
+    grid_wait();
     const uint32_t t = gtid();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
@@ -812,6 +828,7 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_pressure_force(Fluid<R> f, con
                                                                  Consts<R> c, int akinci, const R* __restrict__ bdp,
                                                                  CandLists L)
 {
+    grid_wait();
     __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
@@ -886,6 +903,7 @@ template <typename R, int G, bool LISTS>
 __global__ void __launch_bounds__(kBlock) k_st_normals(Fluid<R> f, GridView g, const uint32_t* __restrict__ cs, Consts<R> c,
                                                        CandLists L)
 {
+    grid_wait();
     __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
@@ -1024,6 +1042,7 @@ __global__ void __launch_bounds__(kBlock) k_npforce(Fluid<R> f, const P4<R>* __r
                                                     Consts<R> c, int akinci, const DevScalars* __restrict__ scr,
                                                     CandLists L)
 {
+    grid_wait();
     __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
     const uint32_t t = gtid();
@@ -1050,6 +1069,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_dfsph_cfl(Fluid<R> f, Consts<R> c, DevScalars* sc, LoopLimits lim,
                                                    double* partials)
 {
+    grid_wait();
     __shared__ R sh[33];
     const uint32_t i = gtid();
     const R dt = (R)sc->dt;
@@ -1082,6 +1102,7 @@ __global__ void __launch_bounds__(256) k_dfsph_cfl(Fluid<R> f, Consts<R> c, DevS
 template <typename R>
 __global__ void k_dfsph_predict_v_warm(Fluid<R> f, Consts<R> c, const DevScalars* __restrict__ sc)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     const R dt = (R)sc->dt;
@@ -1110,6 +1131,7 @@ __global__ void __launch_bounds__(kBlock) k_dfsph_correct(Fluid<R> f, const P4<R
                                                           const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                           Consts<R> c, int akinci, const DevScalars* __restrict__ sc)
 {
+    grid_wait();
     if (MODE != 0 && !sc->active) return;
     const uint32_t t = gtid();
     const uint32_t i = t / G;
@@ -1159,6 +1181,7 @@ __global__ void __launch_bounds__(kBlock) k_dfsph_predict_density(Fluid<R> f, co
                                                                   Consts<R> c, int akinci, DevScalars* sc, LoopLimits lim,
                                                                   double* partials, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     __shared__ double sh[33];
     if (!INITIAL && !sc->active) return;
     const uint32_t t = gtid();
@@ -1228,6 +1251,7 @@ __global__ void __launch_bounds__(kBlock) k_dfsph_divergence(Fluid<R> f, const P
                                                              Consts<R> c, int akinci, DevScalars* sc, LoopLimits lim,
                                                              double* partials, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     __shared__ double sh[33];
     if (!INITIAL && !sc->active) return;
     const uint32_t t = gtid();
@@ -1335,6 +1359,7 @@ __device__ __forceinline__ void cube_clamp(P4<R>& p, P4<R>& v, uint32_t cell, co
 template <typename R>
 __global__ void k_dfsph_cube(Fluid<R> f, GridView g, double h, Consts<R> c)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     P4<R> p = f.pos[i], v = f.vel[i];
@@ -1349,6 +1374,7 @@ __global__ void k_dfsph_cube(Fluid<R> f, GridView g, double h, Consts<R> c)
 template <typename R, bool PCI>
 __global__ void k_integrate(Fluid<R> f, GridView g, double h, Consts<R> c, const DevScalars* __restrict__ sc)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     const R dt = (R)sc->dt;
@@ -1375,6 +1401,7 @@ __global__ void k_integrate(Fluid<R> f, GridView g, double h, Consts<R> c, const
 template <typename R>
 __global__ void k_pcisph_init(Fluid<R> f)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     f.press[i] = 0;
@@ -1385,6 +1412,7 @@ __global__ void k_pcisph_init(Fluid<R> f)
 // previous step's maximum density error is tested, as the reference does.
 static __global__ void k_pcisph_loop_begin(DevScalars* sc, LoopLimits lim, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     sc->iterations = 0;
     sc->disp_bits = 0u;
     sc->active = ((sc->maxDensityError > lim.maxError) || (0u < lim.minIt)) && (0u < lim.maxIt);
@@ -1397,6 +1425,7 @@ static __global__ void k_pcisph_loop_begin(DevScalars* sc, LoopLimits lim, cudaG
 template <typename R, bool TRACK = false>
 __global__ void k_pcisph_predict(Fluid<R> f, Consts<R> c, DevScalars* __restrict__ sc)
 {
+    grid_wait();
     if (!sc->active) return;
     const uint32_t i = gtid();
     float d = 0.f;
@@ -1439,6 +1468,7 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_density_pressure(Fluid<R> f, 
                                                                     Consts<R> c, int akinci, DevScalars* sc, LoopLimits lim,
                                                                     double* partials, CandLists L, float margin)
 {
+    grid_wait();
     __shared__ R sh[33];
     __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (!sc->active) return;
@@ -1501,6 +1531,7 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_pressure_acc(Fluid<R> f, cons
                                                                 Consts<R> c, int akinci, const DevScalars* __restrict__ sc,
                                                                 const R* __restrict__ bdp, CandLists L)
 {
+    grid_wait();
     __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (!sc->active) return;
     if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
@@ -1553,6 +1584,7 @@ template <typename R, int MODE>
 __global__ void k_bh_boundary(Boundary<R> b, Fluid<R> f, GridView g, const uint32_t* __restrict__ cs,
                               const uint32_t* __restrict__ bs, Consts<R> c, const DevScalars* __restrict__ sc)
 {
+    grid_wait();
     if (MODE == 2 && !sc->active) return;
     const uint32_t i = gtid();
     if (i >= b.n) return;
@@ -1588,11 +1620,13 @@ __global__ void k_bh_boundary(Boundary<R> b, Fluid<R> f, GridView g, const uint3
 }
 
 // One more grid build (cell lifetimes of the PCISPH boundary model).
-static __global__ void k_bh_epoch(DevScalars* sc) { sc->grid_epoch += 1; }
+static __global__ void k_bh_epoch(DevScalars* sc) {
+    grid_wait(); sc->grid_epoch += 1; }
 
 // Cells holding boundary points exist from the first build on.
 static __global__ void k_bh_mark_cells(uint32_t n, const uint32_t* __restrict__ key, uint32_t* __restrict__ cell_epoch)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i < n) atomicMin(cell_epoch + key[i], 1u);
 }
@@ -1601,6 +1635,7 @@ static __global__ void k_bh_mark_cells(uint32_t n, const uint32_t* __restrict__ 
 template <typename R>
 __global__ void k_bh_zero_pressure(Boundary<R> b)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= b.n) return;
     b.press[i] = 0;
@@ -1619,6 +1654,7 @@ template <typename R, int MODE>
 __global__ void k_bh_collide(Fluid<R> f, Boundary<R> b, GridView g, const uint32_t* __restrict__ bs, Consts<R> c,
                              const DevScalars* __restrict__ sc, uint32_t* __restrict__ cell_epoch)
 {
+    grid_wait();
     if (MODE == 2 && !sc->active) return;
     const uint32_t i = gtid();
     if (i >= f.count()) return;
@@ -1685,6 +1721,7 @@ __global__ void k_bh_collide(Fluid<R> f, Boundary<R> b, GridView g, const uint32
 template <typename R, bool PRED>
 __global__ void k_bh_correct_velocities(Fluid<R> f, Consts<R> c)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     const V3<R> ni = xyz(f.normal[i]);
@@ -1703,6 +1740,7 @@ __global__ void k_bh_correct_velocities(Fluid<R> f, Consts<R> c)
 template <typename R>
 __global__ void k_bh_upload(const double* __restrict__ nrm, uint32_t n, Boundary<R> b, R mass)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= n) return;
     b.nrm[i] = P4<R>{(R)nrm[3 * i], (R)nrm[3 * i + 1], (R)nrm[3 * i + 2], 0};
@@ -1713,6 +1751,7 @@ __global__ void k_bh_upload(const double* __restrict__ nrm, uint32_t n, Boundary
 // loop test for the next one.
 static __global__ void k_pcisph_loop_next(DevScalars* sc, LoopLimits lim, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     if (!sc->active) return;
     const unsigned it = ++sc->iterations;
     sc->active = sc->next_active;
@@ -1727,6 +1766,7 @@ static __global__ void k_pcisph_loop_next(DevScalars* sc, LoopLimits lim, cudaGr
 static __global__ void k_list_stats(uint32_t n, const uint32_t* __restrict__ count, uint32_t kmax,
                                     unsigned long long* out)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t c = count[i];
@@ -1784,6 +1824,7 @@ __global__ void __launch_bounds__(256) k_emit(Fluid<R> f, EmitterDev* __restrict
                                               GridView g, double h, double gx, double gy, double gz, DevScalars* sc,
                                               uint32_t* __restrict__ na, unsigned flags)
 {
+    grid_wait();
     __shared__ uint32_t base[kMaxEmitters];
     __shared__ double toff[kMaxEmitters];
     __shared__ int any;
@@ -1842,6 +1883,7 @@ __global__ void __launch_bounds__(256) k_emit(Fluid<R> f, EmitterDev* __restrict
 // next emission at the current time.
 static __global__ void k_emit_pause(EmitterDev* __restrict__ em, int nem, uint32_t pause, const DevScalars* __restrict__ sc)
 {
+    grid_wait();
     const int e = (int)threadIdx.x;
     if (e < nem) {
         em[e].pause = pause;
@@ -1852,6 +1894,7 @@ static __global__ void k_emit_pause(EmitterDev* __restrict__ em, int nem, uint32
 // Simulation::step bookkeeping: time += dt, steps++ (DFSPHSolver.cpp:111).
 static __global__ void k_finish_step(DevScalars* sc)
 {
+    grid_wait();
     sc->time = sc->time + sc->dt;
     sc->steps += 1;
 }
@@ -1869,6 +1912,7 @@ __global__ void k_neighbors(Fluid<R> f, const P4<R>* __restrict__ bpos, const ui
                             int* __restrict__ bcnt, int* __restrict__ nbr, int* __restrict__ bnbr, int* __restrict__ cells,
                             int* __restrict__ rank)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     const uint32_t me = f.id[i];

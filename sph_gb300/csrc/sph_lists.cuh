@@ -467,6 +467,7 @@ __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<
                                                            Consts<R> c, int akinci, Lists<R> L, DevScalars* sc,
                                                            LoopLimits lim, double* partials, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     __shared__ uint32_t q[kQueue * kBlock];
     const uint32_t i = gtid();
     constexpr int EB = sizeof(R) == 4 ? 4 : 2;
@@ -602,6 +603,7 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
                                                                  Consts<R> c, int akinci, Lists<R> L, DevScalars* sc,
                                                                  LoopLimits lim, double* partials, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     static_assert(W == 8 || W == 4, "a lane per sum, or two sums a lane");
     constexpr bool FAST = sizeof(R) == 4;
     constexpr uint32_t GROUPS = kWideBlock / W;
@@ -938,6 +940,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_correct_list(Fluid<R> f, co
                                                                   Consts<R> c, int akinci, const DevScalars* __restrict__ sc,
                                                                   Lists<R> L)
 {
+    grid_wait();
     if (MODE != 0 && !sc->active) return;
     const uint32_t i = gtid();
     if (i >= f.count()) return;
@@ -991,6 +994,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_predict_density_list(Fluid<
                                                                        double* partials, cudaGraphConditionalHandle cond,
                                                                        Lists<R> L)
 {
+    grid_wait();
     __shared__ double sh[33];
     if (!INITIAL && !sc->active) return;
     const uint32_t i = gtid();
@@ -1039,6 +1043,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f,
                                                                   double* partials, cudaGraphConditionalHandle cond,
                                                                   Lists<R> L)
 {
+    grid_wait();
     __shared__ double sh[33];
     if (!sc->active) return;
     const uint32_t i = gtid();
@@ -1064,6 +1069,7 @@ template <typename R>
 __global__ void k_pair_lists(uint32_t n, uint32_t base, uint32_t stride, const uint32_t* __restrict__ id, Lists<R> L,
                              const int* __restrict__ off, int* __restrict__ cnt, int* __restrict__ nbr)
 {
+    grid_wait();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const uint32_t i = base + t;
@@ -1128,6 +1134,7 @@ cudaError_t dump_pair_lists(uint32_t n, uint32_t kmax, cudaStream_t st, Launch&&
 template <typename R>
 __global__ void k_dfsph_predict_v_warm_list(Fluid<R> f, Consts<R> c, const DevScalars* __restrict__ sc, R* __restrict__ kbuf)
 {
+    grid_wait();
     const uint32_t i = gtid();
     if (i >= f.count()) return;
     const R dt = (R)sc->dt;

@@ -121,6 +121,7 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* __restrict__ ba
 constexpr int kBoxBlocks = 64;
 __global__ void __launch_bounds__(256) k_point_box(const double* __restrict__ p, uint32_t n, double* __restrict__ part)
 {
+    grid_wait();
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const double x = p[3 * (size_t)i], y = p[3 * (size_t)i + 1], z = p[3 * (size_t)i + 2];
@@ -151,6 +152,7 @@ __global__ void __launch_bounds__(256) k_point_box(const double* __restrict__ p,
 // Scene id of every particle of a layout: segments [base[s], base[s] + len[s]).
 __global__ void k_fill_sid(uint32_t N, const uint32_t* __restrict__ base, uint32_t S, uint32_t* __restrict__ sid)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N) sid[i] = find_segment(base, S, i);
 }
@@ -160,6 +162,7 @@ __global__ void k_fill_sid(uint32_t N, const uint32_t* __restrict__ base, uint32
 __global__ void k_repack_fluid(uint32_t N, const uint32_t* __restrict__ dst_base, const uint32_t* __restrict__ src_base,
                                const uint32_t* __restrict__ len, uint32_t S, Fluid<float> src, Fluid<float> dst)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N || S == 0) return;
     const uint32_t k = find_segment(dst_base, S, i);
@@ -178,6 +181,7 @@ __global__ void k_repack_fluid(uint32_t N, const uint32_t* __restrict__ dst_base
 __global__ void k_repack_boundary(uint32_t N, const uint32_t* __restrict__ dst_base, const uint32_t* __restrict__ src_base,
                                   const uint32_t* __restrict__ len, uint32_t S, Boundary<float> src, Boundary<float> dst)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N || S == 0) return;
     const uint32_t k = find_segment(dst_base, S, i);
@@ -195,6 +199,7 @@ template <bool MOVE>
 __global__ void k_pool_cell_update(uint32_t N, Fluid<float> f, const uint32_t* __restrict__ sid, PoolScene* T,
                                    uint32_t* __restrict__ key, uint32_t* __restrict__ slot, uint32_t* __restrict__ count)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     PoolScene& sd = T[sid[i]];
@@ -229,6 +234,7 @@ __global__ void k_pool_cell_update(uint32_t N, Fluid<float> f, const uint32_t* _
 __global__ void k_pool_bcount(uint32_t N, Boundary<float> b, const uint32_t* __restrict__ bsid, const PoolScene* T,
                               uint32_t* __restrict__ key, uint32_t* __restrict__ slot, uint32_t* __restrict__ count)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const PoolScene& sd = T[bsid[i]];
@@ -245,6 +251,7 @@ __global__ void k_pool_bcount(uint32_t N, Boundary<float> b, const uint32_t* __r
 __global__ void k_pool_boundary_half(uint32_t N, Boundary<float> b, const uint32_t* __restrict__ bsid, const PoolScene* T,
                                      uint4* __restrict__ posh)
 {
+    grid_wait();
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= N) return;
     const float h = T[bsid[d]].c.h;
@@ -256,6 +263,7 @@ __global__ void k_pool_boundary_half(uint32_t N, Boundary<float> b, const uint32
 __global__ void k_pool_psi(uint32_t N, Boundary<float> b, const uint32_t* __restrict__ bsid, const PoolScene* T,
                            const uint32_t* __restrict__ bstarts)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const PoolScene& sd = T[bsid[i]];
@@ -283,6 +291,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_build_lists(Fluid<float> f
                                                                          const uint32_t* __restrict__ bs, Lists<float> L,
                                                                          uint32_t qdepth)
 {
+    grid_wait();
     extern __shared__ uint32_t q[];
     const uint32_t i = blockIdx.x * BLOCK + threadIdx.x;
     uint32_t s = ~0u;
@@ -319,6 +328,7 @@ constexpr int kPoolForces = F_XSPH | F_STD_VISC | F_ART_VISC | F_SURFACE_TENSION
 __global__ void __launch_bounds__(kBlock) k_pool_st_normals(Fluid<float> f, const uint32_t* __restrict__ sid,
                                                             const PoolScene* T, const uint32_t* __restrict__ cs)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f.n) return;
     const PoolScene& sd = T[sid[i]];
@@ -334,6 +344,7 @@ __global__ void __launch_bounds__(kBlock) k_pool_npforce(Fluid<float> f, const P
                                                          const uint32_t* __restrict__ sid, const PoolScene* T,
                                                          const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f.n) return;
     const PoolScene& sd = T[sid[i]];
@@ -353,6 +364,7 @@ __global__ void k_pool_count_work(Fluid<float> f, const P4<float>* __restrict__ 
                                   const PoolScene* T, const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                   unsigned long long* out)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long w[4] = {0ull, 0ull, 0ull, 0ull};
     if (i < f.n) {
@@ -382,6 +394,7 @@ __global__ void k_pool_count_work(Fluid<float> f, const P4<float>* __restrict__ 
 // DFSPHSolver::updateTimeStep per scene: max of sqrt(|v + (a + g) dt|).
 __global__ void k_pool_cfl_accum(Fluid<float> f, const uint32_t* __restrict__ sid, PoolScene* T)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t s = ~0u;
     float m = 0.f;
@@ -408,6 +421,7 @@ __global__ void k_pool_cfl_accum(Fluid<float> f, const uint32_t* __restrict__ si
 
 __global__ void k_pool_cfl_control(PoolScene* T, uint32_t S)
 {
+    grid_wait();
     for (uint32_t k = threadIdx.x; k < S; k += blockDim.x) {
         PoolScene& sd = T[k];
         if (!sd.running) continue;
@@ -429,6 +443,7 @@ __global__ void k_pool_cfl_control(PoolScene* T, uint32_t S)
 __global__ void k_pool_predict_v_warm(Fluid<float> f, const uint32_t* __restrict__ sid, const PoolScene* T,
                                       float* __restrict__ kbuf)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f.n) return;
     const PoolScene& sd = T[sid[i]];
@@ -452,6 +467,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_correct(Fluid<float> f, co
                                                             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                             Lists<float> L)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= f.n) return;
     const PoolScene& sd = T[sid[i]];
@@ -469,6 +485,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_errors(Fluid<float> f, con
                                                            const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                            Lists<float> L)
 {
+    grid_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t s = ~0u;
     unsigned long long contrib = 0ull;
@@ -512,6 +529,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_errors(Fluid<float> f, con
 template <int PHASE>
 __global__ void k_pool_control(PoolScene* T, uint32_t S, PoolCounters* pc, cudaGraphConditionalHandle cond)
 {
+    grid_wait();
     unsigned any = 0;
     for (uint32_t k = threadIdx.x; k < S; k += blockDim.x) {
         PoolScene& sd = T[k];
@@ -579,11 +597,13 @@ __global__ void k_pool_control(PoolScene* T, uint32_t S, PoolCounters* pc, cudaG
 // Each scene's running flag, for a poll that copies S bytes.
 __global__ void k_pool_running(const PoolScene* __restrict__ T, uint32_t S, uint8_t* __restrict__ out)
 {
+    grid_wait();
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < S; k += gridDim.x * blockDim.x) out[k] = T[k].running ? 1 : 0;
 }
 
 __global__ void k_pool_finish(PoolScene* T, uint32_t S)
 {
+    grid_wait();
     for (uint32_t k = threadIdx.x; k < S; k += blockDim.x) {
         PoolScene& sd = T[k];
         if (!sd.running) continue;
@@ -1435,15 +1455,15 @@ private:
         const unsigned per = (unsigned)tune_.scan_per;
         const unsigned nt = blocks(K_, kScanThreads * per);
         run("k_scan_tiles", [&] {
-            if (per == 4) k_scan_tiles<4><<<nt, kScanThreads, 0, ls_>>>(K_, count_.p, out, tile_sums_.p);
-            else if (per == 16) k_scan_tiles<16><<<nt, kScanThreads, 0, ls_>>>(K_, count_.p, out, tile_sums_.p);
-            else k_scan_tiles<8><<<nt, kScanThreads, 0, ls_>>>(K_, count_.p, out, tile_sums_.p);
+            if (per == 4) launch(k_scan_tiles<4>, nt, kScanThreads, 0, K_, count_.p, out, tile_sums_.p);
+            else if (per == 16) launch(k_scan_tiles<16>, nt, kScanThreads, 0, K_, count_.p, out, tile_sums_.p);
+            else launch(k_scan_tiles<8>, nt, kScanThreads, 0, K_, count_.p, out, tile_sums_.p);
         });
-        run("k_scan_tile_sums", [&] { k_scan_tile_sums<<<1, 1024, 0, ls_>>>(nt, tile_sums_.p, out, K_); });
+        run("k_scan_tile_sums", [&] { launch(k_scan_tile_sums, 1, 1024, 0, nt, tile_sums_.p, out, K_); });
         run("k_scan_add", [&] {
-            if (per == 4) k_scan_add<4><<<nt, kScanThreads, 0, ls_>>>(K_, tile_sums_.p, out);
-            else if (per == 16) k_scan_add<16><<<nt, kScanThreads, 0, ls_>>>(K_, tile_sums_.p, out);
-            else k_scan_add<8><<<nt, kScanThreads, 0, ls_>>>(K_, tile_sums_.p, out);
+            if (per == 4) launch(k_scan_add<4>, nt, kScanThreads, 0, K_, tile_sums_.p, out);
+            else if (per == 16) launch(k_scan_add<16>, nt, kScanThreads, 0, K_, tile_sums_.p, out);
+            else launch(k_scan_add<8>, nt, kScanThreads, 0, K_, tile_sums_.p, out);
         });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1458,7 +1478,7 @@ private:
         const uint32_t qd = (uint32_t)tune_.queue;
         const size_t smem = (size_t)qd * (size_t)bb * sizeof(uint32_t);
 #define SPH_BUILD(BL, MB) \
-    k_pool_build_lists<BL, MB, DIV0><<<blocks(N_, BL), BL, smem, ls_>>>(f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L, qd)
+    launch(k_pool_build_lists<BL, MB, DIV0>, blocks(N_, BL), BL, smem, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L, qd)
         if (bb == 128 && bo == 896) SPH_BUILD(128, 7);
         else if (bb == 128) SPH_BUILD(128, 8);
         else if (bo == 1024) SPH_BUILD(256, 4);
@@ -1469,7 +1489,7 @@ private:
     {
         const int sb = tune_.solver_block, so = tune_.solver_occ;
 #define SPH_CORR(BL, MB) \
-    k_pool_correct<BL, MB, MODE><<<blocks(N_, BL), BL, 0, ls_>>>(f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
+    launch(k_pool_correct<BL, MB, MODE>, blocks(N_, BL), BL, 0, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
         if (sb == 128) { if (so == 1536) SPH_CORR(128, 12); else if (so == 2048) SPH_CORR(128, 16); else SPH_CORR(128, 8); }
         else { if (so == 1536) SPH_CORR(256, 6); else if (so == 2048) SPH_CORR(256, 8); else SPH_CORR(256, 4); }
 #undef SPH_CORR
@@ -1478,7 +1498,7 @@ private:
     {
         const int sb = tune_.solver_block, so = tune_.solver_occ;
 #define SPH_ERRS(BL, MB) \
-    k_pool_errors<BL, MB, DIV, INITIAL><<<blocks(N_, BL), BL, 0, ls_>>>(f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
+    launch(k_pool_errors<BL, MB, DIV, INITIAL>, blocks(N_, BL), BL, 0, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
         if (sb == 128) { if (so == 1536) SPH_ERRS(128, 12); else if (so == 2048) SPH_ERRS(128, 16); else SPH_ERRS(128, 8); }
         else { if (so == 1536) SPH_ERRS(256, 6); else if (so == 2048) SPH_ERRS(256, 8); else SPH_ERRS(256, 4); }
 #undef SPH_ERRS
@@ -1494,6 +1514,7 @@ private:
         if (tuning_) tune_family(name, &fam, &sub);
         const bool prof = prof_ && counting_;
         if (fam < 0 && !prof) { fn(); return; }
+        chained_ = false;
         cudaEvent_t a = take_event(), b = take_event();
         cudaEvent_t c = prof && fam >= 0 ? take_event() : nullptr, d = c ? take_event() : nullptr;
         cudaEventRecord(a, ls_);
@@ -1501,9 +1522,15 @@ private:
         fn();
         if (d) cudaEventRecord(d, ls_);
         cudaEventRecord(b, ls_);
+        chained_ = false;
         if (fam >= 0) tpending_.push_back({fam, sub, a, b});
         else pending_.push_back({name, a, b});
         if (c) pending_.push_back({name, c, d});
+    }
+    template <typename... P, typename... A> void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, A&&... args)
+    {
+        launch_kernel(kernel, grid, block, smem, ls_, chained_, std::forward<A>(args)...);
+        chained_ = true;
     }
     cudaEvent_t take_event()
     {
@@ -1717,15 +1744,15 @@ private:
     {
         Fluid<float> a = F(cur_);
         if (move)
-            run("k_pool_cell_update", [&] { k_pool_cell_update<true><<<blocks(N_, 256), 256, 0, ls_>>>(N_, a, sid_.p, table_.p, key_.p, slot_.p, count_.p); });
+            run("k_pool_cell_update", [&] { launch(k_pool_cell_update<true>, blocks(N_, 256), 256, 0, N_, a, sid_.p, table_.p, key_.p, slot_.p, count_.p); });
         else
-            run("k_pool_cell_update", [&] { k_pool_cell_update<false><<<blocks(N_, 256), 256, 0, ls_>>>(N_, a, sid_.p, table_.p, key_.p, slot_.p, count_.p); });
+            run("k_pool_cell_update", [&] { launch(k_pool_cell_update<false>, blocks(N_, 256), 256, 0, N_, a, sid_.p, table_.p, key_.p, slot_.p, count_.p); });
         SPH_CUDA(cudaGetLastError());
         int rc = scan(starts_.p);
         if (rc) return rc;
-        run("k_scatter", [&] { k_scatter<<<blocks(N_, 256), 256, 0, ls_>>>(N_, key_.p, slot_.p, starts_.p, tmp_.p); });
-        run("k_gather_fluid", [&] { k_gather_fluid<float><<<blocks(N_, 256), 256, 0, ls_>>>(N_, tmp_.p, key_.p, starts_.p, F(cur_), F(1 - cur_),
-                                                                                          posh_.p); });
+        run("k_scatter", [&] { launch(k_scatter, blocks(N_, 256), 256, 0, N_, key_.p, slot_.p, starts_.p, tmp_.p, nullptr); });
+        run("k_gather_fluid", [&] { launch(k_gather_fluid<float>, blocks(N_, 256), 256, 0, N_, tmp_.p, key_.p, starts_.p, F(cur_), F(1 - cur_),
+                                                                                          posh_.p, GridView{}, 0.0); });
         SPH_CUDA(cudaGetLastError());
         cur_ = 1 - cur_;
         return SPH_OK;
@@ -1756,7 +1783,9 @@ private:
             SPH_CUDA(cudaStreamBeginCaptureToGraph(st2_, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
             ls_ = st2_;
             loop_ctx_ = loop_id;
+            chained_ = false;
             body(h);
+            chained_ = false;
             loop_ctx_ = 0;
             ls_ = st_;
             cudaGraph_t out;
@@ -1768,6 +1797,7 @@ private:
         for (unsigned it = 0; it < 1000u; ++it) {
             SPH_CUDA(cudaMemcpyAsync(h_pc_, pc_.p, sizeof(PoolCounters), cudaMemcpyDeviceToHost, st_));
             SPH_CUDA(cudaStreamSynchronize(st_));
+            chained_ = false;
             if (!h_pc_->any) break;
             if (loop_id == 1) ++host_body_d_; else ++host_body_v_;
             body((cudaGraphConditionalHandle)0);
@@ -1781,6 +1811,7 @@ private:
     {
         const unsigned nb = blocks(N_, kBlock);
         const unsigned nb256 = blocks(N_, 256);
+        chained_ = false;
         {
             Fluid<float> f = F(cur_);
             const P4<float>* bp = bpos_[bcur_].p;
@@ -1788,13 +1819,13 @@ private:
             if (any_st_ || any_forces_) {
                 auto ph = phase("npForces");
                 if (any_st_)
-                    run("k_pool_st_normals", [&] { k_pool_st_normals<<<nb, kBlock, 0, ls_>>>(f, sid_.p, table_.p, starts_.p); });
+                    run("k_pool_st_normals", [&] { launch(k_pool_st_normals, nb, kBlock, 0, f, sid_.p, table_.p, starts_.p); });
                 if (any_forces_)
-                    run("k_pool_npforce", [&] { k_pool_npforce<<<nb, kBlock, 0, ls_>>>(f, bp, sid_.p, table_.p, starts_.p, bstarts_.p); });
+                    run("k_pool_npforce", [&] { launch(k_pool_npforce, nb, kBlock, 0, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p); });
             }
-            run("k_pool_cfl_accum", [&] { k_pool_cfl_accum<<<nb256, 256, 0, ls_>>>(f, sid_.p, table_.p); });
-            run("k_pool_cfl_control", [&] { k_pool_cfl_control<<<1, 256, 0, ls_>>>(table_.p, S_); });
-            run("k_pool_predict_v_warm", [&] { k_pool_predict_v_warm<<<nb256, 256, 0, ls_>>>(f, sid_.p, table_.p, L.kbuf); });
+            run("k_pool_cfl_accum", [&] { launch(k_pool_cfl_accum, nb256, 256, 0, f, sid_.p, table_.p); });
+            run("k_pool_cfl_control", [&] { launch(k_pool_cfl_control, 1, 256, 0, table_.p, S_); });
+            run("k_pool_predict_v_warm", [&] { launch(k_pool_predict_v_warm, nb256, 256, 0, f, sid_.p, table_.p, L.kbuf); });
             auto ph = phase("Density solver");
             run("k_pool_correct", [&] { launch_correct<0>(f, bp, L); });
             SPH_CUDA(cudaGetLastError());
@@ -1802,12 +1833,12 @@ private:
                 1,
                 [&](cudaGraphConditionalHandle h) {
                     run("k_pool_errors_density", [&] { launch_errors<false, true>(f, bp, L); });
-                    run("k_pool_control", [&] { k_pool_control<0><<<1, 256, 0, ls_>>>(table_.p, S_, pc_.p, h); });
+                    run("k_pool_control", [&] { launch(k_pool_control<0>, 1, 256, 0, table_.p, S_, pc_.p, h); });
                 },
                 [&](cudaGraphConditionalHandle h) {
                     run("k_pool_correct", [&] { launch_correct<1>(f, bp, L); });
                     run("k_pool_errors_density", [&] { launch_errors<false, false>(f, bp, L); });
-                    run("k_pool_control", [&] { k_pool_control<1><<<1, 256, 0, ls_>>>(table_.p, S_, pc_.p, h); });
+                    run("k_pool_control", [&] { launch(k_pool_control<1>, 1, 256, 0, table_.p, S_, pc_.p, h); });
                 });
             if (rc) return rc;
         }
@@ -1831,16 +1862,16 @@ private:
             rc = solve_loop(
                 2,
                 [&](cudaGraphConditionalHandle h) {
-                    run("k_pool_control", [&] { k_pool_control<2><<<1, 256, 0, ls_>>>(table_.p, S_, pc_.p, h); });
+                    run("k_pool_control", [&] { launch(k_pool_control<2>, 1, 256, 0, table_.p, S_, pc_.p, h); });
                 },
                 [&](cudaGraphConditionalHandle h) {
                     run("k_pool_correct", [&] { launch_correct<2>(f, bp, L); });
                     run("k_pool_errors_div", [&] { launch_errors<true, false>(f, bp, L); });
-                    run("k_pool_control", [&] { k_pool_control<3><<<1, 256, 0, ls_>>>(table_.p, S_, pc_.p, h); });
+                    run("k_pool_control", [&] { launch(k_pool_control<3>, 1, 256, 0, table_.p, S_, pc_.p, h); });
                 });
             if (rc) return rc;
         }
-        run("k_pool_finish", [&] { k_pool_finish<<<1, 256, 0, ls_>>>(table_.p, S_); });
+        run("k_pool_finish", [&] { launch(k_pool_finish, 1, 256, 0, table_.p, S_); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1911,6 +1942,7 @@ private:
     std::vector<PoolEntry*> order_;
     int next_id_ = 1;
     bool dirty_ = false, graph_ = false, capturing_ = false;
+    bool chained_ = false;  // the last operation on ls_ is a launch of this step (launch_kernel)
     uint32_t S_ = 0, N_ = 0, NB_ = 0, K_ = 0, kmax_ = 64;
     int cur_ = 0, bcur_ = 0;
     int loop_ctx_ = 0;

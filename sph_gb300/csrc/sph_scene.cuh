@@ -20,6 +20,7 @@
 #include <optional>
 #include <string>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "sph_scene_base.h"
@@ -1040,9 +1041,9 @@ private:
     int scan(uint32_t* out)
     {
         const unsigned nt = blocks(nkeys_, kScanTile);
-        run("k_scan_tiles", [&] { k_scan_tiles<<<nt, kScanThreads, 0, ls_>>>(nkeys_, count_.p, out, tile_sums_.p); });
-        run("k_scan_tile_sums", [&] { k_scan_tile_sums<<<1, 1024, 0, ls_>>>(nt, tile_sums_.p, out, nkeys_); });
-        run("k_scan_add", [&] { k_scan_add<<<nt, kScanThreads, 0, ls_>>>(nkeys_, tile_sums_.p, out); });
+        run("k_scan_tiles", [&] { launch(k_scan_tiles<>, nt, kScanThreads, 0, nkeys_, count_.p, out, tile_sums_.p); });
+        run("k_scan_tile_sums", [&] { launch(k_scan_tile_sums, 1, 1024, 0, nt, tile_sums_.p, out, nkeys_); });
+        run("k_scan_add", [&] { launch(k_scan_add<>, nt, kScanThreads, 0, nkeys_, tile_sums_.p, out); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1054,18 +1055,18 @@ private:
     {
         Fluid<R> a = F();
         uint32_t* ce = bh_ ? cell_epoch_.p : nullptr;
-        if (bh_) run("k_bh_epoch", [&] { k_bh_epoch<<<1, 1, 0, ls_>>>(sc_.p); });
+        if (bh_) run("k_bh_epoch", [&] { launch(k_bh_epoch, 1, 1, 0, sc_.p); });
         if (move)
-            run("k_cell_update", [&] { k_cell_update<R, true><<<blocks(n_, 256), 256, 0, ls_>>>(n_, a.pos, a.vel, a.cell, key_.p, slot_.p, count_.p, gv_,
+            run("k_cell_update", [&] { launch(k_cell_update<R, true>, blocks(n_, 256), 256, 0, n_, a.pos, a.vel, a.cell, key_.p, slot_.p, count_.p, gv_,
                                                                      c_.h, hd_, sc_.p, ce, nullptr, a.na); });
         else
-            run("k_cell_update", [&] { k_cell_update<R, false><<<blocks(n_, 256), 256, 0, ls_>>>(n_, a.pos, a.vel, a.cell, key_.p, slot_.p, count_.p,
+            run("k_cell_update", [&] { launch(k_cell_update<R, false>, blocks(n_, 256), 256, 0, n_, a.pos, a.vel, a.cell, key_.p, slot_.p, count_.p,
                                                                       gv_, c_.h, hd_, sc_.p, ce, nullptr, a.na); });
         SPH_CUDA(cudaGetLastError());
         int rc = scan(starts_.p);
         if (rc) return rc;
-        run("k_scatter", [&] { k_scatter<<<blocks(n_, 256), 256, 0, ls_>>>(n_, key_.p, slot_.p, starts_.p, tmp_.p, a.na); });
-        run("k_gather_fluid", [&] { k_gather_fluid<R><<<blocks(n_, 256), 256, 0, ls_>>>(n_, tmp_.p, key_.p, starts_.p, fl_[cur_], fl_[1 - cur_],
+        run("k_scatter", [&] { launch(k_scatter, blocks(n_, 256), 256, 0, n_, key_.p, slot_.p, starts_.p, tmp_.p, a.na); });
+        run("k_gather_fluid", [&] { launch(k_gather_fluid<R>, blocks(n_, 256), 256, 0, n_, tmp_.p, key_.p, starts_.p, fl_[cur_], fl_[1 - cur_],
                                                                                   posh_.p, gv_, hd_); });
         SPH_CUDA(cudaGetLastError());
         cur_ = 1 - cur_;
@@ -1096,11 +1097,11 @@ private:
         withG([&](auto gt) {
             constexpr int G = decltype(gt)::value;
             if (alpha)
-                run("k_density", [&] { k_density<R, G, true, false><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_); });
+                run("k_density", [&] { launch(k_density<R, G, true, false>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_); });
             else if (eos)
-                run("k_density", [&] { k_density<R, G, false, true><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_); });
+                run("k_density", [&] { launch(k_density<R, G, false, true>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_); });
             else
-                run("k_density", [&] { k_density<R, G, false, false><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_); });
+                run("k_density", [&] { launch(k_density<R, G, false, false>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_); });
         });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1113,7 +1114,7 @@ private:
         const R reach = c_.h + cand_margin();
         // never below the passes' own cull, which has some slack over h
         const R reach2 = std::max(reach * reach, c_.cull2);
-        run("k_density_cand", [&] { k_density_cand<R, EOS><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(
+        run("k_density_cand", [&] { launch(k_density_cand<R, EOS>, blocks(n_, kBlock), kBlock, 0, 
             f, bd_[1].pos, gv_, starts_.p, bstarts_.p, c_, akinci_, reach2, cand_.p, candn_.p, candb_.p, ckmax_); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1144,14 +1145,14 @@ private:
         Lists<R> L = LS();
         auto wide = [&](auto wt) {
             constexpr int W = decltype(wt)::value;
-            run("k_build_lists", [&] { k_build_lists_wide<R, W, DIV0><<<blocks((size_t)n_ * W, kWideBlock), kWideBlock, 0, ls_>>>(
+            run("k_build_lists", [&] { launch(k_build_lists_wide<R, W, DIV0>, blocks((size_t)n_ * W, kWideBlock), kWideBlock, 0, 
                 f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
         };
         const int W = build_lanes();
         if (W == 8) wide(std::integral_constant<int, 8>{});
         else if (W == 4) wide(std::integral_constant<int, 4>{});
         else
-            run("k_build_lists", [&] { k_build_lists<R, DIV0><<<blocks(n_, kBlock), kBlock, 0, ls_>>>(
+            run("k_build_lists", [&] { launch(k_build_lists<R, DIV0>, blocks(n_, kBlock), kBlock, 0, 
                 f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1166,9 +1167,9 @@ private:
         Fluid<R> f = F();
         Boundary<R> b = B(1);
         const unsigned nbk = blocks(nb_, 128);
-        if (mode == 0) run("k_bh_boundary", [&] { k_bh_boundary<R, 0><<<nbk, 128, 0, ls_>>>(b, f, gv_, starts_.p, bstarts_.p, c_, sc_.p); });
-        else if (mode == 1) run("k_bh_boundary", [&] { k_bh_boundary<R, 1><<<nbk, 128, 0, ls_>>>(b, f, gv_, starts_.p, bstarts_.p, c_, sc_.p); });
-        else run("k_bh_boundary", [&] { k_bh_boundary<R, 2><<<nbk, 128, 0, ls_>>>(b, f, gv_, starts_.p, bstarts_.p, c_, sc_.p); });
+        if (mode == 0) run("k_bh_boundary", [&] { launch(k_bh_boundary<R, 0>, nbk, 128, 0, b, f, gv_, starts_.p, bstarts_.p, c_, sc_.p); });
+        else if (mode == 1) run("k_bh_boundary", [&] { launch(k_bh_boundary<R, 1>, nbk, 128, 0, b, f, gv_, starts_.p, bstarts_.p, c_, sc_.p); });
+        else run("k_bh_boundary", [&] { launch(k_bh_boundary<R, 2>, nbk, 128, 0, b, f, gv_, starts_.p, bstarts_.p, c_, sc_.p); });
     }
     // Positions and cells after the integration (and MOVE: after the DFSPH
     // position update), then PCISPHBoundaryModel::correctPositions (MODE 0 /
@@ -1178,17 +1179,17 @@ private:
         Fluid<R> f = F();
         // PCISPH: the predicted positions move into the new cell frames too
         P4<R>* carry = MODE == 1 ? f.predR : nullptr;
-        run("k_cell_update", [&] { k_cell_update<R, MOVE, false><<<blocks(n_, 256), 256, 0, ls_>>>(n_, f.pos, f.vel, f.cell, key_.p, slot_.p,
+        run("k_cell_update", [&] { launch(k_cell_update<R, MOVE, false>, blocks(n_, 256), 256, 0, n_, f.pos, f.vel, f.cell, key_.p, slot_.p,
                                                                                              count_.p, gv_, c_.h, hd_, sc_.p, nullptr,
                                                                                              carry, f.na); });
-        run("k_bh_collide", [&] { k_bh_collide<R, MODE><<<blocks(n_, 128), 128, 0, ls_>>>(f, B(1), gv_, bstarts_.p, c_, sc_.p,
+        run("k_bh_collide", [&] { launch(k_bh_collide<R, MODE>, blocks(n_, 128), 128, 0, f, B(1), gv_, bstarts_.p, c_, sc_.p,
                                                                                           cell_epoch_.p); });
-        if (VEL) run("k_bh_correct_velocities", [&] { k_bh_correct_velocities<R, PRED><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_); });
+        if (VEL) run("k_bh_correct_velocities", [&] { launch(k_bh_correct_velocities<R, PRED>, blocks(n_, 256), 256, 0, f, c_); });
     }
     // DFSPHSolver::step :51-57: correctVelocities after predictVelocities.
     void launch_bh_velocities()
     {
-        if (bh_) run("k_bh_correct_velocities", [&] { k_bh_correct_velocities<R, false><<<blocks(n_, 256), 256, 0, ls_>>>(F(), c_); });
+        if (bh_) run("k_bh_correct_velocities", [&] { launch(k_bh_correct_velocities<R, false>, blocks(n_, 256), 256, 0, F(), c_); });
     }
     // updatePositions, then (PCISPH boundary model) correctPositions
     // DFSPHSolver.cpp:65-75, then the grid build.
@@ -1203,7 +1204,7 @@ private:
             launch_bh_after_move<true, 0, false, false>();
         } else {
             Fluid<R> f = F();
-            run("k_cell_update", [&] { k_cell_update<R, true, false><<<blocks(n_, 256), 256, 0, ls_>>>(n_, f.pos, f.vel, f.cell, key_.p, slot_.p,
+            run("k_cell_update", [&] { launch(k_cell_update<R, true, false>, blocks(n_, 256), 256, 0, n_, f.pos, f.vel, f.cell, key_.p, slot_.p,
                                                                                               count_.p, gv_, c_.h, hd_, sc_.p, nullptr,
                                                                                               nullptr, f.na); });
         }
@@ -1218,7 +1219,7 @@ private:
         if (!nem_) return;
         const unsigned flags = (d.simulation_method == SPH_PCISPH ? EMIT_PCISPH : 0u) | (normal_.n >= n_ ? EMIT_NORMALS : 0u);
         Fluid<R> f = F();
-        run("k_emit", [&] { k_emit<R><<<1, 256, 0, ls_>>>(f, em_.p, nem_, egroup_.p, gv_, hd_, d.gravity[0], d.gravity[1],
+        run("k_emit", [&] { launch(k_emit<R>, 1, 256, 0, f, em_.p, nem_, egroup_.p, gv_, hd_, d.gravity[0], d.gravity[1],
                                                           d.gravity[2], sc_.p, &sc_.p->n_active, flags); });
     }
 
@@ -1279,21 +1280,21 @@ private:
             Fluid<R> f = F();
             const P4<R>* bp = bd_[1].pos;
             Lists<R> L = LS();
-            run("k_dfsph_cfl", [&] { k_dfsph_cfl<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_, sc_.p, lim_, partials_.p); });
-            run("k_dfsph_predict_v_warm", [&] { k_dfsph_predict_v_warm_list<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_, sc_.p, L.kbuf); });
+            run("k_dfsph_cfl", [&] { launch(k_dfsph_cfl<R>, blocks(n_, 256), 256, 0, f, c_, sc_.p, lim_, partials_.p); });
+            run("k_dfsph_predict_v_warm", [&] { launch(k_dfsph_predict_v_warm_list<R>, blocks(n_, 256), 256, 0, f, c_, sc_.p, L.kbuf); });
             launch_bh_velocities();
             auto ph = phase("Density solver");
-            run("k_dfsph_correct_list", [&] { k_dfsph_correct_list<R, 0><<<nb, kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
+            run("k_dfsph_correct_list", [&] { launch(k_dfsph_correct_list<R, 0>, nb, kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
             SPH_CUDA(cudaGetLastError());
             // correctDensityError DFSPHSolver.cpp:311-406
             rc = solve_loop(1,
                 [&](cudaGraphConditionalHandle h) {
-                    run("k_dfsph_predict_density_list", [&] { k_dfsph_predict_density_list<R, true><<<nb, kBlock, 0, ls_>>>(
+                    run("k_dfsph_predict_density_list", [&] { launch(k_dfsph_predict_density_list<R, true>, nb, kBlock, 0, 
                         f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
                 },
                 [&](cudaGraphConditionalHandle h) {
-                    run("k_dfsph_correct_list", [&] { k_dfsph_correct_list<R, 1><<<nb, kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
-                    run("k_dfsph_predict_density_list", [&] { k_dfsph_predict_density_list<R, false><<<nb, kBlock, 0, ls_>>>(
+                    run("k_dfsph_correct_list", [&] { launch(k_dfsph_correct_list<R, 1>, nb, kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
+                    run("k_dfsph_predict_density_list", [&] { launch(k_dfsph_predict_density_list<R, false>, nb, kBlock, 0, 
                         f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
                 },
                 lim_.minIt, lim_.maxIt);
@@ -1318,8 +1319,8 @@ private:
                     solver.emplace(phases_, "Divergence solver", ls_, capturing_, prof_);
                 },
                 [&](cudaGraphConditionalHandle h) {
-                    run("k_dfsph_correct_list", [&] { k_dfsph_correct_list<R, 2><<<nb, kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
-                    run("k_dfsph_divergence_list", [&] { k_dfsph_divergence_list<R><<<nb, kBlock, 0, ls_>>>(
+                    run("k_dfsph_correct_list", [&] { launch(k_dfsph_correct_list<R, 2>, nb, kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
+                    run("k_dfsph_divergence_list", [&] { launch(k_dfsph_divergence_list<R>, nb, kBlock, 0, 
                         f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
                 },
                 lim_.minItV, lim_.maxIt);
@@ -1328,9 +1329,9 @@ private:
         if (c_.has_cube) {
             Fluid<R> f = F();
             auto ph = phase("Boundary handling");
-            run("k_dfsph_cube", [&] { k_dfsph_cube<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, gv_, hd_, c_); });
+            run("k_dfsph_cube", [&] { launch(k_dfsph_cube<R>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_); });
         }
-        run("k_finish_step", [&] { k_finish_step<<<1, 1, 0, ls_>>>(sc_.p); });
+        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1346,8 +1347,8 @@ private:
             constexpr bool LISTS = decltype(lt)::value;
             const CandLists L = CL();
             if (c_.force_flags & F_SURFACE_TENSION)
-                run("k_st_normals", [&] { k_st_normals<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, gv_, starts_.p, c_, L); });
-            run("k_npforce", [&] { k_npforce<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
+                run("k_st_normals", [&] { launch(k_st_normals<R, G, LISTS>, wblocks(), kBlock, 0, f, gv_, starts_.p, c_, L); });
+            run("k_npforce", [&] { launch(k_npforce<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
         });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1382,7 +1383,9 @@ private:
             SPH_CUDA(cudaStreamBeginCaptureToGraph(st2_, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
             ls_ = st2_;
             loop_ctx_ = loop_id;
+            chained_ = false;
             body(h);
+            chained_ = false;
             loop_ctx_ = 0;
             ls_ = st_;
             cudaGraph_t out;
@@ -1401,6 +1404,7 @@ private:
             launched += batch;
             SPH_CUDA(cudaMemcpyAsync(&h_sc_->active, &sc_.p->active, sizeof(unsigned), cudaMemcpyDeviceToHost, st_));
             SPH_CUDA(cudaStreamSynchronize(st_));
+            chained_ = false;
             if (!h_sc_->active) break;
         }
         return SPH_OK;
@@ -1415,11 +1419,18 @@ private:
         if (capturing_) { ++cap_count_[loop_ctx_]; fn(); return; }
         ++launches_;
         if (!prof_) { fn(); return; }
+        chained_ = false;
         cudaEvent_t a = take_event(), b = take_event();
         cudaEventRecord(a, ls_);
         fn();
         cudaEventRecord(b, ls_);
+        chained_ = false;
         pending_.push_back({name, a, b});
+    }
+    template <typename... P, typename... A> void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, A&&... args)
+    {
+        launch_kernel(kernel, grid, block, smem, ls_, chained_, std::forward<A>(args)...);
+        chained_ = true;
     }
     cudaEvent_t take_event()
     {
@@ -1440,15 +1451,15 @@ private:
         if (rc) return rc;
         {
             Fluid<R> f = F();
-            run("k_dfsph_cfl", [&] { k_dfsph_cfl<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_, sc_.p, lim_, partials_.p); });
-            run("k_dfsph_predict_v_warm", [&] { k_dfsph_predict_v_warm<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_, sc_.p); });
+            run("k_dfsph_cfl", [&] { launch(k_dfsph_cfl<R>, blocks(n_, 256), 256, 0, f, c_, sc_.p, lim_, partials_.p); });
+            run("k_dfsph_predict_v_warm", [&] { launch(k_dfsph_predict_v_warm<R>, blocks(n_, 256), 256, 0, f, c_, sc_.p); });
             SPH_CUDA(cudaGetLastError());
             launch_bh_velocities();
             const P4<R>* bp = bd_[1].pos;
             auto ph = phase("Density solver");
             withG([&](auto gt) {
                 constexpr int G = decltype(gt)::value;
-                run("k_dfsph_correct", [&] { k_dfsph_correct<R, G, 0><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p); });
+                run("k_dfsph_correct", [&] { launch(k_dfsph_correct<R, G, 0>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p); });
             });
             SPH_CUDA(cudaGetLastError());
             // correctDensityError DFSPHSolver.cpp:311-406
@@ -1456,16 +1467,16 @@ private:
                 [&](cudaGraphConditionalHandle h) {
                     withG([&](auto gt) {
                         constexpr int G = decltype(gt)::value;
-                        run("k_dfsph_predict_density", [&] { k_dfsph_predict_density<R, G, true><<<wblocks(), kBlock, 0, ls_>>>(
+                        run("k_dfsph_predict_density", [&] { launch(k_dfsph_predict_density<R, G, true>, wblocks(), kBlock, 0, 
                             f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h); });
                     });
                 },
                 [&](cudaGraphConditionalHandle h) {
                     withG([&](auto gt) {
                         constexpr int G = decltype(gt)::value;
-                        run("k_dfsph_correct", [&] { k_dfsph_correct<R, G, 1><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
+                        run("k_dfsph_correct", [&] { launch(k_dfsph_correct<R, G, 1>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
                                                                                  sc_.p); });
-                        run("k_dfsph_predict_density", [&] { k_dfsph_predict_density<R, G, false><<<wblocks(), kBlock, 0, ls_>>>(
+                        run("k_dfsph_predict_density", [&] { launch(k_dfsph_predict_density<R, G, false>, wblocks(), kBlock, 0, 
                             f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h); });
                     });
                 },
@@ -1489,16 +1500,16 @@ private:
                 [&](cudaGraphConditionalHandle h) {
                     withG([&](auto gt) {
                         constexpr int G = decltype(gt)::value;
-                        run("k_dfsph_divergence", [&] { k_dfsph_divergence<R, G, true><<<wblocks(), kBlock, 0, ls_>>>(
+                        run("k_dfsph_divergence", [&] { launch(k_dfsph_divergence<R, G, true>, wblocks(), kBlock, 0, 
                             f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h); });
                     });
                 },
                 [&](cudaGraphConditionalHandle h) {
                     withG([&](auto gt) {
                         constexpr int G = decltype(gt)::value;
-                        run("k_dfsph_correct", [&] { k_dfsph_correct<R, G, 2><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
+                        run("k_dfsph_correct", [&] { launch(k_dfsph_correct<R, G, 2>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
                                                                                  sc_.p); });
-                        run("k_dfsph_divergence", [&] { k_dfsph_divergence<R, G, false><<<wblocks(), kBlock, 0, ls_>>>(
+                        run("k_dfsph_divergence", [&] { launch(k_dfsph_divergence<R, G, false>, wblocks(), kBlock, 0, 
                             f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h); });
                     });
                 },
@@ -1508,9 +1519,9 @@ private:
         if (c_.has_cube) {
             Fluid<R> f = F();
             auto ph = phase("Boundary handling");
-            run("k_dfsph_cube", [&] { k_dfsph_cube<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, gv_, hd_, c_); });
+            run("k_dfsph_cube", [&] { launch(k_dfsph_cube<R>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_); });
         }
-        run("k_finish_step", [&] { k_finish_step<<<1, 1, 0, ls_>>>(sc_.p); });
+        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1538,7 +1549,7 @@ private:
             withGL([&](auto gt, auto lt) {
                 constexpr int G = decltype(gt)::value;
                 constexpr bool LISTS = decltype(lt)::value;
-                run("k_wcsph_pressure_force", [&] { k_wcsph_pressure_force<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, dp, CL()); });
+                run("k_wcsph_pressure_force", [&] { launch(k_wcsph_pressure_force<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, dp, CL()); });
             });
             SPH_CUDA(cudaGetLastError());
         }
@@ -1549,14 +1560,14 @@ private:
         if (rc) return rc;
         {
             auto ph = phase("Integratio");
-            run("k_integrate", [&] { k_integrate<R, false><<<blocks(n_, 256), 256, 0, ls_>>>(f, gv_, hd_, c_, sc_.p); });
+            run("k_integrate", [&] { launch(k_integrate<R, false>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p); });
         }
         if (bh_) {
             auto ph = phase("Boundary Handling");
             launch_bh_after_move<false, 0, true, false>();  // WCSPHSolver.cpp:62-72
         }
         launch_emit();  // WCSPHSolver.cpp:75
-        run("k_finish_step", [&] { k_finish_step<<<1, 1, 0, ls_>>>(sc_.p); });
+        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1591,50 +1602,51 @@ private:
         const R* dp = bdp();
         {
             auto ph = phase("Pressure solver");
-            run("k_pcisph_init", [&] { k_pcisph_init<R><<<blocks(n_, 256), 256, 0, ls_>>>(f); });
-            if (bh_ && nb_) run("k_bh_zero_pressure", [&] { k_bh_zero_pressure<R><<<blocks(nb_, 256), 256, 0, ls_>>>(B(1)); });
+            run("k_pcisph_init", [&] { launch(k_pcisph_init<R>, blocks(n_, 256), 256, 0, f); });
+            if (bh_ && nb_) run("k_bh_zero_pressure", [&] { launch(k_bh_zero_pressure<R>, blocks(nb_, 256), 256, 0, B(1)); });
             rc = solve_loop(1,
-                [&](cudaGraphConditionalHandle h) { run("k_pcisph_loop_begin", [&] { k_pcisph_loop_begin<<<1, 1, 0, ls_>>>(sc_.p, lim_, h); }); },
+                [&](cudaGraphConditionalHandle h) { run("k_pcisph_loop_begin", [&] { launch(k_pcisph_loop_begin, 1, 1, 0, sc_.p, lim_, h); }); },
                 [&](cudaGraphConditionalHandle h) {
                     if (cands_)
-                    run("k_pcisph_predict", [&] { k_pcisph_predict<R, true><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_, sc_.p); });
+                    run("k_pcisph_predict", [&] { launch(k_pcisph_predict<R, true>, blocks(n_, 256), 256, 0, f, c_, sc_.p); });
                 else
-                    run("k_pcisph_predict", [&] { k_pcisph_predict<R><<<blocks(n_, 256), 256, 0, ls_>>>(f, c_, sc_.p); });
+                    run("k_pcisph_predict", [&] { launch(k_pcisph_predict<R>, blocks(n_, 256), 256, 0, f, c_, sc_.p); });
                     if (bh_)  // correctPredPositions PCISPHSolver.cpp:367-377
-                        run("k_bh_collide", [&] { k_bh_collide<R, 2><<<blocks(n_, 128), 128, 0, ls_>>>(f, B(1), gv_, bstarts_.p, c_, sc_.p,
+                        run("k_bh_collide", [&] { launch(k_bh_collide<R, 2>, blocks(n_, 128), 128, 0, f, B(1), gv_, bstarts_.p, c_, sc_.p,
                                                                                                   cell_epoch_.p); });
                     withGL([&](auto gt, auto lt) {
                         constexpr int G = decltype(gt)::value;
                         constexpr bool LISTS = decltype(lt)::value;
                         const CandLists L = CL();
                         const float margin = (float)cand_margin();
-                        run("k_pcisph_density_pressure", [&] { k_pcisph_density_pressure<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_,
+                        run("k_pcisph_density_pressure", [&] { launch(k_pcisph_density_pressure<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_,
                                                                                        hasb_, sc_.p, lim_, partials_.p, L, margin); });
                         launch_bh_boundary(2);
-                        run("k_pcisph_pressure_acc", [&] { k_pcisph_pressure_acc<R, G, LISTS><<<wblocks(), kBlock, 0, ls_>>>(f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
+                        run("k_pcisph_pressure_acc", [&] { launch(k_pcisph_pressure_acc<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_,
                                                                                    sc_.p, dp, L); });
                     });
-                    run("k_pcisph_loop_next", [&] { k_pcisph_loop_next<<<1, 1, 0, ls_>>>(sc_.p, lim_, h); });
+                    run("k_pcisph_loop_next", [&] { launch(k_pcisph_loop_next, 1, 1, 0, sc_.p, lim_, h); });
                 },
                 lim_.minIt, lim_.maxIt);
         }
         if (rc) return rc;
         {
             auto ph = phase("Integration");
-            run("k_integrate", [&] { k_integrate<R, true><<<blocks(n_, 256), 256, 0, ls_>>>(f, gv_, hd_, c_, sc_.p); });
+            run("k_integrate", [&] { launch(k_integrate<R, true>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p); });
         }
         if (bh_) {
             auto ph = phase("Boundary handling");
             launch_bh_after_move<false, 1, true, true>();  // PCISPHSolver.cpp:65-75
         }
         launch_emit();  // PCISPHSolver.cpp:78
-        run("k_finish_step", [&] { k_finish_step<<<1, 1, 0, ls_>>>(sc_.p); });
+        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
 
     int one_step()
     {
+        chained_ = false;
         switch (d.simulation_method) {
             case SPH_WCSPH: return wcsph_step();
             case SPH_PCISPH: return pcisph_step();
@@ -1691,6 +1703,7 @@ private:
     uint32_t nkeys_ = 0;
     int cur_ = 0;
     bool graph_ = false, capturing_ = false;
+    bool chained_ = false;  // the last operation on ls_ is a launch of this step (launch_kernel)
     cudaGraphExec_t gexec_[2] = {nullptr, nullptr};
     int loop_ctx_ = 0;
     unsigned cap_count_[3] = {0, 0, 0};
