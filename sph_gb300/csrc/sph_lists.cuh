@@ -216,10 +216,11 @@ __device__ __noinline__ BuildSums<R> build_walk_all(uint32_t i, const Fluid<R>& 
 
 // The dot product of the velocity divergence terms with its rounding written
 // out (FP32: the contraction the compiler chose for the pass over the lists
-// first), so that the sum the build forms and the passes' agree bit for bit.
-template <typename R> __device__ __forceinline__ R dot3_div(V3<R> a, V3<R> b)
+// first), so that the sums of the one-scene build and of its passes agree bit
+// for bit.  The pool's kernels (POOL) keep the compiler's contraction of each.
+template <bool POOL = false, typename R> __device__ __forceinline__ R dot3_div(V3<R> a, V3<R> b)
 {
-    if constexpr (sizeof(R) == 8) return dot3(a, b);
+    if constexpr (sizeof(R) == 8 || POOL) return dot3(a, b);
     else return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
 }
 
@@ -231,7 +232,7 @@ __device__ __noinline__ DivSum<R> velocity_div_cells(const Fluid<R>& f, const P4
                                                      const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                      const Consts<R>& c, int akinci, uint32_t i, V3<R> vi);
 
-template <typename R>
+template <typename R, bool POOL = false>
 __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint32_t i, V3<R> vi, uint32_t cnt)
 {
     const uint32_t n = f.n;
@@ -240,7 +241,7 @@ __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint3
         const P4<R> pr = L.pairs[(size_t)k * n + i];
         const uint32_t j = as_idx(pr.w);
         if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-        dv += dot3_div(vi - xyz(f.vel[j]), xyz(pr));
+        dv += dot3_div<POOL>(vi - xyz(f.vel[j]), xyz(pr));
     }
     return dv;
 }
@@ -254,7 +255,7 @@ __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint3
 // the finished lists (same terms, same order), into *div0, with the count of
 // neighbours into *nn0 (a particle whose list or queue overflowed takes the
 // same list or cell walk as velocity_div_one).
-template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1>
+template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1, bool POOL = false>
 __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                                 const GridView& g, const uint32_t* __restrict__ cs,
                                                 const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
@@ -289,7 +290,7 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             }
             if (cnt < L.kmax) L.pairs[(size_t)cnt * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j)};
             ++cnt;
-            if constexpr (DIV0) dv += dot3_div(vi - vj, mg);
+            if constexpr (DIV0) dv += dot3_div<POOL>(vi - vj, mg);
         }
     };
     // phase 1: cull.  The half-precision cull needs all 27 cells inside the
@@ -407,8 +408,8 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             *div0 = d.dv;
             *nn0 = d.nn;
         } else {
-            if (nq > qcap) dv = reread_div<R>(f, L, i, vi, cnt);
-            if (akinci) dv += dot3_div(vi, bg);
+            if (nq > qcap) dv = reread_div<R, POOL>(f, L, i, vi, cnt);
+            if (akinci) dv += dot3_div<POOL>(vi, bg);
             *div0 = dv;
             *nn0 = cnt;
         }
@@ -949,7 +950,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_correct_list(Fluid<R> f, co
 }
 
 // Sum over the list of m (v_i - v_j) . gradW_ij plus the boundary term.
-template <typename R>
+template <typename R, bool POOL = false>
 __device__ __forceinline__ R velocity_div_list(const Fluid<R>& f, const Lists<R>& L, uint32_t i, V3<R> vi, int akinci)
 {
     const uint32_t n = f.n;
@@ -961,15 +962,15 @@ __device__ __forceinline__ R velocity_div_list(const Fluid<R>& f, const Lists<R>
         const P4<R> q = ldcs4(p + (size_t)k * n);
         const uint32_t j = as_idx(q.w);
         if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-        d += dot3_div(vi - xyz(ldg4(f.vel + j)), xyz(q));
+        d += dot3_div<POOL>(vi - xyz(ldg4(f.vel + j)), xyz(q));
     }
-    if (akinci) d += dot3_div(vi, xyz(L.bgrad[i]));
+    if (akinci) d += dot3_div<POOL>(vi, xyz(L.bgrad[i]));
     return d;
 }
 
 // m (v_i - v_j) . gradW summed over the neighbours (list or fallback walk);
 // *nn receives the number of neighbours with a non-zero gradient.
-template <typename R>
+template <typename R, bool POOL = false>
 __device__ __forceinline__ R velocity_div_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                               const GridView& g, const uint32_t* __restrict__ cs,
                                               const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
@@ -978,7 +979,7 @@ __device__ __forceinline__ R velocity_div_one(uint32_t i, const Fluid<R>& f, con
     const uint32_t cnt = L.count[i];
     if (cnt <= L.kmax) {
         *nn = cnt;
-        return velocity_div_list(f, L, i, vi, akinci);
+        return velocity_div_list<R, POOL>(f, L, i, vi, akinci);
     }
     const DivSum<R> d = velocity_div_cells(f, bpos, g, cs, bs, c, akinci, i, vi);
     *nn = d.nn;

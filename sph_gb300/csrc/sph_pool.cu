@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_build_lists(Fluid<float> f
         if (sd.running) {
             float d = 0.f;
             uint32_t nn = 0;
-            build_lists_one<float, true, DIV0>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c, sd.akinci, L,
+            build_lists_one<float, true, DIV0, 1, true>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c, sd.akinci, L,
                                                q, (uint32_t)BLOCK, qdepth, &d, &nn);
             if constexpr (DIV0) {
                 // the divergence solve's first error pass (k_pool_errors<true,
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_errors(Fluid<float> f, con
             const float dt = (float)sd.s.dt;
             const V3<float> vi = xyz(f.vel[i]);
             uint32_t nn;
-            float d = velocity_div_one(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, c, sd.akinci, L, vi, &nn);
+            float d = velocity_div_one<float, true>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, c, sd.akinci, L, vi, &nn);
             // the particle's relative error in FP32 (FP64 arithmetic is slow on
             // this part); its fixed-point quantum 2^-28 is still far coarser
             // than the FP32 rounding of an error of order 1e-3
