@@ -38,7 +38,7 @@ UNITS = {
     "sph_mesh.cpp": [],
     "sph_serve.cpp": [],
 }
-HEADERS = ["sph_device.cuh", "sph_kernels.cuh", "sph_lists.cuh", "sph_scene.cuh", "sph_scene_base.h", "sph_ctx.h",
+HEADERS = ["sph_device.cuh", "sph_kernels.cuh", "sph_lists.cuh", "sph_cand.cuh", "sph_scene.cuh", "sph_scene_base.h", "sph_ctx.h",
            "sph_phase.cuh"]
 VARIANTS = {"": ([], OBJDIR, LIB),
             "checked": (["-DSPH_BOUNDS_CHECK"], OBJDIR + "_checked", os.path.join(LIBDIR, "libsph_gb300_checked.so"))}

@@ -1,0 +1,236 @@
+// The density passes that build the PCISPH / WCSPH candidate lists (CandLists,
+// sph_kernels.cuh), and WCSPH's force pass over them.
+//
+// Like the DFSPH list build, candidates are culled from the half-precision
+// positions into a queue in shared memory and evaluated from it: a walk that
+// evaluates as it goes runs the kernel's arithmetic with one lane in five
+// active and waits for each candidate's load in turn (90k particles: 78 us,
+// 45 us here), and in FP64 fills the two FP64 lanes of an SM with distance
+// tests.
+#pragma once
+
+#include "sph_lists.cuh"
+
+namespace sph {
+
+struct CandOut {
+    uint32_t* idx;
+    uint32_t* cnt;
+    uint32_t* bcnt;
+    uint32_t kmax;
+    const uint4* posh;       // half-precision positions (fluid, boundary or nullptr)
+    const uint4* bposh;
+    const uint32_t* bcell;
+};
+
+// cell offset code of a candidate in cell cj around cell ci (walk_reach's)
+__device__ __forceinline__ uint32_t cell_code(uint32_t ci, uint32_t cj)
+{
+    return (uint32_t)((cell_x(cj) - cell_x(ci) + 1) * 9 + (cell_y(cj) - cell_y(ci) + 1) * 3 + (cell_z(cj) - cell_z(ci) + 1));
+}
+
+template <typename R> struct CandSums {
+    R density;
+    uint32_t m;
+};
+
+// A particle the half-precision cull does not serve, or whose queue
+// overflowed: the walk, out of line.  Boundary points (BND) carry their weight.
+template <typename R, bool BND>
+__device__ __noinline__ CandSums<R> cand_walk(uint32_t i, uint32_t n, const P4<R>* __restrict__ pos, const GridView& g,
+                                              const uint32_t* __restrict__ starts, const Consts<R>& c, uint32_t pc, V3<R> xi,
+                                              R reach2, uint32_t* idx, uint32_t kmax, uint32_t first, R density)
+{
+    uint32_t m = 0;
+    walk_reach<R>(g, starts, pc, xi, c.h, reach2, [&](uint32_t j, V3<R> s, uint32_t code) {
+        const P4<R> p = ldg4(pos + j);
+        const V3<R> r = s - xyz(p);
+        const R r2 = dot3(r, r);
+        if (r2 <= reach2) {
+            if (first + m < kmax) idx[(size_t)(first + m) * n + i] = j | (code << kCandIdxBits);
+            ++m;
+        }
+        if (r2 <= c.cull2) density += (BND ? p.w : c.mass) * cubic_W(c, sqrt(r2));
+    });
+    return CandSums<R>{density, m};
+}
+
+// WCSPH's equation of state (WCSPHSolver::computeFluidPressures
+// WCSPHSolver.cpp:80-95) and p / rho^2 for the pressure-force pass.
+template <typename R> __device__ __forceinline__ void cand_eos(uint32_t i, const Fluid<R>& f, const Consts<R>& c, V3<R> xi, R density)
+{
+    const R p = fmax((R)0, c.k_eos * (pow(density / c.density0, c.gamma) - (R)1));
+    f.press[i] = p;
+    f.xk[i] = P4<R>{xi.x, xi.y, xi.z, p / (density * density)};
+}
+
+// Densities (SPHSolver::computeFluidDensities SPHSolver.cpp:44-91, as
+// k_density<R, 1, false, EOS>, EOS: with WCSPH's equation of state) fused
+// with the candidate lists' build, one lane per particle: the terms and their
+// order are the cell walk's.
+template <typename R, bool EOS>
+__global__ void __launch_bounds__(kBlock, 7) k_density_cand(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
+                                                            const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
+                                                            Consts<R> c, int akinci, R reach2, CandOut o)
+{
+    grid_wait();
+    __shared__ uint32_t q[kQueue * kBlock];
+    constexpr int EB = kListBatch<R>;
+    const uint32_t i = gtid();
+    if (i >= f.count()) return;
+    const uint32_t n = f.n;
+    const V3<R> xi = xyz(f.pos[i]);
+    const uint32_t pc = f.cell[i];
+    V3<float> xr;
+    const bool half = half_cull_ok(g, pc, xi, c.h, &xr);
+    R density = 0;
+    uint32_t m = 0;
+    uint32_t nq = kQueue + 1u;
+    if (half) nq = cull_half(g, cs, pc, xr, (float)c.h, (float)reach2, o.posh, q, kBlock, kQueue);
+    if (nq <= kQueue) {
+        for (uint32_t k = 0; k < nq; k += EB) {
+            uint32_t j[EB], cj[EB];
+            P4<R> pj[EB];
+#pragma unroll
+            for (int b = 0; b < EB; ++b) {
+                j[b] = q[(k + b < nq ? k + b : nq - 1) * kBlock + threadIdx.x];
+                pj[b] = ldg4(f.pos + j[b]);
+                cj[b] = __ldg(f.cell + j[b]);
+            }
+#pragma unroll
+            for (int b = 0; b < EB; ++b) {
+                if (k + b >= nq) break;
+                const V3<R> r = pair_vec(xi, pc, pj[b], cj[b], c.h);
+                const R r2 = dot3(r, r);
+                if (r2 <= reach2) {
+                    if (m < o.kmax) o.idx[(size_t)m * n + i] = j[b] | (cell_code(pc, cj[b]) << kCandIdxBits);
+                    ++m;
+                }
+                if (r2 <= c.cull2) density += c.mass * cubic_W(c, sqrt(r2));
+            }
+        }
+    } else {
+        const CandSums<R> w = cand_walk<R, false>(i, n, f.pos, g, cs, c, pc, xi, reach2, o.idx, o.kmax, 0u, density);
+        density = w.density;
+        m = w.m;
+    }
+    uint32_t mb = 0;
+    if (akinci) {
+        uint32_t nb = kQueue + 1u;
+        if (half) nb = cull_half(g, bs, pc, xr, (float)c.h, (float)reach2, o.bposh, q, kBlock, kQueue);
+        if (nb <= kQueue) {
+            for (uint32_t k = 0; k < nb; k += EB) {
+                uint32_t j[EB], cj[EB];
+                P4<R> pj[EB];
+#pragma unroll
+                for (int b = 0; b < EB; ++b) {
+                    j[b] = q[(k + b < nb ? k + b : nb - 1) * kBlock + threadIdx.x];
+                    pj[b] = ldg4(bpos + j[b]);
+                    cj[b] = __ldg(o.bcell + j[b]);
+                }
+#pragma unroll
+                for (int b = 0; b < EB; ++b) {
+                    if (k + b >= nb) break;
+                    const V3<R> r = pair_vec(xi, pc, pj[b], cj[b], c.h);
+                    const R r2 = dot3(r, r);
+                    if (r2 <= reach2) {
+                        if (m + mb < o.kmax) o.idx[(size_t)(m + mb) * n + i] = j[b] | (cell_code(pc, cj[b]) << kCandIdxBits);
+                        ++mb;
+                    }
+                    if (r2 <= c.cull2) density += pj[b].w * cubic_W(c, sqrt(r2));
+                }
+            }
+        } else {
+            const CandSums<R> w = cand_walk<R, true>(i, n, bpos, g, bs, c, pc, xi, reach2, o.idx, o.kmax, m, density);
+            density = w.density;
+            mb = w.m;
+        }
+    }
+    f.rho[i] = density;
+    f.vel[i].w = density;
+    o.cnt[i] = m;
+    o.bcnt[i] = mb;
+    if (EOS) cand_eos(i, f, c, xi, density);
+}
+
+// The same with W lanes per particle (small scenes): lanes share the cull and
+// the evaluation, the list keeps the walk's order, and each lane's part of the
+// density is added across the lanes.
+template <typename R, int W, bool EOS>
+__global__ void __launch_bounds__(kWideBlock) k_density_cand_wide(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
+                                                                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
+                                                                  Consts<R> c, int akinci, R reach2, CandOut o)
+{
+    grid_wait();
+    constexpr uint32_t GROUPS = kWideBlock / W;
+    __shared__ uint32_t queue[GROUPS][kQueue], bqueue[GROUPS][kQueue];
+    const int gl = (int)(threadIdx.x % W), grp = (int)(threadIdx.x / W);
+    const int g0 = (int)(threadIdx.x & 31) & ~(W - 1);
+    const uint32_t i = (blockIdx.x * kWideBlock + threadIdx.x) / W;
+    const uint32_t n = f.n;
+    const bool valid = i < f.count();
+    V3<R> xi = {0, 0, 0};
+    uint32_t pc = 0;
+    V3<float> xr = {0, 0, 0};
+    bool half = false;
+    if (valid) {
+        xi = xyz(f.pos[i]);
+        pc = f.cell[i];
+        half = half_cull_ok(g, pc, xi, c.h, &xr);
+    }
+    const bool bhalf = half && akinci;
+    const float hf = (float)c.h, rf2 = (float)reach2;
+    const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf, rf2), rb = wide_ranges<W>(bhalf, gl, g, bs, pc, xr, hf, rf2);
+    const uint32_t nq = cull_half_wide<W>(gl, rf, cell_z(pc), xr, hf, rf2, o.posh, queue[grp], kQueue);
+    const uint32_t nb = akinci ? cull_half_wide<W>(gl, rb, cell_z(pc), xr, hf, rf2, o.bposh, bqueue[grp], kQueue) : 0u;
+    __syncwarp();
+    R density = 0;
+    uint32_t m = 0, mb = 0;
+    // queued entries, W a round; the ones within reach are listed in order
+    auto visit = [&](const uint32_t* q, uint32_t ne, const P4<R>* pos, const uint32_t* cell, bool bnd, uint32_t first) -> uint32_t {
+        uint32_t listed = 0;
+        for (uint32_t k = 0; __any_sync(0xffffffffu, k < ne); k += W) {
+            bool near = false;
+            uint32_t entry = 0;
+            if (k + gl < ne) {
+                const uint32_t j = q[k + gl];
+                const P4<R> pj = ldg4(pos + j);
+                const uint32_t cj = __ldg(cell + j);
+                const V3<R> r = pair_vec(xi, pc, pj, cj, c.h);
+                const R r2 = dot3(r, r);
+                near = r2 <= reach2;
+                entry = j | (cell_code(pc, cj) << kCandIdxBits);
+                if (r2 <= c.cull2) density += (bnd ? pj.w : c.mass) * cubic_W(c, sqrt(r2));
+            }
+            const uint32_t b = (__ballot_sync(0xffffffffu, near) >> g0) & ((1u << W) - 1u);
+            const uint32_t at = first + listed + __popc(b & ((1u << gl) - 1u));
+            if (near && at < o.kmax) o.idx[(size_t)at * n + i] = entry;
+            listed += __popc(b);
+        }
+        return listed;
+    };
+    const bool fwalk = valid && (!half || nq > kQueue), bwalk = valid && akinci && (!half || nb > kQueue);
+    m = visit(queue[grp], fwalk ? 0u : nq, f.pos, f.cell, false, 0u);
+    if (fwalk && gl == 0) {
+        const CandSums<R> w = cand_walk<R, false>(i, n, f.pos, g, cs, c, pc, xi, reach2, o.idx, o.kmax, 0u, density);
+        density = w.density;
+        m = w.m;
+    }
+    m = __shfl_sync(0xffffffffu, m, 0, W);
+    if (akinci) mb = visit(bqueue[grp], bwalk ? 0u : nb, bpos, o.bcell, true, m);
+    if (bwalk && gl == 0) {
+        const CandSums<R> w = cand_walk<R, true>(i, n, bpos, g, bs, c, pc, xi, reach2, o.idx, o.kmax, m, density);
+        density = w.density;
+        mb = w.m;
+    }
+    __syncwarp();
+    density = group_sum<W>(density);
+    if (!valid || gl != 0) return;
+    f.rho[i] = density;
+    f.vel[i].w = density;
+    o.cnt[i] = m;
+    o.bcnt[i] = mb;
+    if (EOS) cand_eos(i, f, c, xi, density);
+}
+
+}  // namespace sph

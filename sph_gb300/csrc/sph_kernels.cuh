@@ -523,7 +523,7 @@ __global__ void k_boundary_psi(Boundary<R> b, GridView g, const uint32_t* __rest
 }
 
 // ---------------------------------------------------------------------------
-// PCISPH / WCSPH candidate lists (one lane per particle).  The reference's
+// PCISPH / WCSPH candidate lists.  The reference's
 // PCISPH and WCSPH sums run over the particles of the 27 cells found at the
 // start of the step (HashTable::neighborhoodSearch, HashTable.h:136-170), at
 // the current positions (densities, normals, non-pressure forces, pressure
@@ -536,8 +536,8 @@ __global__ void k_boundary_psi(Boundary<R> b, GridView g, const uint32_t* __rest
 // at the predicted ones while every predicted displacement stays below
 // margin / 2 (checked per loop iteration; otherwise the predicted-density
 // pass walks the cells): its terms are the ones the walks skip, so the sums
-// are the same, bit for bit.  A particle with more than kmax candidates
-// walks the cells.
+// are the same (bit for bit with one lane per particle; G lanes take every
+// G-th entry).  A particle with more than kmax candidates walks the cells.
 constexpr uint32_t kCandIdxBits = 27;
 constexpr uint32_t kCandIdxMask = (1u << kCandIdxBits) - 1u;
 
@@ -612,19 +612,19 @@ __device__ __forceinline__ void fill_shift_table(float4* t, float h)
     __syncthreads();
 }
 
-template <typename R, int B, typename Load, typename Eval>
+template <typename R, int G, int B, typename Load, typename Eval>
 __device__ __forceinline__ void list_visit(const CandLists& L, uint32_t n, uint32_t i, uint32_t first, uint32_t cnt,
-                                           uint32_t nj, V3<R> xi, const float4* shift, Load&& load, Eval&& eval)
+                                           uint32_t nj, V3<R> xi, int lane, const float4* shift, Load&& load, Eval&& eval)
 {
     constexpr bool REL = sizeof(R) == 4;
     const uint32_t* __restrict__ p = L.idx + (size_t)first * n + i;
 #pragma unroll 1
-    for (uint32_t k = 0; k < cnt; k += B) {
+    for (uint32_t k = lane; k < cnt; k += G * B) {
         uint32_t e[B];
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             // past the end: the last entry once more, not evaluated
-            const uint32_t kk = k + b < cnt ? k + b : cnt - 1;
+            const uint32_t kk = k + b * G < cnt ? k + b * G : cnt - 1;
             e[b] = __ldg(p + (size_t)kk * n);
         }
         decltype(load(0u)) q[B];
@@ -632,7 +632,7 @@ __device__ __forceinline__ void list_visit(const CandLists& L, uint32_t n, uint3
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             const uint32_t j = e[b] & kCandIdxMask;
-            ok[b] = k + b < cnt;
+            ok[b] = k + b * G < cnt;
             if (SPH_INDEX_OK(j, nj, L.fault)) q[b] = load(j);
             else ok[b] = false;
         }
@@ -649,28 +649,29 @@ __device__ __forceinline__ void list_visit(const CandLists& L, uint32_t n, uint3
     }
 }
 
-// The cell walk of a particle that has no list, out of line and one column at
-// a time: its registers are not carried by the list loop (64 -> 48 in the
-// predicted-density pass; 490k drop: 108 -> 89 us with the shift table).
-template <typename R, bool TRIM, typename Acc, typename Load, typename Eval>
+// The cell walk of a particle that has no list, out of line and (one lane) one
+// column at a time: its registers are not carried by the list loop (64 -> 48
+// in the predicted-density pass; 490k drop: 108 -> 89 us with the shift table).
+template <typename R, int G, bool TRIM, typename Acc, typename Load, typename Eval>
 __device__ __noinline__ Acc walk_out_of_line(const GridView& g, const uint32_t* __restrict__ starts, uint32_t pc, V3<R> xi,
-                                             R h, Acc acc, Load load, Eval eval)
+                                             R h, int lane, Acc acc, Load load, Eval eval)
 {
-    walk<R, 1, TRIM, true>(g, starts, pc, xi, h, 0, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
+    walk<R, G, TRIM, G == 1>(g, starts, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
     return acc;
 }
 
 // Fluid candidates of particle i at lane LANE of G, summed into acc by
-// eval(acc, load(j), s): LISTS (G = 1): the stored list, or the walk out of
-// line where it did not fit; else the cell walk.
+// eval(acc, load(j), s): LISTS: every G-th entry of the stored list, or the
+// walk out of line where it did not fit; else the cell walk.
 template <typename R, int G, bool LISTS, int B, bool TRIM = true, typename Acc, typename Load, typename Eval>
 __device__ __forceinline__ void fluid_visit(const CandLists& L, uint32_t n, uint32_t i, const GridView& g,
                                             const uint32_t* __restrict__ cs, uint32_t pc, V3<R> xi, R h, int lane,
                                             const float4* shift, Acc& acc, Load load, Eval eval)
 {
     if constexpr (LISTS) {
-        if (L.has(i)) list_visit<R, B>(L, n, i, 0u, L.cnt[i], n, xi, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
-        else acc = walk_out_of_line<R, TRIM>(g, cs, pc, xi, h, acc, load, eval);
+        if (L.has(i))
+            list_visit<R, G, B>(L, n, i, 0u, L.cnt[i], n, xi, lane, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
+        else acc = walk_out_of_line<R, G, TRIM>(g, cs, pc, xi, h, lane, acc, load, eval);
     } else {
         walk<R, G, TRIM>(g, cs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
     }
@@ -684,60 +685,11 @@ __device__ __forceinline__ void boundary_visit(const CandLists& L, uint32_t n, u
 {
     if constexpr (LISTS) {
         if (L.has_boundary(i))
-            list_visit<R, B>(L, n, i, L.cnt[i], L.bcnt[i], L.nb, xi, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
-        else acc = walk_out_of_line<R, true>(g, bs, pc, xi, h, acc, load, eval);
+            list_visit<R, G, B>(L, n, i, L.cnt[i], L.bcnt[i], L.nb, xi, lane, shift, load,
+                                [&](const auto& q, V3<R> s) { eval(acc, q, s); });
+        else acc = walk_out_of_line<R, G, true>(g, bs, pc, xi, h, lane, acc, load, eval);
     } else {
         walk<R, G>(g, bs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
-    }
-}
-
-// Densities (SPHSolver::computeFluidDensities SPHSolver.cpp:44-91, as
-// k_density<R, 1, false, EOS>, EOS: with WCSPH's equation of state) fused
-// with the candidate lists' build.
-template <typename R, bool EOS = false>
-__global__ void __launch_bounds__(kBlock) k_density_cand(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
-                                                         const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
-                                                         Consts<R> c, int akinci, R reach2, uint32_t* __restrict__ idx,
-                                                         uint32_t* __restrict__ cnt, uint32_t* __restrict__ bcnt,
-                                                         uint32_t kmax)
-{
-    grid_wait();
-    const uint32_t i = gtid();
-    if (i >= f.count()) return;
-    const uint32_t n = f.n;
-    const V3<R> xi = xyz(f.pos[i]);
-    const uint32_t pc = f.cell[i];
-    R density = 0;
-    uint32_t m = 0;
-    walk_reach<R>(g, cs, pc, xi, c.h, reach2, [&](uint32_t j, V3<R> s, uint32_t code) {
-        const V3<R> r = s - xyz(ldg4(f.pos + j));
-        const R r2 = dot3(r, r);
-        if (r2 <= reach2) {
-            if (m < kmax) idx[(size_t)m * n + i] = j | (code << kCandIdxBits);
-            ++m;
-        }
-        if (r2 <= c.cull2) density += c.mass * cubic_W(c, sqrt(r2));
-    });
-    uint32_t mb = 0;
-    if (akinci)
-        walk_reach<R>(g, bs, pc, xi, c.h, reach2, [&](uint32_t j, V3<R> s, uint32_t code) {
-            const P4<R> pb = ldg4(bpos + j);
-            const V3<R> r = s - xyz(pb);
-            const R r2 = dot3(r, r);
-            if (r2 <= reach2) {
-                if (m + mb < kmax) idx[(size_t)(m + mb) * n + i] = j | (code << kCandIdxBits);
-                ++mb;
-            }
-            if (r2 <= c.cull2) density += pb.w * cubic_W(c, sqrt(r2));
-        });
-    f.rho[i] = density;
-    f.vel[i].w = density;
-    cnt[i] = m;
-    bcnt[i] = mb;
-    if (EOS) {  // as k_density<R, G, false, true>
-        const R p = fmax((R)0, c.k_eos * (pow(density / c.density0, c.gamma) - (R)1));
-        f.press[i] = p;
-        f.xk[i] = P4<R>{xi.x, xi.y, xi.z, p / (density * density)};
     }
 }
 

@@ -67,10 +67,15 @@ template <typename R> struct Lists {
 // is kept; pairs beyond h evaluate to W = 0, grad W = 0 in phase 2 and are
 // dropped there.  Returns the number of accepted candidates (the queue
 // holds the first qcap).
+//
+// reach2: the square of the distance wanted, up to (1.1 h)^2 (candidate lists;
+// the same bounds scale to 1.9 % of h^2 against a slack of 3.6 %, and a true
+// |dz| above 1.9 h may read as little as h: such candidates are dropped by
+// the exact test on the queued ones).
 __device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 
 __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t* __restrict__ starts, uint32_t pc,
-                                              V3<float> xi, float h, float cull2, const uint4* __restrict__ posh,
+                                              V3<float> xi, float h, float reach2, const uint4* __restrict__ posh,
                                               uint32_t* q, uint32_t qstride, uint32_t qcap)
 {
     const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
@@ -78,8 +83,8 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
     const float gxm = ofx > 0.f ? ofx * ofx : 0.f, gxp = h - ofx > 0.f ? (h - ofx) * (h - ofx) : 0.f;
     const float gym = ofy > 0.f ? ofy * ofy : 0.f, gyp = h - ofy > 0.f ? (h - ofy) * (h - ofy) : 0.f;
     const float gzm = ofz > 0.f ? ofz * ofz : 0.f, gzp = h - ofz > 0.f ? (h - ofz) * (h - ofz) : 0.f;
-    const float lim = h * h * (float)(1.0 + 1e-5);
-    const __half2 thr = __float2half2_rn(cull2 * 1.03f);
+    const float lim = fmaxf(reach2, h * h) * (float)(1.0 + 1e-5);
+    const __half2 thr = __float2half2_rn(reach2 * 1.03f);
     const __half2 zq = __float2half2_rn(zframe3(xi.z, cz, h));
     const __half2 h3 = __float2half2_rn(3.f * h);
     uint32_t nq = 0;
@@ -143,6 +148,20 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
         }
     }
     return nq;
+}
+
+// Whether the half-precision cull serves a particle (see cull_half), and its
+// position in its cell's frame.
+template <typename R>
+__device__ __forceinline__ bool half_cull_ok(const GridView& g, uint32_t pc, V3<R> xi, R h, V3<float>* xr)
+{
+    const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
+    if constexpr (sizeof(R) == 4) *xr = xi;
+    else *xr = V3<float>{(float)(xi.x - (R)(cx + g.ox) * h), (float)(xi.y - (R)(cy + g.oy) * h),
+                         (float)(xi.z - (R)(cz + g.oz) * h)};
+    const float hf = (float)h, hh = 0.5f * hf;
+    return cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
+           fabsf(xr->x - hh) <= hf && fabsf(xr->y - hh) <= hf && fabsf(xr->z - hh) <= hf;
 }
 
 __device__ __forceinline__ float idx_as(float, uint32_t j) { return __uint_as_float(j); }
@@ -517,14 +536,14 @@ template <int W> struct WideRanges {
 };
 template <int W>
 __device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const GridView& g, const uint32_t* __restrict__ starts,
-                                                     uint32_t pc, V3<float> xi, float h)
+                                                     uint32_t pc, V3<float> xi, float h, float reach2)
 {
     const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
     const float ofx = xi.x, ofy = xi.y, ofz = xi.z;
     const float gxm = ofx > 0.f ? ofx * ofx : 0.f, gxp = h - ofx > 0.f ? (h - ofx) * (h - ofx) : 0.f;
     const float gym = ofy > 0.f ? ofy * ofy : 0.f, gyp = h - ofy > 0.f ? (h - ofy) * (h - ofy) : 0.f;
     const float gzm = ofz > 0.f ? ofz * ofz : 0.f, gzp = h - ofz > 0.f ? (h - ofz) * (h - ofz) : 0.f;
-    const float lim = h * h * (float)(1.0 + 1e-5);
+    const float lim = fmaxf(reach2, h * h) * (float)(1.0 + 1e-5);
     WideRanges<W> r;
 #pragma unroll
     for (int t = 0; t < WideRanges<W>::C; ++t) {
@@ -547,10 +566,10 @@ __device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const Grid
 // queue; every lane returns their number.  gl = lane in the group; all lanes
 // of the warp call it.
 template <int W>
-__device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W>& rg, int cz, V3<float> xi, float h, float cull2,
+__device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W>& rg, int cz, V3<float> xi, float h, float reach2,
                                                    const uint4* __restrict__ posh, uint32_t* q, uint32_t qcap)
 {
-    const __half2 thr = __float2half2_rn(cull2 * 1.03f);
+    const __half2 thr = __float2half2_rn(reach2 * 1.03f);
     const __half2 zq = __float2half2_rn(zframe3(xi.z, cz, h));
     const __half2 h3 = __float2half2_rn(3.f * h);
     const int g0 = (int)(threadIdx.x & 31) & ~(W - 1);
@@ -638,7 +657,8 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
                fabsf(xr.x - hh) <= hf && fabsf(xr.y - hh) <= hf && fabsf(xr.z - hh) <= hf;
     }
     const bool bhalf = half && akinci && L.bposh;
-    const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf), rb = wide_ranges<W>(bhalf, gl, g, bs, pc, xr, hf);
+    const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf, (float)c.cull2),
+                        rb = wide_ranges<W>(bhalf, gl, g, bs, pc, xr, hf, (float)c.cull2);
     uint32_t nq = cull_half_wide<W>(gl, rf, cell_z(pc), xr, hf, (float)c.cull2, L.posh, q, qcap);
     uint32_t nb = __any_sync(0xffffffffu, bhalf)
                       ? cull_half_wide<W>(gl, rb, cell_z(pc), xr, hf, (float)c.cull2, L.bposh, bqueue[grp], qcap) : 0u;

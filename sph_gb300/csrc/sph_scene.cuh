@@ -26,6 +26,7 @@
 #include "sph_scene_base.h"
 #include "sph_kernels.cuh"
 #include "sph_lists.cuh"
+#include "sph_cand.cuh"
 #include "sph_phase.cuh"
 
 namespace sph {
@@ -263,8 +264,10 @@ public:
         int G = d.threads_per_particle;
         if (G == 0) {
             // by default enough lanes for ~160k walking threads: a small
-            // scene's walks run out of warps to hide their load latency with
-            // one lane per particle (8,000 WCSPH particles: 2.4x faster at 8)
+            // scene's passes run out of warps to hide their load latency with
+            // one lane per particle (8,000 WCSPH particles: 2.4x faster at 8
+            // over cell walks; 62 -> 36 us/step in FP32 and 495 -> 189 in FP64
+            // with lanes sharing candidate lists instead)
             const unsigned long long n = std::max<unsigned long long>(hx.size() / 3, 1ull);
             const unsigned long long want = (160000ull + n - 1) / n;
             G = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
@@ -356,7 +359,7 @@ public:
             k_gather_boundary<R><<<blocks(nb_, 256), 256, 0, st_>>>(nb_, tmp_.p, key_.p, bstarts_.p, B(0), B(1));
             SPH_CUDA(cudaGetLastError());
             if (akinci_) k_boundary_psi<R><<<blocks(nb_, 128), 128, 0, st_>>>(B(1), gv_, bstarts_.p, c_);
-            if (lists_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
+            if (lists_ || cands_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
             SPH_CUDA(cudaGetLastError());
             SPH_CUDA(cudaStreamSynchronize(st_));
         } else {
@@ -481,7 +484,7 @@ public:
             k_gather_boundary<R><<<blocks(nb_, 256), 256, 0, st_>>>(nb_, tmp_.p, key_.p, bstarts_.p, B(1), B(0));
             std::swap(bd_[0], bd_[1]);
             if (akinci_) k_boundary_psi<R><<<blocks(nb_, 128), 128, 0, st_>>>(B(1), gv_, bstarts_.p, c_);
-            if (lists_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
+            if (lists_ || cands_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
             SPH_CUDA(cudaGetLastError());
         } else {
             SPH_CUDA(cudaMemsetAsync(bstarts_.p, 0, (nkeys_ + 1) * sizeof(uint32_t), st_));
@@ -974,11 +977,10 @@ private:
         }
         lists_ = d.simulation_method == SPH_DFSPH && d.neighbor_list_max > 0;
         kmax_ = lists_ ? (uint32_t)d.neighbor_list_max : 0u;
-        // PCISPH / WCSPH candidate lists: one lane per particle, Akinci or no
-        // boundary (the PCISPH boundary model moves predicted positions after
+        // PCISPH / WCSPH candidate lists: Akinci or no boundary (the PCISPH boundary model moves predicted positions after
         // the prediction), indices below 2^27
         cands_ = (d.simulation_method == SPH_PCISPH || d.simulation_method == SPH_WCSPH) && d.neighbor_list_max > 0 &&
-                 G_ == 1 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask;
+                 !bh_ && std::max(n, nb) < (size_t)kCandIdxMask;
         if (cands_) {
             ckmax_ = (uint32_t)d.neighbor_list_max;
             SPH_CUDA(cand_.alloc((size_t)ckmax_ * n));
@@ -991,10 +993,10 @@ private:
         SPH_CUDA(lcount_.alloc(lists_ ? n : 1));
         SPH_CUDA(bgrad_.alloc(lists_ ? n : 1));
         SPH_CUDA(kbuf_.alloc(n));
-        // pair lists: half-precision positions for the build's cull (pairs of
+        // half-precision positions for the list builds' culls (pairs of
         // points, the last one whole, and a spare word for the cull), the
         // fluid's written by every gather, the boundary's once per grid box
-        if (lists_) {
+        if (lists_ || cands_) {
             SPH_CUDA(posh_.alloc(n / 2 + 2));
             SPH_CUDA(cudaMemsetAsync(posh_.p, 0, (n / 2 + 2) * sizeof(uint4), st_));
             SPH_CUDA(bposh_.alloc(nb / 2 + 2));
@@ -1082,10 +1084,10 @@ private:
             default: fn(std::integral_constant<int, 1>{}); break;
         }
     }
-    // the same for the passes that can visit candidate lists (one lane): fn(G, lists)
+    // the same for the passes that can visit candidate lists: fn(G, lists)
     template <typename Fn> void withGL(Fn&& fn)
     {
-        if (cands_) fn(std::integral_constant<int, 1>{}, std::true_type{});
+        if (cands_) withG([&](auto gt) { fn(gt, std::true_type{}); });
         else withG([&](auto gt) { fn(gt, std::false_type{}); });
     }
     unsigned wblocks() const { return blocks((size_t)n_ * G_, kBlock); }
@@ -1114,8 +1116,18 @@ private:
         const R reach = c_.h + cand_margin();
         // never below the passes' own cull, which has some slack over h
         const R reach2 = std::max(reach * reach, c_.cull2);
-        run("k_density_cand", [&] { launch(k_density_cand<R, EOS>, blocks(n_, kBlock), kBlock, 0, 
-            f, bd_[1].pos, gv_, starts_.p, bstarts_.p, c_, akinci_, reach2, cand_.p, candn_.p, candb_.p, ckmax_); });
+        const CandOut o{cand_.p, candn_.p, candb_.p, ckmax_, posh_.p, bposh_.p, bd_[1].cell};
+        const P4<R>* bp = bd_[1].pos;
+        const int akinci = nb_ ? akinci_ : 0;
+        withG([&](auto gt) {
+            constexpr int G = decltype(gt)::value;
+            if constexpr (G == 1)
+                run("k_density_cand", [&] { launch(k_density_cand<R, EOS>, blocks(n_, kBlock), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p,
+                                                   c_, akinci, reach2, o); });
+            else
+                run("k_density_cand", [&] { launch(k_density_cand_wide<R, G, EOS>, blocks((size_t)n_ * G, kWideBlock), kWideBlock, 0, f, bp,
+                                                   gv_, starts_.p, bstarts_.p, c_, akinci, reach2, o); });
+        });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }

@@ -5,6 +5,7 @@
 * The DFSPH list build that also forms the divergence solve's first error pass, at block edges.
 * The list build with 8, 4 and 1 lanes per particle (chosen by scene size), with lists that hold every neighbour and
   lists that overflow.
+* Candidate lists built and visited by several lanes per particle.
 """
 import numpy as np
 import pytest
@@ -94,3 +95,32 @@ def test_build_lanes_match_the_pool(gpu_lib, side, lists):
     for f, tol in (("x", 1e-6), ("rho", 1e-5), ("alpha", 4e-5)):
         g, w = s.get(f), P.get(k, f)
         assert np.abs(g - w).max() <= tol * np.abs(w).max(), f
+
+
+@pytest.mark.parametrize("method", ["wcsph", "pcisph"])
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("lanes,lists", [(8, 64), (4, 64), (2, 64), (8, 30), (8, 1), (4, 40)])
+@pytest.mark.parametrize("n", [1, 17, 600])
+def test_candidate_lists_shared_by_lanes(gpu_lib, method, precision, lanes, lists, n):
+    """Candidate lists built and visited by several lanes per particle against the cell walks, after one step: sums
+    of at most 64 terms, added in another order."""
+    r = 0.02
+    d = 2 * r
+    x = jitter(lattice(r, (d, d, d), (0.45, 0.45, 0.45)), r, 3)
+    x = x[np.random.default_rng(n).permutation(len(x))[:n]]
+    p = dict(boundary=2, radius=r, precision=precision, dt=1e-4, visc_method=2, visc=0.01, bvisc=0.01)
+    p.update(dict(method=0) if method == "wcsph" else dict(method=1, min_it=1, max_it=1, eta=0.001))
+    out = []
+    for k in (lists, 0):
+        s = sph_gb300.Scene(threads_per_particle=lanes, neighbor_list_max=k, **p)
+        s.set_fluid(x, np.random.default_rng(5).uniform(-0.2, 0.2, x.shape))
+        s.add_boundary_points(sph_gb300.sample_box(4 * r, (0, 0, 0), (0.6, 0.6, 0.6)))
+        s.init()
+        s.step(1)
+        out.append((s.get("rho"), s.get("v")))
+    eps = 2.0**-24 if precision == "f32" else 2.0**-53
+    (rho, v), (rho0, v0) = out
+    assert np.abs(rho - rho0).max() <= 64 * eps * np.abs(rho0).max()
+    if method == "wcsph":
+        # p = k ((rho / rho0)^7 - 1), k = 1.43e5: 7 k 64 eps; 64 terms of 2 p / rho^2 times m |grad W| <= 500; dt
+        assert np.abs(v - v0).max() <= 7 * 1.43e5 * 64 * eps * 2 / 1e6 * 64 * 500 * 1e-4
