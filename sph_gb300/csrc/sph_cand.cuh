@@ -13,22 +13,6 @@
 
 namespace sph {
 
-struct CandOut {
-    uint32_t* idx;
-    uint32_t* cnt;
-    uint32_t* bcnt;
-    uint32_t kmax;
-    const uint4* posh;       // half-precision positions (fluid, boundary or nullptr)
-    const uint4* bposh;
-    const uint32_t* bcell;
-};
-
-// cell offset code of a candidate in cell cj around cell ci (walk_reach's)
-__device__ __forceinline__ uint32_t cell_code(uint32_t ci, uint32_t cj)
-{
-    return (uint32_t)((cell_x(cj) - cell_x(ci) + 1) * 9 + (cell_y(cj) - cell_y(ci) + 1) * 3 + (cell_z(cj) - cell_z(ci) + 1));
-}
-
 template <typename R> struct CandSums {
     R density;
     uint32_t m;
@@ -153,19 +137,28 @@ __global__ void __launch_bounds__(kBlock, 7) k_density_cand(Fluid<R> f, const P4
     if (EOS) cand_eos(i, f, c, xi, density);
 }
 
-// The same with W lanes per particle (small scenes): lanes share the cull and
-// the evaluation, the list keeps the walk's order, and each lane's part of the
-// density is added across the lanes.
-template <typename R, int W, bool EOS>
+// The same with W lanes per particle (small scenes), each lane with a list and
+// a partial density of its own.  The lanes share the cull into a common queue.
+// EVEN: the listed candidates are dealt to the lanes in turn (a particle's
+// lists are then all stored or all walked).  Otherwise each takes the candidates of its part
+// of the cell walk (CandLists), so that the FP32 solvers' sums stay the walk's
+// bit for bit: DFSPH's and PCISPH's solves amplify rounding (a change of 1e-7
+// in the velocities grows to 1e-5 in five steps), WCSPH's and FP64's do not
+// need it, and the lanes' shares are uneven (8,000 WCSPH particles: 36 against
+// 41 us/step, FP64 189 against 279).
+// DENS = false: the lists alone (DFSPH's non-pressure forces).
+template <typename R, int W, bool EOS, bool EVEN, bool DENS = true>
 __global__ void __launch_bounds__(kWideBlock) k_density_cand_wide(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                   Consts<R> c, int akinci, R reach2, CandOut o)
 {
     grid_wait();
     constexpr uint32_t GROUPS = kWideBlock / W;
-    __shared__ uint32_t queue[GROUPS][kQueue], bqueue[GROUPS][kQueue];
+    constexpr uint32_t OWN = kQueue / (W / 2);  // a lane's candidates: twice its even share of the queue
+    constexpr int EB = kListBatch<R>;
+    __shared__ uint32_t queue[GROUPS][kQueue];
+    __shared__ uint32_t own[EVEN ? 1 : OWN][kWideBlock];
     const int gl = (int)(threadIdx.x % W), grp = (int)(threadIdx.x / W);
-    const int g0 = (int)(threadIdx.x & 31) & ~(W - 1);
     const uint32_t i = (blockIdx.x * kWideBlock + threadIdx.x) / W;
     const uint32_t n = f.n;
     const bool valid = i < f.count();
@@ -178,58 +171,111 @@ __global__ void __launch_bounds__(kWideBlock) k_density_cand_wide(Fluid<R> f, co
         pc = f.cell[i];
         half = half_cull_ok(g, pc, xi, c.h, &xr);
     }
-    const bool bhalf = half && akinci;
     const float hf = (float)c.h, rf2 = (float)reach2;
-    const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf, rf2), rb = wide_ranges<W>(bhalf, gl, g, bs, pc, xr, hf, rf2);
-    const uint32_t nq = cull_half_wide<W>(gl, rf, cell_z(pc), xr, hf, rf2, o.posh, queue[grp], kQueue);
-    const uint32_t nb = akinci ? cull_half_wide<W>(gl, rb, cell_z(pc), xr, hf, rf2, o.bposh, bqueue[grp], kQueue) : 0u;
-    __syncwarp();
+    uint32_t* q = queue[grp];
+    constexpr Rank RANK = EVEN ? kNoRank : (sizeof(R) == 4 ? kCellRank : kColumnRank);
+    const WideRanges<W, RANK> rf = wide_ranges<W, RANK>(half, gl, g, cs, pc, xr, hf, rf2),
+                              rb = wide_ranges<W, RANK>(half && akinci, gl, g, bs, pc, xr, hf, rf2);
     R density = 0;
-    uint32_t m = 0, mb = 0;
-    // queued entries, W a round; the ones within reach are listed in order
-    auto visit = [&](const uint32_t* q, uint32_t ne, const P4<R>* pos, const uint32_t* cell, bool bnd, uint32_t first) -> uint32_t {
-        uint32_t listed = 0;
-        for (uint32_t k = 0; __any_sync(0xffffffffu, k < ne); k += W) {
-            bool near = false;
-            uint32_t entry = 0;
-            if (k + gl < ne) {
-                const uint32_t j = q[k + gl];
-                const P4<R> pj = ldg4(pos + j);
-                const uint32_t cj = __ldg(cell + j);
-                const V3<R> r = pair_vec(xi, pc, pj, cj, c.h);
-                const R r2 = dot3(r, r);
-                near = r2 <= reach2;
-                entry = j | (cell_code(pc, cj) << kCandIdxBits);
-                if (r2 <= c.cull2) density += (bnd ? pj.w : c.mass) * cubic_W(c, sqrt(r2));
+    // this lane's part of the candidates of one kind; `first` slots are taken
+    // (EVEN: the particle's candidates, `first` listed so far)
+    auto visit = [&](const WideRanges<W, RANK>& rg, const uint4* posh, const P4<R>* pos, const uint32_t* cell,
+                     const uint32_t* __restrict__ starts, bool bnd, uint32_t first) -> uint32_t {
+        __syncwarp();  // the queue's last reader
+        const uint32_t nq = cull_half_wide<W, RANK>(gl, rg, cell_z(pc), xr, hf, rf2, posh, q, kQueue);
+        __syncwarp();
+        if constexpr (EVEN) {
+            const bool queued = half && nq <= kQueue;
+            uint32_t listed = 0;
+            for (uint32_t k = 0; __any_sync(0xffffffffu, queued && k < nq); k += W) {
+                bool near = false;
+                uint32_t entry = 0;
+                if (queued && k + gl < nq) {
+                    const uint32_t j = q[k + gl];
+                    const P4<R> pj = ldg4(pos + j);
+                    const uint32_t cj = __ldg(cell + j);
+                    const V3<R> r = pair_vec(xi, pc, pj, cj, c.h);
+                    const R r2 = dot3(r, r);
+                    near = r2 <= reach2;
+                    entry = j | (cell_code(pc, cj) << kCandIdxBits);
+                    if (r2 <= c.cull2) density += (bnd ? pj.w : c.mass) * cubic_W(c, sqrt(r2));
+                }
+                const uint32_t b = (__ballot_sync(0xffffffffu, near) >> ((threadIdx.x & 31) & ~(W - 1))) & ((1u << W) - 1u);
+                const uint32_t at = first + listed + __popc(b & ((1u << gl) - 1u));
+                if (near && at / W < o.kmax) o.idx[((size_t)(at / W) * n + i) * W + at % W] = entry;
+                listed += __popc(b);
             }
-            const uint32_t b = (__ballot_sync(0xffffffffu, near) >> g0) & ((1u << W) - 1u);
-            const uint32_t at = first + listed + __popc(b & ((1u << gl) - 1u));
-            if (near && at < o.kmax) o.idx[(size_t)at * n + i] = entry;
-            listed += __popc(b);
+            if (queued) return listed;
+            if (valid)
+                walk<R, W, false>(g, starts, pc, xi, c.h, gl, [&](uint32_t j, V3<R> s) {
+                    const P4<R> pj = ldg4(pos + j);
+                    const V3<R> r = s - xyz(pj);
+                    const R r2 = dot3(r, r);
+                    if (r2 <= c.cull2) density += (bnd ? pj.w : c.mass) * cubic_W(c, sqrt(r2));
+                });
+            return W * o.kmax + 1u;  // not stored
+        }
+        uint32_t listed = 0, mine = 0;
+        auto eval = [&](uint32_t j, uint32_t cj, const P4<R>& pj) {
+            const V3<R> r = pair_vec(xi, pc, pj, cj, c.h);
+            const R r2 = dot3(r, r);
+            if (r2 <= reach2) {
+                if (first + listed < o.kmax) o.idx[((size_t)(first + listed) * n + i) * W + gl] = j | (cell_code(pc, cj) << kCandIdxBits);
+                ++listed;
+            }
+            if (DENS && r2 <= c.cull2) density += (bnd ? pj.w : c.mass) * cubic_W(c, sqrt(r2));
+        };
+        if (half && nq <= kQueue) {
+#pragma unroll 4
+            for (uint32_t e = 0; e < nq; ++e) {
+                const uint32_t x = q[e];
+                if ((x >> kCandIdxBits) == (uint32_t)gl) {
+                    if (mine < OWN) own[mine][threadIdx.x] = x & kCandIdxMask;
+                    ++mine;
+                }
+            }
+        }
+        if (half && nq <= kQueue && mine <= OWN) {
+            for (uint32_t k = 0; k < mine; k += EB) {
+                uint32_t j[EB], cj[EB];
+                P4<R> pj[EB];
+#pragma unroll
+                for (int b = 0; b < EB; ++b) {
+                    j[b] = own[k + b < mine ? k + b : mine - 1][threadIdx.x];
+                    pj[b] = ldg4(pos + j[b]);
+                    cj[b] = __ldg(cell + j[b]);
+                }
+#pragma unroll
+                for (int b = 0; b < EB; ++b) {
+                    if (k + b >= mine) break;
+                    eval(j[b], cj[b], pj[b]);
+                }
+            }
+        } else if (valid) {
+            walk<R, W, false>(g, starts, pc, xi, c.h, gl, [&](uint32_t j, V3<R>) { eval(j, __ldg(cell + j), ldg4(pos + j)); });
         }
         return listed;
     };
-    const bool fwalk = valid && (!half || nq > kQueue), bwalk = valid && akinci && (!half || nb > kQueue);
-    m = visit(queue[grp], fwalk ? 0u : nq, f.pos, f.cell, false, 0u);
-    if (fwalk && gl == 0) {
-        const CandSums<R> w = cand_walk<R, false>(i, n, f.pos, g, cs, c, pc, xi, reach2, o.idx, o.kmax, 0u, density);
-        density = w.density;
-        m = w.m;
-    }
-    m = __shfl_sync(0xffffffffu, m, 0, W);
-    if (akinci) mb = visit(bqueue[grp], bwalk ? 0u : nb, bpos, o.bcell, true, m);
-    if (bwalk && gl == 0) {
-        const CandSums<R> w = cand_walk<R, true>(i, n, bpos, g, bs, c, pc, xi, reach2, o.idx, o.kmax, m, density);
-        density = w.density;
-        mb = w.m;
-    }
+    uint32_t m = visit(rf, o.posh, f.pos, f.cell, cs, false, 0u);
+    uint32_t mb = 0;
+    if (akinci) mb = visit(rb, o.bposh, bpos, o.bcell, bs, true, m);
     __syncwarp();
+    if constexpr (EVEN) {
+        // the particle's counts to this lane's; a particle's lists fit together
+        const uint32_t all = m + mb, fits = W * o.kmax, dealt = W - 1u - (uint32_t)gl;
+        const uint32_t own_m = m > fits ? o.kmax + 1u : (m + dealt) / W;
+        mb = m > fits || all > fits ? o.kmax + 1u : (all + dealt) / W - own_m;
+        m = own_m;
+    }
+    if (valid) {
+        o.cnt[(size_t)i * W + gl] = m;
+        o.bcnt[(size_t)i * W + gl] = mb;
+    }
+    if (!DENS) return;
     density = group_sum<W>(density);
     if (!valid || gl != 0) return;
     f.rho[i] = density;
     f.vel[i].w = density;
-    o.cnt[i] = m;
-    o.bcnt[i] = mb;
     if (EOS) cand_eos(i, f, c, xi, density);
 }
 

@@ -536,21 +536,25 @@ __global__ void k_boundary_psi(Boundary<R> b, GridView g, const uint32_t* __rest
 // at the predicted ones while every predicted displacement stays below
 // margin / 2 (checked per loop iteration; otherwise the predicted-density
 // pass walks the cells): its terms are the ones the walks skip, so the sums
-// are the same (bit for bit with one lane per particle; G lanes take every
-// G-th entry).  A particle with more than kmax candidates walks the cells.
+// are the same, bit for bit.  A list that does not fit its slots is walked.
 constexpr uint32_t kCandIdxBits = 27;
 constexpr uint32_t kCandIdxMask = (1u << kCandIdxBits) - 1u;
 
+//
+// With G lanes per particle each lane has a list of its own: the candidates
+// its share of the cell walk visits (every G-th of a cell's run), in that
+// order.  So its partial sums, and the result, are the walk's bit for bit.
+// Layout: idx[(t * n + i) * G + lane], counts [i * G + lane].
 struct CandLists {
-    const uint32_t* idx = nullptr;   // kmax * n, slot-major: j | (cell offset code << 27), the fluid candidates and then
-                           // the boundary's; nullptr: no lists
-    const uint32_t* cnt = nullptr;   // fluid candidates per particle (may exceed kmax)
-    const uint32_t* bcnt = nullptr;  // boundary candidates per particle; they are listed when both fit into kmax slots
-    uint32_t kmax = 0;
+    const uint32_t* idx = nullptr;   // j | (cell offset code << 27), the fluid candidates and then the boundary's;
+                                     // nullptr: no lists
+    const uint32_t* cnt = nullptr;   // fluid candidates (may exceed the slots)
+    const uint32_t* bcnt = nullptr;  // boundary candidates; listed when both fit
+    uint32_t slots = 0;              // list slots per lane
     uint32_t nb = 0;                 // boundary points
     unsigned* fault = nullptr;       // status word of the bounds-checked build (SPH_INDEX_OK)
-    __device__ __forceinline__ bool has(uint32_t i) const { return idx && cnt[i] <= kmax; }
-    __device__ __forceinline__ bool has_boundary(uint32_t i) const { return idx && cnt[i] + bcnt[i] <= kmax; }
+    __device__ __forceinline__ bool has(size_t l) const { return idx && cnt[l] <= slots; }
+    __device__ __forceinline__ bool has_boundary(size_t l) const { return idx && cnt[l] + bcnt[l] <= slots; }
 };
 
 // walk<R, 1> (rolled out, cells within reach2 of the particle), passing each
@@ -617,22 +621,22 @@ __device__ __forceinline__ void list_visit(const CandLists& L, uint32_t n, uint3
                                            uint32_t nj, V3<R> xi, int lane, const float4* shift, Load&& load, Eval&& eval)
 {
     constexpr bool REL = sizeof(R) == 4;
-    const uint32_t* __restrict__ p = L.idx + (size_t)first * n + i;
+    const uint32_t* __restrict__ p = L.idx + ((size_t)first * n + i) * G + lane;
 #pragma unroll 1
-    for (uint32_t k = lane; k < cnt; k += G * B) {
+    for (uint32_t k = 0; k < cnt; k += B) {
         uint32_t e[B];
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             // past the end: the last entry once more, not evaluated
-            const uint32_t kk = k + b * G < cnt ? k + b * G : cnt - 1;
-            e[b] = __ldg(p + (size_t)kk * n);
+            const uint32_t kk = k + b < cnt ? k + b : cnt - 1;
+            e[b] = __ldg(p + (size_t)kk * n * G);
         }
         decltype(load(0u)) q[B];
         bool ok[B];
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             const uint32_t j = e[b] & kCandIdxMask;
-            ok[b] = k + b * G < cnt;
+            ok[b] = k + b < cnt;
             if (SPH_INDEX_OK(j, nj, L.fault)) q[b] = load(j);
             else ok[b] = false;
         }
@@ -661,16 +665,17 @@ __device__ __noinline__ Acc walk_out_of_line(const GridView& g, const uint32_t* 
 }
 
 // Fluid candidates of particle i at lane LANE of G, summed into acc by
-// eval(acc, load(j), s): LISTS: every G-th entry of the stored list, or the
-// walk out of line where it did not fit; else the cell walk.
+// eval(acc, load(j), s): LISTS: the lane's stored list, or its part of the
+// walk out of line where the list did not fit; else the cell walk.
 template <typename R, int G, bool LISTS, int B, bool TRIM = true, typename Acc, typename Load, typename Eval>
 __device__ __forceinline__ void fluid_visit(const CandLists& L, uint32_t n, uint32_t i, const GridView& g,
                                             const uint32_t* __restrict__ cs, uint32_t pc, V3<R> xi, R h, int lane,
                                             const float4* shift, Acc& acc, Load load, Eval eval)
 {
     if constexpr (LISTS) {
-        if (L.has(i))
-            list_visit<R, G, B>(L, n, i, 0u, L.cnt[i], n, xi, lane, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
+        const size_t l = (size_t)i * G + lane;
+        if (L.has(l))
+            list_visit<R, G, B>(L, n, i, 0u, L.cnt[l], n, xi, lane, shift, load, [&](const auto& q, V3<R> s) { eval(acc, q, s); });
         else acc = walk_out_of_line<R, G, TRIM>(g, cs, pc, xi, h, lane, acc, load, eval);
     } else {
         walk<R, G, TRIM>(g, cs, pc, xi, h, lane, [&](uint32_t j, V3<R> s) { eval(acc, load(j), s); });
@@ -684,8 +689,9 @@ __device__ __forceinline__ void boundary_visit(const CandLists& L, uint32_t n, u
                                                const float4* shift, Acc& acc, Load load, Eval eval)
 {
     if constexpr (LISTS) {
-        if (L.has_boundary(i))
-            list_visit<R, G, B>(L, n, i, L.cnt[i], L.bcnt[i], L.nb, xi, lane, shift, load,
+        const size_t l = (size_t)i * G + lane;
+        if (L.has_boundary(l))
+            list_visit<R, G, B>(L, n, i, L.cnt[l], L.bcnt[l], L.nb, xi, lane, shift, load,
                                 [&](const auto& q, V3<R> s) { eval(acc, q, s); });
         else acc = walk_out_of_line<R, G, true>(g, bs, pc, xi, h, lane, acc, load, eval);
     } else {
@@ -888,14 +894,17 @@ template <typename R> struct PosVelIdx {
 template <typename R> struct NPFluid { V3<R> av, ast; };
 template <typename R> struct NPBoundary { V3<R> avb, aad; };
 
-template <typename R, int G, bool LISTS = false>
+// FL: the scene's force plugins where they are known when compiling (boundary
+// viscosity apart); kAnyForces: from the constants.
+constexpr int kAnyForces = -1;
+template <typename R, int G, bool LISTS = false, int FL = kAnyForces>
 __device__ __forceinline__ NPForces<R> npforce_sums(uint32_t i, int lane, const Fluid<R>& f,
                                                     const P4<R>* __restrict__ bpos, const GridView& g,
                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                     const Consts<R>& c, int akinci, R dt,
                                                     const CandLists& L = CandLists{}, const float4* shift = nullptr)
 {
-    const int fl = c.force_flags;
+    const int fl = FL == kAnyForces ? c.force_flags : (FL | (c.force_flags & F_BVISC));
     NPFluid<R> sf = {{0, 0, 0}, {0, 0, 0}};
     NPBoundary<R> sb = {{0, 0, 0}, {0, 0, 0}};
     const V3<R> xi = xyz(f.pos[i]);
@@ -988,7 +997,7 @@ __device__ __forceinline__ void npforce_apply(uint32_t i, const Fluid<R>& f, con
 }
 
 // Non-pressure forces in one walk (npforce_sums), lanes added, then applied.
-template <typename R, int G, bool LISTS>
+template <typename R, int G, bool LISTS, int FL>
 __global__ void __launch_bounds__(kBlock) k_npforce(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                     Consts<R> c, int akinci, const DevScalars* __restrict__ scr,
@@ -1002,7 +1011,7 @@ __global__ void __launch_bounds__(kBlock) k_npforce(Fluid<R> f, const P4<R>* __r
     const int lane = (int)(t % G);
     const bool valid = i < f.count();
     NPForces<R> s = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    if (valid) s = npforce_sums<R, G, LISTS>(i, lane, f, bpos, g, cs, bs, c, akinci, (R)scr->dt, L, shift);
+    if (valid) s = npforce_sums<R, G, LISTS, FL>(i, lane, f, bpos, g, cs, bs, c, akinci, (R)scr->dt, L, shift);
     if (G > 1) {
         s.av = group_sum3<G>(s.av); s.avb = group_sum3<G>(s.avb); s.ast = group_sum3<G>(s.ast); s.aad = group_sum3<G>(s.aad);
     }

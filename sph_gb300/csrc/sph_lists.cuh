@@ -47,6 +47,24 @@ template <typename R> struct Lists {
     const uint32_t* bcell;
 };
 
+// Where a density pass writes the candidate lists (CandLists, sph_kernels.cuh).
+struct CandOut {
+    uint32_t* idx;
+    uint32_t* cnt;
+    uint32_t* bcnt;
+    uint32_t kmax;           // slots per lane
+    uint32_t lanes;          // lanes per particle of the passes that visit the lists
+    const uint4* posh;       // half-precision positions (fluid, boundary or nullptr)
+    const uint4* bposh;
+    const uint32_t* bcell;
+};
+
+// cell offset code of a candidate in cell cj around cell ci (walk_reach's)
+__device__ __forceinline__ uint32_t cell_code(uint32_t ci, uint32_t cj)
+{
+    return (uint32_t)((cell_x(cj) - cell_x(ci) + 1) * 9 + (cell_y(cj) - cell_y(ci) + 1) * 3 + (cell_z(cj) - cell_z(ci) + 1));
+}
+
 // Phase 1 of the list build from the half-precision positions: the
 // nine columns of the 27-cell neighbourhood (trimmed as walk() trims them),
 // two candidates per half2 operation, accepted indices queued in walk order.
@@ -74,9 +92,16 @@ template <typename R> struct Lists {
 // the exact test on the queued ones).
 __device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
 
+//
+// RANK: each queued candidate with the lane whose part of a cell walk by
+// `lanes` lanes it is, above the index's 27 bits: its rank modulo the lanes
+// in its cell (kCellRank, the FP32 walk) or in its column (kColumnRank, FP64).
+enum Rank { kNoRank, kCellRank, kColumnRank };
+
+template <Rank RANK = kNoRank>
 __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t* __restrict__ starts, uint32_t pc,
                                               V3<float> xi, float h, float reach2, const uint4* __restrict__ posh,
-                                              uint32_t* q, uint32_t qstride, uint32_t qcap)
+                                              uint32_t* q, uint32_t qstride, uint32_t qcap, uint32_t lanes = 1u)
 {
     const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
     const float ofx = xi.x, ofy = xi.y, ofz = xi.z;
@@ -89,21 +114,26 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
     const __half2 h3 = __float2half2_rn(3.f * h);
     uint32_t nq = 0;
     // a column's candidate range (empty when trimmed); loaded one column ahead
-    auto range = [&](int c, uint32_t* b, uint32_t* e) {
+    auto range = [&](int c, uint32_t* b, uint32_t* e, uint32_t* s1, uint32_t* s2) {
         const int dx = c / 3 - 1, dy = c - (c / 3) * 3 - 1;
         const float gxy = (dx < 0 ? gxm : (dx > 0 ? gxp : 0.f)) + (dy < 0 ? gym : (dy > 0 ? gyp : 0.f));
         if (!(gxy <= lim)) { *b = 0u; *e = 0u; return; }
         const uint32_t base = (__ldg(g.mortx + cx + dx) | __ldg(g.morty + cy + dy)) * (uint32_t)g.nz;
         *b = __ldg(starts + base + (gxy + gzm <= lim ? cz - 1 : cz));
         *e = __ldg(starts + base + (gxy + gzp <= lim ? cz + 2 : cz + 1));
+        if constexpr (RANK == kCellRank) {
+            *s1 = __ldg(starts + base + cz);
+            *s2 = __ldg(starts + base + cz + 1);
+        }
+        if constexpr (RANK == kColumnRank) *s1 = __ldg(starts + base + cz - 1);
     };
-    uint32_t nb, ne;
-    range(0, &nb, &ne);
+    uint32_t nb, ne, n1 = 0u, n2 = 0u;
+    range(0, &nb, &ne, &n1, &n2);
 #pragma unroll 1
     for (int c = 0; c < 9; ++c) {
         const int dx = c / 3 - 1, dy = c - (c / 3) * 3 - 1;
-        const uint32_t bb = nb, ee = ne;
-        if (c < 8) range(c + 1, &nb, &ne);
+        const uint32_t bb = nb, ee = ne, s1 = n1, s2 = n2;
+        if (c < 8) range(c + 1, &nb, &ne, &n1, &n2);
         const __half2 sx = __float2half2_rn(xi.x - (float)dx * h), sy = __float2half2_rn(xi.y - (float)dy * h);
         // The column's candidates 32 at a time (16 words): the test's
         // acceptance bits are gathered into one word, candidate j0 + b at
@@ -142,7 +172,10 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
             while (bits) {
                 const uint32_t b = __ffs(bits) - 1;
                 bits &= bits - 1;
-                if (nq < qcap) q[nq * qstride + threadIdx.x] = j0 + b;
+                uint32_t x = j0 + b;
+                if constexpr (RANK == kColumnRank) x |= ((x - s1) & (lanes - 1)) << kCandIdxBits;
+                if constexpr (RANK == kCellRank) x |= ((x - (x < s1 ? bb : (x < s2 ? s1 : s2))) & (lanes - 1)) << kCandIdxBits;
+                if (nq < qcap) q[nq * qstride + threadIdx.x] = x;
                 ++nq;
             }
         }
@@ -274,12 +307,15 @@ __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint3
 // the finished lists (same terms, same order), into *div0, with the count of
 // neighbours into *nn0 (a particle whose list or queue overflowed takes the
 // same list or cell walk as velocity_div_one).
-template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1, bool POOL = false>
+// CAND (scenes with non-pressure forces): also the candidate list those
+// forces' passes visit, every candidate within their cull.
+template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1, bool POOL = false, bool CAND = false>
 __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                                 const GridView& g, const uint32_t* __restrict__ cs,
                                                 const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
                                                 const Lists<R>& L, uint32_t* q, uint32_t qstride = kBlock,
-                                                uint32_t qdepth = kQueue, R* div0 = nullptr, uint32_t* nn0 = nullptr)
+                                                uint32_t qdepth = kQueue, R* div0 = nullptr, uint32_t* nn0 = nullptr,
+                                                const CandOut& o = CandOut{})
 {
     const uint32_t n = f.n;
     const V3<R> xi = xyz(f.pos[i]);
@@ -319,16 +355,9 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
     uint32_t nq = 0;
     bool half_cull = false;
     V3<float> xr;  // the position in its cell's frame
-    {
-        const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
-        if constexpr (sizeof(R) == 4) xr = xi;
-        else xr = V3<float>{(float)(xi.x - (R)(cx + g.ox) * c.h), (float)(xi.y - (R)(cy + g.oy) * c.h),
-                            (float)(xi.z - (R)(cz + g.oz) * c.h)};
-        const float hf = (float)c.h, hh = 0.5f * hf;
-        half_cull = L.posh && cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
-                    fabsf(xr.x - hh) <= hf && fabsf(xr.y - hh) <= hf && fabsf(xr.z - hh) <= hf;
-        if (half_cull) nq = cull_half(g, cs, pc, xr, hf, (float)c.cull2, L.posh, q, qstride, qcap);
-    }
+    half_cull = L.posh && half_cull_ok(g, pc, xi, c.h, &xr);
+    constexpr Rank RANK = !CAND ? kNoRank : (sizeof(R) == 4 ? kCellRank : kColumnRank);
+    if (half_cull) nq = cull_half<RANK>(g, cs, pc, xr, (float)c.h, (float)c.cull2, L.posh, q, qstride, qcap, o.lanes);
     if (!half_cull)
         walk<R, 1, true, FAST>(g, cs, pc, xi, c.h, 0, [&](uint32_t j, V3<R> s) {
             const V3<R> r = s - xyz(ldg4(f.pos + j));
@@ -337,26 +366,38 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
                 ++nq;
             }
         });
+    // CAND: the candidate lists, one per lane of the force passes (CandLists);
+    // x: a queued candidate with its lane.  Counts packed in bytes.
+    unsigned long long nl = 0, nlf = 0;
+    auto list = [&](uint32_t x, uint32_t cj, R r2) {
+        if (!(r2 <= c.cull2)) return;
+        const uint32_t t = x >> kCandIdxBits, slot = (uint32_t)(nl >> (8 * t)) & 255u;
+        if (slot < o.kmax) o.idx[((size_t)slot * n + i) * o.lanes + t] = (x & kCandIdxMask) | (cell_code(pc, cj) << kCandIdxBits);
+        nl += 1ull << (8 * t);
+    };
+    bool fwalk = !half_cull, bwalk = !half_cull;  // its force passes walk
     if (nq <= qcap) {
         // phase 2: evaluate the queued candidates in walk order
         for (uint32_t k = 0; k < nq; k += EB) {
-            uint32_t j[EB], cj[EB];
+            uint32_t j[EB], cj[EB], x[EB];
             P4<R> pj[EB];
             V3<R> vj[EB];
 #pragma unroll
             for (int b = 0; b < EB; ++b) {
                 // (past the end: the last candidate once more, not evaluated)
-                j[b] = q[(EB == 1 || k + b < nq ? k + b : nq - 1) * qstride + threadIdx.x];
+                x[b] = q[(EB == 1 || k + b < nq ? k + b : nq - 1) * qstride + threadIdx.x];
+                j[b] = CAND ? x[b] & kCandIdxMask : x[b];
                 // (a plain load for the velocity: other threads write its w here)
                 vj[b] = V3<R>{0, 0, 0};
                 if constexpr (DIV0) vj[b] = xyz(f.vel[j[b]]);
                 pj[b] = ldg4(f.pos + j[b]);
-                cj[b] = sizeof(R) == 4 ? __ldg(f.cell + j[b]) : 0u;
+                cj[b] = CAND || sizeof(R) == 4 ? __ldg(f.cell + j[b]) : 0u;
             }
 #pragma unroll
             for (int b = 0; b < EB; ++b) {
                 if (EB > 1 && k + b >= nq) break;
                 const V3<R> r = pair_vec(xi, pc, pj[b], cj[b], c.h);
+                if constexpr (CAND) list(x[b], cj[b], dot3(r, r));
                 accept(j[b], r, dot3(r, r), vj[b]);
             }
         }
@@ -366,7 +407,9 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
         sumSq = b.sumSq;
         sumGrad = b.sumGrad;
         cnt = b.cnt;
+        fwalk = true;
     }
+    nlf = nl;
     V3<R> bg = {0, 0, 0};
     if (akinci) {
         auto bterm = [&](const P4<R>& pb, V3<R> r) {
@@ -384,24 +427,28 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
         // the same order as the walk, the gradient sum compiled apart from
         // the walk's, so its last bit may differ); or the walk itself.
         uint32_t nb = qcap + 1u;
-        if (half_cull && L.bposh) nb = cull_half(g, bs, pc, xr, (float)c.h, (float)c.cull2, L.bposh, q, qstride, qcap);
+        if (half_cull && L.bposh) nb = cull_half<RANK>(g, bs, pc, xr, (float)c.h, (float)c.cull2, L.bposh, q, qstride, qcap, o.lanes);
         if (nb <= qcap) {
             for (uint32_t k = 0; k < nb; k += EB) {
                 P4<R> pb[EB];
-                uint32_t cb[EB];
+                uint32_t cb[EB], x[EB];
 #pragma unroll
                 for (int b = 0; b < EB; ++b) {
-                    const uint32_t j = q[(EB == 1 || k + b < nb ? k + b : nb - 1) * qstride + threadIdx.x];
+                    x[b] = q[(EB == 1 || k + b < nb ? k + b : nb - 1) * qstride + threadIdx.x];
+                    const uint32_t j = CAND ? x[b] & kCandIdxMask : x[b];
                     pb[b] = ldg4(bpos + j);
-                    cb[b] = sizeof(R) == 4 ? __ldg(L.bcell + j) : 0u;
+                    cb[b] = CAND || sizeof(R) == 4 ? __ldg(L.bcell + j) : 0u;
                 }
 #pragma unroll
                 for (int b = 0; b < EB; ++b) {
                     if (EB > 1 && k + b >= nb) break;
-                    bterm(pb[b], pair_vec(xi, pc, pb[b], cb[b], c.h));
+                    const V3<R> r = pair_vec(xi, pc, pb[b], cb[b], c.h);
+                    if constexpr (CAND) list(x[b], cb[b], dot3(r, r));
+                    bterm(pb[b], r);
                 }
             }
         } else {
+            bwalk = true;
             walk<R, 1>(g, bs, pc, xi, c.h, 0, [&](uint32_t j, V3<R> s) {
                 const P4<R> pb = ldg4(bpos + j);
                 bterm(pb, s - xyz(pb));
@@ -421,6 +468,13 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
     f.alpha[i] = (fabs(den) > c.eps) ? density / den : (R)0;
     L.count[i] = cnt;
     L.bgrad[i] = P4<R>{bg.x, bg.y, bg.z, 0};
+    if constexpr (CAND) {
+        for (uint32_t t = 0; t < o.lanes; ++t) {
+            const uint32_t m = (uint32_t)(nlf >> (8 * t)) & 255u, all = (uint32_t)(nl >> (8 * t)) & 255u;
+            o.cnt[(size_t)i * o.lanes + t] = fwalk ? o.kmax + 1u : m;
+            o.bcnt[(size_t)i * o.lanes + t] = bwalk ? o.kmax + 1u : all - m;
+        }
+    }
     if constexpr (DIV0) {
         if (cnt > L.kmax) {
             const DivSum<R> d = velocity_div_cells(f, bpos, g, cs, bs, c, akinci, i, vi);
@@ -481,11 +535,12 @@ __device__ __forceinline__ void divergence_control(DevScalars* sc, const LoopLim
 // (9 FP64 operations on each of ~150 candidates, at two FP64 lanes per SM)
 // was a third of the build: 125k particles 1454 -> 1003 us with the boundary's
 // cull and the fused error pass.
-template <typename R, bool DIV0>
+template <typename R, bool DIV0, bool CAND>
 __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                            const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                            Consts<R> c, int akinci, Lists<R> L, DevScalars* sc,
-                                                           LoopLimits lim, double* partials, cudaGraphConditionalHandle cond)
+                                                           LoopLimits lim, double* partials, cudaGraphConditionalHandle cond,
+                                                           CandOut o)
 {
     grid_wait();
     __shared__ uint32_t q[kQueue * kBlock];
@@ -495,7 +550,8 @@ __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<
     if (i < f.count()) {
         R dv = 0;
         uint32_t nn = 0;
-        build_lists_one<R, sizeof(R) == 4, DIV0, EB>(i, f, bpos, g, cs, bs, c, akinci, L, q, kBlock, kQueue, &dv, &nn);
+        build_lists_one<R, sizeof(R) == 4, DIV0, EB, false, CAND>(i, f, bpos, g, cs, bs, c, akinci, L, q, kBlock, kQueue, &dv,
+                                                                  &nn, o);
         if (DIV0) err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
     }
     if constexpr (DIV0) {
@@ -530,12 +586,13 @@ constexpr uint32_t kWideBlock = 128, kWideChunk = 32;
 
 // The candidate ranges of cull_half's nine columns, lane gl of W holding
 // columns gl, gl + W, ...: in b[], e[] (empty where trimmed, or with !on).
-template <int W> struct WideRanges {
+// RANK: also what a candidate's rank is counted from.
+template <int W, Rank RANK = kNoRank> struct WideRanges {
     static constexpr int C = (9 + W - 1) / W;
-    uint32_t b[C], e[C];
+    uint32_t b[C], e[C], m0[RANK ? C : 1], m1[RANK ? C : 1];
 };
-template <int W>
-__device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const GridView& g, const uint32_t* __restrict__ starts,
+template <int W, Rank RANK = kNoRank>
+__device__ __forceinline__ WideRanges<W, RANK> wide_ranges(bool on, int gl, const GridView& g, const uint32_t* __restrict__ starts,
                                                      uint32_t pc, V3<float> xi, float h, float reach2)
 {
     const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
@@ -544,11 +601,12 @@ __device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const Grid
     const float gym = ofy > 0.f ? ofy * ofy : 0.f, gyp = h - ofy > 0.f ? (h - ofy) * (h - ofy) : 0.f;
     const float gzm = ofz > 0.f ? ofz * ofz : 0.f, gzp = h - ofz > 0.f ? (h - ofz) * (h - ofz) : 0.f;
     const float lim = fmaxf(reach2, h * h) * (float)(1.0 + 1e-5);
-    WideRanges<W> r;
+    WideRanges<W, RANK> r;
 #pragma unroll
     for (int t = 0; t < WideRanges<W>::C; ++t) {
         const int c = gl + t * W;
         r.b[t] = r.e[t] = 0u;
+        if constexpr (RANK) r.m0[t] = r.m1[t] = 0u;
         if (on && c < 9) {
             const int dx = c / 3 - 1, dy = c % 3 - 1;
             const float gxy = (dx < 0 ? gxm : (dx > 0 ? gxp : 0.f)) + (dy < 0 ? gym : (dy > 0 ? gyp : 0.f));
@@ -556,6 +614,11 @@ __device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const Grid
                 const uint32_t base = (__ldg(g.mortx + cx + dx) | __ldg(g.morty + cy + dy)) * (uint32_t)g.nz;
                 r.b[t] = __ldg(starts + base + (gxy + gzm <= lim ? cz - 1 : cz));
                 r.e[t] = __ldg(starts + base + (gxy + gzp <= lim ? cz + 2 : cz + 1));
+                if constexpr (RANK == kCellRank) {
+                    r.m0[t] = __ldg(starts + base + cz);
+                    r.m1[t] = __ldg(starts + base + cz + 1);
+                }
+                if constexpr (RANK == kColumnRank) r.m0[t] = __ldg(starts + base + cz - 1);
             }
         }
     }
@@ -564,9 +627,10 @@ __device__ __forceinline__ WideRanges<W> wide_ranges(bool on, int gl, const Grid
 
 // cull_half by W lanes: accepted candidates in walk order into the group's
 // queue; every lane returns their number.  gl = lane in the group; all lanes
-// of the warp call it.
-template <int W>
-__device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W>& rg, int cz, V3<float> xi, float h, float reach2,
+// of the warp call it.  RANK: each with the lane whose part of the cell walk
+// it is (its rank modulo W) above the index's 27 bits.
+template <int W, Rank RANK = kNoRank>
+__device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W, RANK>& rg, int cz, V3<float> xi, float h, float reach2,
                                                    const uint4* __restrict__ posh, uint32_t* q, uint32_t qcap)
 {
     const __half2 thr = __float2half2_rn(reach2 * 1.03f);
@@ -587,6 +651,9 @@ __device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W>& 
     for (int c = 0; c < 9; ++c) {
         const int dx = c / 3 - 1, dy = c % 3 - 1;
         const uint32_t bb = __shfl_sync(0xffffffffu, rg.b[c / W], c % W, W), ee = __shfl_sync(0xffffffffu, rg.e[c / W], c % W, W);
+        uint32_t s1 = 0u, s2 = 0u;
+        if constexpr (RANK) s1 = __shfl_sync(0xffffffffu, rg.m0[c / W], c % W, W);
+        if constexpr (RANK == kCellRank) s2 = __shfl_sync(0xffffffffu, rg.m1[c / W], c % W, W);
         const __half2 sx = __float2half2_rn(xi.x - (float)dx * h), sy = __float2half2_rn(xi.y - (float)dy * h);
         uint32_t word = (bb >> 1) + gl;
         uint4 w = w0[c];
@@ -604,11 +671,20 @@ __device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W>& 
             const uint32_t b1 = (__ballot_sync(0xffffffffu, a1) >> g0) & ((1u << W) - 1u);
             const uint32_t below = (1u << gl) - 1u;
             uint32_t at = nq + __popc(b0 & below) + __popc(b1 & below);
+            uint32_t t0 = j, t1 = j + 1;
+            if constexpr (RANK == kColumnRank) {
+                t0 |= ((j - s1) & (W - 1)) << kCandIdxBits;
+                t1 |= ((j + 1 - s1) & (W - 1)) << kCandIdxBits;
+            }
+            if constexpr (RANK == kCellRank) {
+                t0 |= ((j - (j < s1 ? bb : (j < s2 ? s1 : s2))) & (W - 1)) << kCandIdxBits;
+                t1 |= ((j + 1 - (j + 1 < s1 ? bb : (j + 1 < s2 ? s1 : s2))) & (W - 1)) << kCandIdxBits;
+            }
             if (a0) {
-                if (at < qcap) q[at] = j;
+                if (at < qcap) q[at] = t0;
                 ++at;
             }
-            if (a1 && at < qcap) q[at] = j + 1;
+            if (a1 && at < qcap) q[at] = t1;
             nq += __popc(b0) + __popc(b1);
             word += W;
             if (2 * word < ee) w = __ldg(posh + word);
@@ -648,13 +724,7 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
         xi = xyz(f.pos[i]);
         pc = f.cell[i];
         if constexpr (DIV0) vi = xyz(f.vel[i]);
-        const int cx = cell_x(pc), cy = cell_y(pc), cz = cell_z(pc);
-        if constexpr (sizeof(R) == 4) xr = xi;
-        else xr = V3<float>{(float)(xi.x - (R)(cx + g.ox) * c.h), (float)(xi.y - (R)(cy + g.oy) * c.h),
-                            (float)(xi.z - (R)(cz + g.oz) * c.h)};
-        const float hh = 0.5f * hf;
-        half = cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
-               fabsf(xr.x - hh) <= hf && fabsf(xr.y - hh) <= hf && fabsf(xr.z - hh) <= hf;
+        half = half_cull_ok(g, pc, xi, c.h, &xr);
     }
     const bool bhalf = half && akinci && L.bposh;
     const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf, (float)c.cull2),
@@ -706,11 +776,13 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
             for (int t = 0; t < 2; ++t) {
                 bool listed = false;
                 V3<R> mg = {0, 0, 0};
+                R r2 = 0;
                 if (in[t]) {
                     const V3<R> r = pair_vec(xi, pc, pj[t], cj[t], c.h);
+                    r2 = dot3(r, r);
                     R w;
                     V3<R> gw;
-                    cubic_W_gradW<FAST>(c, r, dot3(r, r), &w, &gw);
+                    cubic_W_gradW<FAST>(c, r, r2, &w, &gw);
                     mg = c.mass * gw;
                     const R mg2 = dot3_div(mg, mg);
                     listed = mg2 > (R)0;

@@ -977,17 +977,19 @@ private:
         }
         lists_ = d.simulation_method == SPH_DFSPH && d.neighbor_list_max > 0;
         kmax_ = lists_ ? (uint32_t)d.neighbor_list_max : 0u;
-        // PCISPH / WCSPH candidate lists: Akinci or no boundary (the PCISPH boundary model moves predicted positions after
-        // the prediction), indices below 2^27
-        cands_ = (d.simulation_method == SPH_PCISPH || d.simulation_method == SPH_WCSPH) && d.neighbor_list_max > 0 &&
-                 !bh_ && std::max(n, nb) < (size_t)kCandIdxMask;
+        // candidate lists, PCISPH and WCSPH, and DFSPH for its non-pressure
+        // forces: Akinci or no boundary (the PCISPH boundary model moves
+        // predicted positions after the prediction), indices below 2^27
+        cands_ = d.neighbor_list_max > 0 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask &&
+                 (d.simulation_method != SPH_DFSPH || (c_.force_flags != 0 && (G_ > 1 || build_lanes() == 1)));
         if (cands_) {
-            ckmax_ = (uint32_t)d.neighbor_list_max;
-            SPH_CUDA(cand_.alloc((size_t)ckmax_ * n));
-            SPH_CUDA(candn_.alloc(n));
-            SPH_CUDA(candb_.alloc(n));
-            SPH_CUDA(cudaMemsetAsync(candn_.p, 0, n * sizeof(uint32_t), st_));
-            SPH_CUDA(cudaMemsetAsync(candb_.p, 0, n * sizeof(uint32_t), st_));
+            // one lane: the whole list; G lanes: each twice its even share
+            cslots_ = G_ == 1 ? (uint32_t)d.neighbor_list_max : std::max(1u, 2u * (uint32_t)d.neighbor_list_max / (unsigned)G_);
+            SPH_CUDA(cand_.alloc((size_t)cslots_ * n * G_));
+            SPH_CUDA(candn_.alloc(n * G_));
+            SPH_CUDA(candb_.alloc(n * G_));
+            SPH_CUDA(cudaMemsetAsync(candn_.p, 0, n * G_ * sizeof(uint32_t), st_));
+            SPH_CUDA(cudaMemsetAsync(candb_.p, 0, n * G_ * sizeof(uint32_t), st_));
         }
         SPH_CUDA(pairs_.alloc(lists_ ? (size_t)kmax_ * n : 1));
         SPH_CUDA(lcount_.alloc(lists_ ? n : 1));
@@ -1116,7 +1118,7 @@ private:
         const R reach = c_.h + cand_margin();
         // never below the passes' own cull, which has some slack over h
         const R reach2 = std::max(reach * reach, c_.cull2);
-        const CandOut o{cand_.p, candn_.p, candb_.p, ckmax_, posh_.p, bposh_.p, bd_[1].cell};
+        const CandOut o = CO();
         const P4<R>* bp = bd_[1].pos;
         const int akinci = nb_ ? akinci_ : 0;
         withG([&](auto gt) {
@@ -1125,7 +1127,7 @@ private:
                 run("k_density_cand", [&] { launch(k_density_cand<R, EOS>, blocks(n_, kBlock), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p,
                                                    c_, akinci, reach2, o); });
             else
-                run("k_density_cand", [&] { launch(k_density_cand_wide<R, G, EOS>, blocks((size_t)n_ * G, kWideBlock), kWideBlock, 0, f, bp,
+                run("k_density_cand", [&] { launch(k_density_cand_wide<R, G, EOS, EOS || sizeof(R) == 8>, blocks((size_t)n_ * G, kWideBlock), kWideBlock, 0, f, bp,
                                                    gv_, starts_.p, bstarts_.p, c_, akinci, reach2, o); });
         });
         SPH_CUDA(cudaGetLastError());
@@ -1155,17 +1157,25 @@ private:
         Fluid<R> f = F();
         const P4<R>* bp = bd_[1].pos;
         Lists<R> L = LS();
-        auto wide = [&](auto wt) {
+        auto build = [&](auto wt, auto ct) {
             constexpr int W = decltype(wt)::value;
-            run("k_build_lists", [&] { launch(k_build_lists_wide<R, W, DIV0>, blocks((size_t)n_ * W, kWideBlock), kWideBlock, 0, 
-                f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
+            constexpr bool CAND = decltype(ct)::value;
+            run("k_build_lists", [&] {
+                if constexpr (W == 1)
+                    launch(k_build_lists<R, DIV0, CAND>, blocks(n_, kBlock), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L,
+                           sc_.p, lim_, partials_.p, h, CO());
+                else
+                    launch(k_build_lists_wide<R, W, DIV0>, blocks((size_t)n_ * W, kWideBlock), kWideBlock, 0, f, bp, gv_, starts_.p,
+                           bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h);
+            });
         };
         const int W = build_lanes();
-        if (W == 8) wide(std::integral_constant<int, 8>{});
-        else if (W == 4) wide(std::integral_constant<int, 4>{});
-        else
-            run("k_build_lists", [&] { launch(k_build_lists<R, DIV0>, blocks(n_, kBlock), kBlock, 0, 
-                f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h); });
+        if (W == 8) build(std::integral_constant<int, 8>{}, std::false_type{});
+        else if (W == 4) build(std::integral_constant<int, 4>{}, std::false_type{});
+        // with force plugins this build also writes the candidate lists of their
+        // passes (scenes below that: launch_npforces)
+        else if (cands_) build(std::integral_constant<int, 1>{}, std::true_type{});
+        else build(std::integral_constant<int, 1>{}, std::false_type{});
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1354,13 +1364,35 @@ private:
         if (!c_.force_flags) return SPH_OK;
         Fluid<R> f = F();
         const P4<R>* bp = bd_[1].pos;
+        if (cands_ && d.simulation_method == SPH_DFSPH && build_lanes() > 1) {
+            // the candidate lists of the current positions: the DFSPH build
+            // with lanes writes its pair lists only
+            const int akinci = nb_ ? akinci_ : 0;
+            withG([&](auto gt) {
+                constexpr int G = decltype(gt)::value;
+                if constexpr (G > 1)
+                    run("k_cand_lists", [&] { launch(k_density_cand_wide<R, G, false, false, false>, blocks((size_t)n_ * G, kWideBlock), kWideBlock, 0, f,
+                                                     bp, gv_, starts_.p, bstarts_.p, c_, akinci, c_.cull2, CO()); });
+            });
+        }
         withGL([&](auto gt, auto lt) {
             constexpr int G = decltype(gt)::value;
             constexpr bool LISTS = decltype(lt)::value;
             const CandLists L = CL();
             if (c_.force_flags & F_SURFACE_TENSION)
                 run("k_st_normals", [&] { launch(k_st_normals<R, G, LISTS>, wblocks(), kBlock, 0, f, gv_, starts_.p, c_, L); });
-            run("k_npforce", [&] { launch(k_npforce<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
+            auto go = [&](auto ft) {
+                constexpr int FL = decltype(ft)::value;
+                run("k_npforce", [&] { launch(k_npforce<R, G, LISTS, FL>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
+            };
+            // usual combinations compiled apart: fewer registers and no tests
+            // of the flags in the loop
+            constexpr int XSPH = F_XSPH, STD_ALL = F_STD_VISC | F_SURFACE_TENSION | F_ADHESION, XSPH_ALL = F_XSPH | F_SURFACE_TENSION | F_ADHESION;
+            const int fl = c_.force_flags & ~F_BVISC;
+            if (LISTS && fl == XSPH) go(std::integral_constant<int, LISTS ? XSPH : kAnyForces>{});
+            else if (LISTS && fl == STD_ALL) go(std::integral_constant<int, LISTS ? STD_ALL : kAnyForces>{});
+            else if (LISTS && fl == XSPH_ALL) go(std::integral_constant<int, LISTS ? XSPH_ALL : kAnyForces>{});
+            else go(std::integral_constant<int, kAnyForces>{});
         });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
@@ -1752,12 +1784,13 @@ private:
     bool lists_ = false;
     uint32_t kmax_ = 0;
     bool cands_ = false;            // PCISPH candidate lists (CandLists)
-    uint32_t ckmax_ = 0;
+    uint32_t cslots_ = 0;           // list slots per lane
     DevBuf<uint32_t> cand_, candn_, candb_;
     CandLists CL() const
     {
-        return cands_ ? CandLists{cand_.p, candn_.p, candb_.p, ckmax_, nb_, &sc_.p->status} : CandLists{};
+        return cands_ ? CandLists{cand_.p, candn_.p, candb_.p, cslots_, nb_, &sc_.p->status} : CandLists{};
     }
+    CandOut CO() const { return CandOut{cand_.p, candn_.p, candb_.p, cslots_, (uint32_t)G_, posh_.p, bposh_.p, bd_[1].cell}; }
     // the lists' reach beyond h: predicted displacements up to half of it keep them exact
     // (WCSPH visits them at the current positions only)
     R cand_margin() const { return d.simulation_method == SPH_PCISPH ? (R)0.1 * c_.h : (R)0; }
