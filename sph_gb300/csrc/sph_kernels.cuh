@@ -58,6 +58,13 @@ template <typename R> struct Boundary {
 constexpr unsigned kBlock = 128;
 
 __device__ __forceinline__ unsigned gtid() { return blockIdx.x * blockDim.x + threadIdx.x; }
+// The same with the blocks in descending order.  The solver passes over the
+// neighbour lists run back and forth (corrections and pressure accelerations
+// descending, error passes and list builds ascending), so that a pass starts
+// on the lists the pass before it read last and finds them in L2 (129 MB).
+// us/step: 250,000 particles DFSPH (106 MB of pair records) 463 -> 452, 490k
+// PCISPH drop 1017 -> 1006, mix of 256 scenes (1.7 GB) 4560 -> 4522.
+__device__ __forceinline__ unsigned gtid_back() { return (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; }
 
 template <int G, typename T> __device__ __forceinline__ T group_sum(T v)
 {
@@ -1496,7 +1503,7 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_pressure_acc(Fluid<R> f, cons
     __shared__ float4 shift[LISTS ? kShiftCodes : 1];
     if (!sc->active) return;
     if (LISTS && sizeof(R) == 4) fill_shift_table(shift, (float)c.h);
-    const uint32_t t = gtid();
+    const uint32_t t = gtid_back();
     const uint32_t i = t / G;
     const int lane = (int)(t % G);
     const bool valid = i < f.count();

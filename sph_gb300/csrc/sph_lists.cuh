@@ -269,11 +269,20 @@ __device__ __noinline__ BuildSums<R> build_walk_all(uint32_t i, const Fluid<R>& 
 // The dot product of the velocity divergence terms with its rounding written
 // out (FP32: the contraction the compiler chose for the pass over the lists
 // first), so that the sums of the one-scene build and of its passes agree bit
-// for bit.  The pool's kernels (POOL) keep the compiler's contraction of each.
-template <bool POOL = false, typename R> __device__ __forceinline__ R dot3_div(V3<R> a, V3<R> b)
+// for bit.  The pool's kernels (kPool) keep the plain expression, whose
+// contraction differs from one copy of its unrolled loop to the next.
+enum Rounding { kOneScene, kPool };
+template <Rounding WHERE = kOneScene, typename R> __device__ __forceinline__ R dot3_div(V3<R> a, V3<R> b)
 {
-    if constexpr (sizeof(R) == 8 || POOL) return dot3(a, b);
+    if constexpr (sizeof(R) == 8 || WHERE == kPool) return dot3(a, b);
     else return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+
+// The other contraction of a dot product.
+template <typename R> __device__ __forceinline__ R dot3_zyx(V3<R> a, V3<R> b)
+{
+    if constexpr (sizeof(R) == 8) return dot3(a, b);
+    else return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
 }
 
 // Forward declarations: the list build's DIV0 form ends with the velocity
@@ -284,7 +293,7 @@ __device__ __noinline__ DivSum<R> velocity_div_cells(const Fluid<R>& f, const P4
                                                      const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                      const Consts<R>& c, int akinci, uint32_t i, V3<R> vi);
 
-template <typename R, bool POOL = false>
+template <typename R, Rounding WHERE = kOneScene>
 __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint32_t i, V3<R> vi, uint32_t cnt)
 {
     const uint32_t n = f.n;
@@ -293,7 +302,7 @@ __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint3
         const P4<R> pr = L.pairs[(size_t)k * n + i];
         const uint32_t j = as_idx(pr.w);
         if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-        dv += dot3_div<POOL>(vi - xyz(f.vel[j]), xyz(pr));
+        dv += dot3_div<WHERE>(vi - xyz(f.vel[j]), xyz(pr));
     }
     return dv;
 }
@@ -309,7 +318,7 @@ __device__ __noinline__ R reread_div(const Fluid<R>& f, const Lists<R>& L, uint3
 // same list or cell walk as velocity_div_one).
 // CAND (scenes with non-pressure forces): also the candidate list those
 // forces' passes visit, every candidate within their cull.
-template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1, bool POOL = false, bool CAND = false>
+template <typename R, bool FAST = false, bool DIV0 = false, int EB = 1, Rounding WHERE = kOneScene, bool CAND = false>
 __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                                 const GridView& g, const uint32_t* __restrict__ cs,
                                                 const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
@@ -345,7 +354,7 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             }
             if (cnt < L.kmax) L.pairs[(size_t)cnt * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j)};
             ++cnt;
-            if constexpr (DIV0) dv += dot3_div<POOL>(vi - vj, mg);
+            if constexpr (DIV0) dv += dot3_div<WHERE>(vi - vj, mg);
         }
     };
     // phase 1: cull.  The half-precision cull needs all 27 cells inside the
@@ -481,8 +490,8 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             *div0 = d.dv;
             *nn0 = d.nn;
         } else {
-            if (nq > qcap) dv = reread_div<R, POOL>(f, L, i, vi, cnt);
-            if (akinci) dv += dot3_div<POOL>(vi, bg);
+            if (nq > qcap) dv = reread_div<R, WHERE>(f, L, i, vi, cnt);
+            if (akinci) dv += dot3_div<WHERE>(vi, bg);
             *div0 = dv;
             *nn0 = cnt;
         }
@@ -550,7 +559,7 @@ __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<
     if (i < f.count()) {
         R dv = 0;
         uint32_t nn = 0;
-        build_lists_one<R, sizeof(R) == 4, DIV0, EB, false, CAND>(i, f, bpos, g, cs, bs, c, akinci, L, q, kBlock, kQueue, &dv,
+        build_lists_one<R, sizeof(R) == 4, DIV0, EB, kOneScene, CAND>(i, f, bpos, g, cs, bs, c, akinci, L, q, kBlock, kQueue, &dv,
                                                                   &nn, o);
         if (DIV0) err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
     }
@@ -577,10 +586,6 @@ __global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<
 // FP64 parity form (compiled without contraction)
 __device__ __forceinline__ float mul_add(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double mul_add(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
-
-// |a|^2 as build_lists_one rounds it for the sum of the gradients
-__device__ __forceinline__ float sum_sq(V3<float> a) { return __fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))); }
-__device__ __forceinline__ double sum_sq(V3<double> a) { return dot3(a, a); }
 
 constexpr uint32_t kWideBlock = 128, kWideChunk = 32;
 
@@ -893,7 +898,7 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
             const R m = sqrt(dot3(sumGrad, sumGrad));
             den = m * m + sumSq;
         } else {
-            den = sum_sq(sumGrad) + sumSq;
+            den = dot3_zyx(sumGrad, sumGrad) + sumSq;  // (build_lists_one's rounding)
         }
         f.alpha[i] = (fabs(den) > c.eps) ? density / den : (R)0;
         L.count[i] = cnt;
@@ -982,13 +987,79 @@ __device__ __noinline__ DivSum<R> velocity_div_cells(const Fluid<R>& f, const P4
 
 // ---- list walks ------------------------------------------------------------
 
+// The FP32 passes stream a particle's records through a ring in shared memory
+// filled by asynchronous copies: kRingBatch records are used while the next
+// kRingDepth - kRingBatch are on their way, which needs no registers.  Loaded
+// into registers, the records in flight and the gathers behind them take turns.
+// One scene, us/step: 13,000 particles 132 -> 122, 125,000 259 -> 254,
+// 1,000,000 1441 -> 1368 (corrections at 6.6 TB/s of records and fields).
+// Each thread copies and reads its own column of the ring, so no block
+// synchronisation is needed; a slot is refilled only after the gathers that
+// depend on its record have been issued.
+constexpr int kRingDepth = 8, kRingBatch = 4;
+template <typename R> struct Ring {};
+template <> struct Ring<float> {
+    float4* slot;    // this thread's first slot; slots are `stride` apart
+    uint32_t stride;
+};
+__device__ __forceinline__ void copy_async16(float4* dst, const P4<float>* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+template <typename R> __device__ __forceinline__ Ring<R> make_ring(float4* slots, uint32_t block)
+{
+    if constexpr (sizeof(R) == 4) return Ring<float>{slots + threadIdx.x, block};
+    else return Ring<R>{};
+}
+
+// Records p[k * n], k < cnt, a batch at a time: load(j) starts the gather of a
+// record's neighbour j, eval(record, loaded) uses it, in list order.
+template <typename Load, typename Eval>
+__device__ __forceinline__ void stream_pairs(const Ring<float>& ring, const P4<float>* __restrict__ p, size_t n, uint32_t cnt,
+                                             uint32_t nj, unsigned* fault, Load&& load, Eval&& eval)
+{
+    constexpr int D = kRingDepth, B = kRingBatch;
+    static_assert(D == 2 * B, "one batch on its way while one is used");
+    auto fill = [&](uint32_t k0) {
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            if (k0 + b < cnt) copy_async16(ring.slot + ((k0 + b) % D) * ring.stride, p + (size_t)(k0 + b) * n);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fill(0);
+    fill(B);
+#pragma unroll 1
+    for (uint32_t k = 0; k < cnt; k += B) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        float4 r[B];
+        decltype(load(0u)) v[B];
+        bool ok[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            ok[b] = k + b < cnt;
+            if (ok[b]) {
+                r[b] = ring.slot[((k + b) % D) * ring.stride];
+                const uint32_t j = __float_as_uint(r[b].w);
+                ok[b] = SPH_INDEX_OK(j, nj, fault);
+                if (ok[b]) v[b] = load(j);
+            }
+        }
+        fill(k + D);
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+            if (ok[b]) eval(V3<float>{r[b].x, r[b].y, r[b].z}, v[b]);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // DFSPH velocity corrections (MODE 0 warm start, 1 density, 2 divergence),
 // as k_dfsph_correct but over the pair lists; kbuf holds this pass's k.
 template <typename R, int MODE>
 __device__ __forceinline__ V3<R> correct_sum_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                                  const GridView& g, const uint32_t* __restrict__ cs,
                                                  const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
-                                                 const Lists<R>& L)
+                                                 const Lists<R>& L, const Ring<R>& ring)
 {
     const uint32_t n = f.n;
     const R* __restrict__ kb_ = L.kbuf;
@@ -997,13 +1068,21 @@ __device__ __forceinline__ V3<R> correct_sum_one(uint32_t i, const Fluid<R>& f, 
     V3<R> sum = {0, 0, 0};
     if (cnt <= L.kmax) {
         const P4<R>* __restrict__ p = L.pairs + i;
+        if constexpr (sizeof(R) == 4) {
+            stream_pairs(ring, p, n, cnt, n, L.fault, [&](uint32_t j) { return __ldg(kb_ + j); },
+                         [&](V3<R> g, R kj) {
+                             const R kSum = ki + kj;
+                             if (fabs(kSum) > c.eps) sum = sum + kSum * g;
+                         });
+        } else {
 #pragma unroll 8
-        for (uint32_t k = 0; k < cnt; ++k) {
-            const P4<R> q = ldcs4(p + (size_t)k * n);
-            const uint32_t j = as_idx(q.w);
-            if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-            const R kSum = ki + __ldg(kb_ + j);
-            if (fabs(kSum) > c.eps) sum = sum + kSum * xyz(q);
+            for (uint32_t k = 0; k < cnt; ++k) {
+                const P4<R> q = ldcs4(p + (size_t)k * n);
+                const uint32_t j = as_idx(q.w);
+                if (!SPH_INDEX_OK(j, n, L.fault)) continue;
+                const R kSum = ki + __ldg(kb_ + j);
+                if (fabs(kSum) > c.eps) sum = sum + kSum * xyz(q);
+            }
         }
         const R kb = MODE == 0 ? c.bwarm * ki : ki;
         if (akinci && fabs(kb) > c.eps) sum = sum + kb * xyz(L.bgrad[i]);
@@ -1034,44 +1113,52 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_correct_list(Fluid<R> f, co
                                                                   Lists<R> L)
 {
     grid_wait();
+    __shared__ float4 slots[sizeof(R) == 4 ? kRingDepth * kBlock : 1];
     if (MODE != 0 && !sc->active) return;
-    const uint32_t i = gtid();
+    const uint32_t i = gtid_back();
     if (i >= f.count()) return;
-    const V3<R> sum = correct_sum_one<R, MODE>(i, f, bpos, g, cs, bs, c, akinci, L);
+    const V3<R> sum = correct_sum_one<R, MODE>(i, f, bpos, g, cs, bs, c, akinci, L, make_ring<R>(slots, kBlock));
     correct_apply<R, MODE>(i, f, c, (R)sc->dt, sum);
 }
 
 // Sum over the list of m (v_i - v_j) . gradW_ij plus the boundary term.
-template <typename R, bool POOL = false>
-__device__ __forceinline__ R velocity_div_list(const Fluid<R>& f, const Lists<R>& L, uint32_t i, V3<R> vi, int akinci)
+template <typename R, Rounding WHERE = kOneScene>
+__device__ __forceinline__ R velocity_div_list(const Fluid<R>& f, const Lists<R>& L, uint32_t i, V3<R> vi, int akinci,
+                                               const Ring<R>& ring)
 {
     const uint32_t n = f.n;
     const uint32_t cnt = L.count[i];
     const P4<R>* __restrict__ p = L.pairs + i;
     R d = 0;
+    if constexpr (sizeof(R) == 4 && WHERE == kOneScene) {
+        const P4<R>* vel = f.vel;
+        stream_pairs(ring, p, n, cnt, n, L.fault, [&](uint32_t j) { return xyz(ldg4(vel + j)); },
+                     [&](V3<R> g, V3<R> vj) { d += dot3_div(vi - vj, g); });
+    } else {
 #pragma unroll 8
-    for (uint32_t k = 0; k < cnt; ++k) {
-        const P4<R> q = ldcs4(p + (size_t)k * n);
-        const uint32_t j = as_idx(q.w);
-        if (!SPH_INDEX_OK(j, n, L.fault)) continue;
-        d += dot3_div<POOL>(vi - xyz(ldg4(f.vel + j)), xyz(q));
+        for (uint32_t k = 0; k < cnt; ++k) {
+            const P4<R> q = ldcs4(p + (size_t)k * n);
+            const uint32_t j = as_idx(q.w);
+            if (!SPH_INDEX_OK(j, n, L.fault)) continue;
+            d += dot3(vi - xyz(ldg4(f.vel + j)), xyz(q));
+        }
     }
-    if (akinci) d += dot3_div<POOL>(vi, xyz(L.bgrad[i]));
+    if (akinci) d += dot3_div<WHERE>(vi, xyz(L.bgrad[i]));
     return d;
 }
 
 // m (v_i - v_j) . gradW summed over the neighbours (list or fallback walk);
 // *nn receives the number of neighbours with a non-zero gradient.
-template <typename R, bool POOL = false>
+template <typename R, Rounding WHERE = kOneScene>
 __device__ __forceinline__ R velocity_div_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                               const GridView& g, const uint32_t* __restrict__ cs,
                                               const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
-                                              const Lists<R>& L, V3<R> vi, uint32_t* nn)
+                                              const Lists<R>& L, V3<R> vi, uint32_t* nn, const Ring<R>& ring)
 {
     const uint32_t cnt = L.count[i];
     if (cnt <= L.kmax) {
         *nn = cnt;
-        return velocity_div_list<R, POOL>(f, L, i, vi, akinci);
+        return velocity_div_list<R, WHERE>(f, L, i, vi, akinci, ring);
     }
     const DivSum<R> d = velocity_div_cells(f, bpos, g, cs, bs, c, akinci, i, vi);
     *nn = d.nn;
@@ -1088,6 +1175,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_predict_density_list(Fluid<
                                                                        Lists<R> L)
 {
     grid_wait();
+    __shared__ float4 slots[sizeof(R) == 4 ? kRingDepth * kBlock : 1];
     __shared__ double sh[33];
     if (!INITIAL && !sc->active) return;
     const uint32_t i = gtid();
@@ -1095,7 +1183,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_predict_density_list(Fluid<
     if (i < f.count()) {
         const V3<R> vi = xyz(f.vel[i]);
         uint32_t nn;
-        const R dc = velocity_div_one(i, f, bpos, g, cs, bs, c, akinci, L, vi, &nn);
+        const R dc = velocity_div_one(i, f, bpos, g, cs, bs, c, akinci, L, vi, &nn, make_ring<R>(slots, kBlock));
         const R dt = (R)sc->dt;
         const R rho = f.rho[i];
         R pred = rho + dc * dt;
@@ -1137,6 +1225,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f,
                                                                   Lists<R> L)
 {
     grid_wait();
+    __shared__ float4 slots[sizeof(R) == 4 ? kRingDepth * kBlock : 1];
     __shared__ double sh[33];
     if (!sc->active) return;
     const uint32_t i = gtid();
@@ -1144,7 +1233,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f,
     if (i < f.count()) {
         const V3<R> vi = xyz(f.vel[i]);
         uint32_t nn;
-        const R dv = velocity_div_one(i, f, bpos, g, cs, bs, c, akinci, L, vi, &nn);
+        const R dv = velocity_div_one(i, f, bpos, g, cs, bs, c, akinci, L, vi, &nn, make_ring<R>(slots, kBlock));
         err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
     }
     double total;

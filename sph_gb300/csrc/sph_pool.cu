@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_build_lists(Fluid<float> f
         if (sd.running) {
             float d = 0.f;
             uint32_t nn = 0;
-            build_lists_one<float, true, DIV0, 1, true>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c, sd.akinci, L,
+            build_lists_one<float, true, DIV0, 1, kPool>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c, sd.akinci, L,
                                                q, (uint32_t)BLOCK, qdepth, &d, &nn);
             if constexpr (DIV0) {
                 // the divergence solve's first error pass (k_pool_errors<true,
@@ -468,12 +468,13 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_correct(Fluid<float> f, co
                                                             Lists<float> L)
 {
     grid_wait();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ float4 slots[kRingDepth * BLOCK];
+    const uint32_t i = gtid_back();
     if (i >= f.n) return;
     const PoolScene& sd = T[sid[i]];
     if (!sd.running || (MODE != 0 && !sd.loop_active)) return;
     const V3<float> sum = correct_sum_one<float, MODE>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c,
-                                                       sd.akinci, L);
+                                                       sd.akinci, L, make_ring<float>(slots, BLOCK));
     correct_apply<float, MODE>(i, f, sd.c, (float)sd.s.dt, sum);
 }
 
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_pool_errors(Fluid<float> f, con
             const float dt = (float)sd.s.dt;
             const V3<float> vi = xyz(f.vel[i]);
             uint32_t nn;
-            float d = velocity_div_one<float, true>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, c, sd.akinci, L, vi, &nn);
+            float d = velocity_div_one<float, kPool>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, c, sd.akinci, L, vi, &nn, Ring<float>{});
             // the particle's relative error in FP32 (FP64 arithmetic is slow on
             // this part); its fixed-point quantum 2^-28 is still far coarser
             // than the FP32 rounding of an error of order 1e-3
@@ -1485,13 +1486,15 @@ private:
         else SPH_BUILD(256, 3);
 #undef SPH_BUILD
     }
+    // (the corrections hold 8 ring slots a thread in shared memory and need
+    // their 64 registers: below that they spill, so 1536 and 2048 threads per
+    // SM select the same kernel)
     template <int MODE> void launch_correct(Fluid<float> f, const P4<float>* bp, Lists<float> L)
     {
-        const int sb = tune_.solver_block, so = tune_.solver_occ;
 #define SPH_CORR(BL, MB) \
     launch(k_pool_correct<BL, MB, MODE>, blocks(N_, BL), BL, 0, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
-        if (sb == 128) { if (so == 1536) SPH_CORR(128, 12); else if (so == 2048) SPH_CORR(128, 16); else SPH_CORR(128, 8); }
-        else { if (so == 1536) SPH_CORR(256, 6); else if (so == 2048) SPH_CORR(256, 8); else SPH_CORR(256, 4); }
+        if (tune_.solver_block == 128) SPH_CORR(128, 8);
+        else SPH_CORR(256, 4);
 #undef SPH_CORR
     }
     template <bool DIV, bool INITIAL> void launch_errors(Fluid<float> f, const P4<float>* bp, Lists<float> L)
