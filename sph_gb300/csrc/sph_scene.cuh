@@ -1588,20 +1588,31 @@ private:
         Fluid<R> f = F();
         const P4<R>* bp = bd_[1].pos;
         const R* dp = bdp();
-        {
-            auto ph = phase("Pressure force");
-            withGL([&](auto gt, auto lt) {
+        if (cands_ && (c_.force_flags & ~F_BVISC) == F_XSPH) {
+            // both forces from one visit (the host-driven step's timers name them together)
+            auto ph = phase("Pressure force+NPForces");
+            withG([&](auto gt) {
                 constexpr int G = decltype(gt)::value;
-                constexpr bool LISTS = decltype(lt)::value;
-                run("k_wcsph_pressure_force", [&] { launch(k_wcsph_pressure_force<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, dp, CL()); });
+                run("k_wcsph_forces", [&] { launch(k_wcsph_forces<R, G>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p,
+                                                   CL()); });
             });
             SPH_CUDA(cudaGetLastError());
+        } else {
+            {
+                auto ph = phase("Pressure force");
+                withGL([&](auto gt, auto lt) {
+                    constexpr int G = decltype(gt)::value;
+                    constexpr bool LISTS = decltype(lt)::value;
+                    run("k_wcsph_pressure_force", [&] { launch(k_wcsph_pressure_force<R, G, LISTS>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, dp, CL()); });
+                });
+                SPH_CUDA(cudaGetLastError());
+            }
+            {
+                auto ph = phase("NPForces");
+                rc = launch_npforces();
+            }
+            if (rc) return rc;
         }
-        {
-            auto ph = phase("NPForces");
-            rc = launch_npforces();
-        }
-        if (rc) return rc;
         {
             auto ph = phase("Integratio");
             run("k_integrate", [&] { launch(k_integrate<R, false>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p); });
