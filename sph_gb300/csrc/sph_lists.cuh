@@ -231,6 +231,16 @@ template <typename R> struct BuildSums {
     uint32_t cnt;
 };
 
+// A record stored in 16-byte parts.  In build_walk_all the compiler (CUDA 13.0)
+// left out the one 32-byte store of an FP64 record in all but one of its
+// callers' forms: right sums, and lists of whatever the memory held.
+__device__ __forceinline__ void store_record(P4<float>* d, V3<float> v, uint32_t j) { *d = P4<float>{v.x, v.y, v.z, idx_as(0.f, j)}; }
+__device__ __forceinline__ void store_record(P4<double>* d, V3<double> v, uint32_t j)
+{
+    asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(d), "d"(v.x), "d"(v.y) : "memory");
+    asm volatile("st.global.v2.f64 [%0 + 16], {%1, %2};" ::"l"(d), "d"(v.z), "d"(idx_as(0.0, j)) : "memory");
+}
+
 // Particles whose candidates overflow the shared queue: the whole
 // evaluation inside the walk.  Out of line, so the common path's register
 // allocation does not carry it.
@@ -259,7 +269,7 @@ __device__ __noinline__ BuildSums<R> build_walk_all(uint32_t i, const Fluid<R>& 
             } else {
                 b.sumSq += mg2;
             }
-            if (b.cnt < L.kmax) L.pairs[(size_t)b.cnt * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j)};
+            if (b.cnt < L.kmax) store_record(L.pairs + (size_t)b.cnt * n + i, mg, j);
             ++b.cnt;
         }
     });

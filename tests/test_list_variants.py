@@ -6,6 +6,7 @@
 * The list build with 8, 4 and 1 lanes per particle (chosen by scene size), with lists that hold every neighbour and
   lists that overflow.
 * Candidate lists built and visited by several lanes per particle.
+* Particles whose candidates overflow the build's queue but whose neighbours fit the list.
 """
 import numpy as np
 import pytest
@@ -124,3 +125,33 @@ def test_candidate_lists_shared_by_lanes(gpu_lib, method, precision, lanes, list
     if method == "wcsph":
         # p = k ((rho / rho0)^7 - 1), k = 1.43e5: 7 k 64 eps; 64 terms of 2 p / rho^2 times m |grad W| <= 500; dt
         assert np.abs(v - v0).max() <= 7 * 1.43e5 * 64 * eps * 2 / 1e6 * 64 * 500 * 1e-4
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("side", [7, 17, 31])  # 8, 4 lanes and 1 lane per particle
+def test_lists_of_particles_whose_queue_overflows(gpu_lib, precision, side):
+    """Slots for about the number of neighbours: more candidates than the queue holds, in particles whose lists still
+    fit.  What is stored is what long lists hold, at the start and after a step's build."""
+    r = 0.01
+    e = 2 * r * (side + 1) + 1e-9
+    x = jitter(lattice(r, (2 * r, 2 * r, 2 * r), (e, e, e)), r, 3)
+    assert len(x) == side**3
+    v = np.random.default_rng(side).uniform(-0.2, 0.2, x.shape)
+    b = sph_gb300.sample_box(4 * r, (0, 0, 0), (e + 2 * r, e + 2 * r, e + 2 * r))
+
+    def lists(kmax, steps):
+        s = sph_gb300.Scene(neighbor_list_max=kmax, method=2, boundary=2, radius=r, precision=precision, max_it=0, min_it=0,
+                            max_it_v=0, min_it_v=0)
+        s.set_fluid(x, v)
+        s.add_boundary_points(b)
+        s.init()
+        if steps:
+            s.step(steps)
+        return s.pair_lists()
+
+    for steps in (0, 1):
+        a, w = lists(30, steps), lists(64, steps)
+        assert np.array_equal(a["count"], w["count"])
+        fits = w["count"] <= 30
+        assert fits.any() and not fits.all()
+        assert np.array_equal(a["nbr"], w["nbr"][np.repeat(fits, w["count"])])
