@@ -1460,6 +1460,15 @@ private:
             else if (per == 16) launch(k_scan_tiles<16>, nt, kScanThreads, 0, K_, count_.p, out, tile_sums_.p);
             else launch(k_scan_tiles<8>, nt, kScanThreads, 0, K_, count_.p, out, tile_sums_.p);
         });
+        if (nt <= kScanFused) {
+            run("k_scan_add", [&] {
+                if (per == 4) launch(k_scan_finish<4>, nt, kScanThreads, 0, K_, tile_sums_.p, out);
+                else if (per == 16) launch(k_scan_finish<16>, nt, kScanThreads, 0, K_, tile_sums_.p, out);
+                else launch(k_scan_finish<8>, nt, kScanThreads, 0, K_, tile_sums_.p, out);
+            });
+            SPH_CUDA(cudaGetLastError());
+            return SPH_OK;
+        }
         run("k_scan_tile_sums", [&] { launch(k_scan_tile_sums, 1, 1024, 0, nt, tile_sums_.p, out, K_); });
         run("k_scan_add", [&] {
             if (per == 4) launch(k_scan_add<4>, nt, kScanThreads, 0, K_, tile_sums_.p, out);

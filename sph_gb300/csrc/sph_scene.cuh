@@ -1046,11 +1046,18 @@ private:
     {
         const unsigned nt = blocks(nkeys_, kScanTile);
         run("k_scan_tiles", [&] { launch(k_scan_tiles<>, nt, kScanThreads, 0, nkeys_, count_.p, out, tile_sums_.p); });
-        run("k_scan_tile_sums", [&] { launch(k_scan_tile_sums, 1, 1024, 0, nt, tile_sums_.p, out, nkeys_); });
-        run("k_scan_add", [&] { launch(k_scan_add<>, nt, kScanThreads, 0, nkeys_, tile_sums_.p, out); });
+        if (nt <= kScanFused) {
+            run("k_scan_add", [&] { launch(k_scan_finish<>, nt, kScanThreads, 0, nkeys_, tile_sums_.p, out); });
+        } else {
+            run("k_scan_tile_sums", [&] { launch(k_scan_tile_sums, 1, 1024, 0, nt, tile_sums_.p, out, nkeys_); });
+            run("k_scan_add", [&] { launch(k_scan_add<>, nt, kScanThreads, 0, nkeys_, tile_sums_.p, out); });
+        }
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
+
+    // the step's bookkeeping is done by the kernel that moves the particles
+    bool finish_early() const { return !bh_ && !nem_; }
 
     // SPHSolver::insertFluidParticles + neighborhoodSearch
     // (SPHSolver.cpp:172-221): recompute cells (after the position update
@@ -1062,10 +1069,10 @@ private:
         if (bh_) run("k_bh_epoch", [&] { launch(k_bh_epoch, 1, 1, 0, sc_.p); });
         if (move)
             run("k_cell_update", [&] { launch(k_cell_update<R, true>, blocks(n_, 256), 256, 0, n_, a.pos, a.vel, a.cell, key_.p, slot_.p, count_.p, gv_,
-                                                                     c_.h, hd_, sc_.p, ce, nullptr, a.na); });
+                                                                     c_.h, hd_, sc_.p, ce, nullptr, a.na, (int)finish_early()); });
         else
             run("k_cell_update", [&] { launch(k_cell_update<R, false>, blocks(n_, 256), 256, 0, n_, a.pos, a.vel, a.cell, key_.p, slot_.p, count_.p,
-                                                                      gv_, c_.h, hd_, sc_.p, ce, nullptr, a.na); });
+                                                                      gv_, c_.h, hd_, sc_.p, ce, nullptr, a.na, 0); });
         SPH_CUDA(cudaGetLastError());
         int rc = scan(starts_.p);
         if (rc) return rc;
@@ -1203,7 +1210,7 @@ private:
         P4<R>* carry = MODE == 1 ? f.predR : nullptr;
         run("k_cell_update", [&] { launch(k_cell_update<R, MOVE, false>, blocks(n_, 256), 256, 0, n_, f.pos, f.vel, f.cell, key_.p, slot_.p,
                                                                                              count_.p, gv_, c_.h, hd_, sc_.p, nullptr,
-                                                                                             carry, f.na); });
+                                                                                             carry, f.na, 0); });
         run("k_bh_collide", [&] { launch(k_bh_collide<R, MODE>, blocks(n_, 128), 128, 0, f, B(1), gv_, bstarts_.p, c_, sc_.p,
                                                                                           cell_epoch_.p); });
         if (VEL) run("k_bh_correct_velocities", [&] { launch(k_bh_correct_velocities<R, PRED>, blocks(n_, 256), 256, 0, f, c_); });
@@ -1228,7 +1235,7 @@ private:
             Fluid<R> f = F();
             run("k_cell_update", [&] { launch(k_cell_update<R, true, false>, blocks(n_, 256), 256, 0, n_, f.pos, f.vel, f.cell, key_.p, slot_.p,
                                                                                               count_.p, gv_, c_.h, hd_, sc_.p, nullptr,
-                                                                                              nullptr, f.na); });
+                                                                                              nullptr, f.na, 0); });
         }
         launch_emit();  // Simulation::emitParticles DFSPHSolver.cpp:77, before the grid fill
         auto ph = phase("Fill grid");
@@ -1353,7 +1360,7 @@ private:
             auto ph = phase("Boundary handling");
             run("k_dfsph_cube", [&] { launch(k_dfsph_cube<R>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_); });
         }
-        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
+        if (!finish_early()) run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1565,7 +1572,7 @@ private:
             auto ph = phase("Boundary handling");
             run("k_dfsph_cube", [&] { launch(k_dfsph_cube<R>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_); });
         }
-        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
+        if (!finish_early()) run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1615,14 +1622,14 @@ private:
         }
         {
             auto ph = phase("Integratio");
-            run("k_integrate", [&] { launch(k_integrate<R, false>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p); });
+            run("k_integrate", [&] { launch(k_integrate<R, false>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p, (int)finish_early()); });
         }
         if (bh_) {
             auto ph = phase("Boundary Handling");
             launch_bh_after_move<false, 0, true, false>();  // WCSPHSolver.cpp:62-72
         }
         launch_emit();  // WCSPHSolver.cpp:75
-        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
+        if (!finish_early()) run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
@@ -1687,14 +1694,14 @@ private:
         if (rc) return rc;
         {
             auto ph = phase("Integration");
-            run("k_integrate", [&] { launch(k_integrate<R, true>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p); });
+            run("k_integrate", [&] { launch(k_integrate<R, true>, blocks(n_, 256), 256, 0, f, gv_, hd_, c_, sc_.p, (int)finish_early()); });
         }
         if (bh_) {
             auto ph = phase("Boundary handling");
             launch_bh_after_move<false, 1, true, true>();  // PCISPHSolver.cpp:65-75
         }
         launch_emit();  // PCISPHSolver.cpp:78
-        run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
+        if (!finish_early()) run("k_finish_step", [&] { launch(k_finish_step, 1, 1, 0, sc_.p); });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }

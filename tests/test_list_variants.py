@@ -7,6 +7,7 @@
   lists that overflow.
 * Candidate lists built and visited by several lanes per particle.
 * Particles whose candidates overflow the build's queue but whose neighbours fit the list.
+* The grid's key scan in two launches and in three, at the edges of its tiles.
 """
 import numpy as np
 import pytest
@@ -155,3 +156,30 @@ def test_lists_of_particles_whose_queue_overflows(gpu_lib, precision, side):
         fits = w["count"] <= 30
         assert fits.any() and not fits.all()
         assert np.array_equal(a["nbr"], w["nbr"][np.repeat(fits, w["count"])])
+
+
+@pytest.mark.parametrize("cells", [(8, 5), (8, 32), (8, 33), (16, 40), (64, 512), (64, 513)])
+def test_key_scan_tiles(gpu_lib, cells):
+    """A part of a 2048-key tile, one tile, one and a part, five, 1024 (the last with the scan's sums folded into its
+    second launch) and 1026, against the same particles in a box of 128 columns a side and at least 1100 tiles: the
+    same neighbours, summed in another order (at most 60 terms)."""
+    side, nz = cells
+    r = 0.02
+    h = 4 * r
+    rng = np.random.default_rng(side * nz)
+    top = (nz - 4) * h
+    x = rng.uniform((0, 0, 0), (3 * h, 3 * h, min(top, 4 * h)), (60, 3))
+    x[30:, 2] = top - x[30:, 2]  # at both ends of the keys
+    x = np.clip(x, 1e-3 * h, (3.999 * h, 3.999 * h, top - 1e-3 * h))
+
+    def density(s, z):
+        lo = (0.5 * h, 0.5 * h, 0.5 * h)
+        hi = ((s - 4.5) * h, (s - 4.5) * h, (z - 4.5) * h)
+        sc = sph_gb300.Scene(method=0, boundary=2, radius=r, precision="f64", dt=1e-5, domain_min=lo, domain_max=hi)
+        sc.set_fluid(x)
+        sc.init()
+        sc.step(1)
+        return sc.get("rho")
+
+    a, w = density(side, nz), density(128, max(nz, 138))
+    assert np.abs(a - w).max() <= 60 * 2.0**-53 * np.abs(w).max()
