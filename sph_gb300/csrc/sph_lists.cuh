@@ -554,22 +554,21 @@ __device__ __forceinline__ void divergence_control(DevScalars* sc, const LoopLim
 // (9 FP64 operations on each of ~150 candidates, at two FP64 lanes per SM)
 // was a third of the build: 125k particles 1454 -> 1003 us with the boundary's
 // cull and the fused error pass.
-template <typename R, bool DIV0, bool CAND>
-__global__ void __launch_bounds__(kBlock, 7) k_build_lists(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
+template <typename R, bool DIV0, bool CAND, int BLOCK, int MINB, int EB, int QD>
+__global__ void __launch_bounds__(BLOCK, MINB) k_build_lists(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                            const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                            Consts<R> c, int akinci, Lists<R> L, DevScalars* sc,
                                                            LoopLimits lim, double* partials, cudaGraphConditionalHandle cond,
                                                            CandOut o)
 {
     grid_wait();
-    __shared__ uint32_t q[kQueue * kBlock];
+    __shared__ uint32_t q[QD * BLOCK];
     const uint32_t i = gtid();
-    constexpr int EB = sizeof(R) == 4 ? 4 : 2;
     double err = 0.0;
     if (i < f.count()) {
         R dv = 0;
         uint32_t nn = 0;
-        build_lists_one<R, sizeof(R) == 4, DIV0, EB, kOneScene, CAND>(i, f, bpos, g, cs, bs, c, akinci, L, q, kBlock, kQueue, &dv,
+        build_lists_one<R, sizeof(R) == 4, DIV0, EB, kOneScene, CAND>(i, f, bpos, g, cs, bs, c, akinci, L, q, BLOCK, QD, &dv,
                                                                   &nn, o);
         if (DIV0) err = divergence_error(i, f, L, c, (R)sc->dt, dv, nn);
     }

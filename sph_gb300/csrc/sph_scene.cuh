@@ -1168,10 +1168,26 @@ private:
             constexpr int W = decltype(wt)::value;
             constexpr bool CAND = decltype(ct)::value;
             run("k_build_lists", [&] {
-                if constexpr (W == 1)
-                    launch(k_build_lists<R, DIV0, CAND>, blocks(n_, kBlock), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L,
-                           sc_.p, lim_, partials_.p, h, CO());
-                else
+                if constexpr (W == 1) {
+                    constexpr int EB = kListBatch<R>;
+                    auto one = [&](auto kernel) {
+                        launch(kernel, blocks(n_, kBlock), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_,
+                               partials_.p, h, CO());
+                    };
+                    // FP64 above five blocks per SM: eight resident blocks (64
+                    // registers, 48 queue entries) instead of seven (72, 64),
+                    // 125,000 particles 1761 -> 1692 us/step; below, the
+                    // registers win.  FP32 keeps seven (125,000 particles would
+                    // gain 249 -> 232, but its sums round differently there and
+                    // the solvers carry that into everything that follows).
+                    if constexpr (sizeof(R) == 8) {
+                        if ((size_t)n_ > (size_t)sms_ * 5 * kBlock) {
+                            one(k_build_lists<R, DIV0, CAND, kBlock, 8, EB, 48>);
+                            return;
+                        }
+                    }
+                    one(k_build_lists<R, DIV0, CAND, kBlock, 7, EB, kQueue>);
+                } else
                     launch(k_build_lists_wide<R, W, DIV0>, blocks((size_t)n_ * W, kWideBlock), kWideBlock, 0, f, bp, gv_, starts_.p,
                            bstarts_.p, c_, hasb_, L, sc_.p, lim_, partials_.p, h);
             });

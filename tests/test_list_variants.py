@@ -7,6 +7,7 @@
   lists that overflow.
 * Candidate lists built and visited by several lanes per particle.
 * Particles whose candidates overflow the build's queue but whose neighbours fit the list.
+* The FP64 list build with eight blocks per SM, on either side of the size that chooses it.
 * The grid's key scan in two launches and in three, at the edges of its tiles.
 """
 import numpy as np
@@ -156,6 +157,34 @@ def test_lists_of_particles_whose_queue_overflows(gpu_lib, precision, side):
         fits = w["count"] <= 30
         assert fits.any() and not fits.all()
         assert np.array_equal(a["nbr"], w["nbr"][np.repeat(fits, w["count"])])
+
+
+@pytest.mark.parametrize("lists", [64, 24])
+def test_f64_build_by_size(gpu_lib, lists):
+    """Five blocks of 128 particles per SM, and the same with one particle more that is far from all others: FP64 is
+    compiled without contraction and the sums keep their order, so the two forms of the build agree bit for bit, with
+    lists that hold every neighbour and with lists (and candidate queues) that overflow."""
+    torch = pytest.importorskip("torch")
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 5 * 128
+    r = 0.01
+    side = int(np.ceil(n ** (1 / 3)))
+    e = 2 * r * (side + 1) + 1e-9
+    x = jitter(lattice(r, (2 * r, 2 * r, 2 * r), (e, e, e)), r, 3)[:n]
+    v = np.random.default_rng(n).uniform(-0.2, 0.2, x.shape)
+    b = sph_gb300.sample_box(4 * r, (0, 0, 0), (e + 2 * r, e + 2 * r, e + 2 * r))
+    x = np.vstack([x, [[e + 20 * r, e, e]]])
+    v = np.vstack([v, np.zeros((1, 3))])
+    out = []
+    for m in (n, n + 1):
+        s = sph_gb300.Scene(neighbor_list_max=lists, method=2, boundary=2, radius=r, precision="f64", eta=0.001, eta_v=0.001,
+                            max_it_v=0, min_it_v=0, domain_min=(-4 * r,) * 3, domain_max=(e + 30 * r,) * 3)
+        s.set_fluid(x[:m], v[:m])
+        s.add_boundary_points(b)
+        s.init()
+        s.step(1)
+        out.append([s.get(f)[:n] for f in ("rho", "alpha", "div", "v")])
+    for a, w in zip(*out):
+        assert np.array_equal(a, w)
 
 
 @pytest.mark.parametrize("cells", [(8, 5), (8, 32), (8, 33), (16, 40), (64, 512), (64, 513)])
