@@ -979,9 +979,13 @@ private:
         kmax_ = lists_ ? (uint32_t)d.neighbor_list_max : 0u;
         // candidate lists, PCISPH and WCSPH, and DFSPH for its non-pressure
         // forces: Akinci or no boundary (the PCISPH boundary model moves
-        // predicted positions after the prediction), indices below 2^27
+        // predicted positions after the prediction), indices below 2^27.  Not
+        // DFSPH in a cube: its clamp moves particles after the grid build whose
+        // candidates (and half-precision positions) the next step's forces
+        // would visit, so those walk the cells.
         cands_ = d.neighbor_list_max > 0 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask &&
-                 (d.simulation_method != SPH_DFSPH || (c_.force_flags != 0 && (G_ > 1 || build_lanes() == 1)));
+                 (d.simulation_method != SPH_DFSPH ||
+                  (c_.force_flags != 0 && !c_.has_cube && (G_ > 1 || build_lanes() == 1)));
         if (cands_) {
             // one lane: the whole list; G lanes: each twice its even share
             cslots_ = G_ == 1 ? (uint32_t)d.neighbor_list_max : std::max(1u, 2u * (uint32_t)d.neighbor_list_max / (unsigned)G_);
