@@ -470,15 +470,22 @@ __device__ __forceinline__ uint32_t final_slot(uint32_t p, const uint32_t* __res
     return s + rank;
 }
 
+// The power of two that brings the support radius into [1, 2).
+__device__ __forceinline__ float half_scale(float h) { return __uint_as_float((254u - (__float_as_uint(h) >> 23)) << 23); }
+
 // Half-precision copy of cell-relative positions, two points (2k, 2k+1) per
 // 16-byte word: {x pair, y pair, z pair, unused} as half2, z in the cell's
-// modulo-3 frame.
-__device__ __forceinline__ void store_half(uint4* __restrict__ posh, uint32_t d, float x, float y, float zf)
+// modulo-3 frame, in units in which the support radius is in [1, 2)
+// (half_scale): in metres the squares of the distances would leave half
+// precision's normal range below h = 8 mm (at particle radii around 0.1 mm the
+// cull lost pairs with q > 0.8) and the distances its whole range above 2e4 m.
+__device__ __forceinline__ void store_half(uint4* __restrict__ posh, uint32_t d, float x, float y, float zf, float h)
 {
+    const float sc = half_scale(h);
     __half* ph = reinterpret_cast<__half*>(posh) + (size_t)(d >> 1) * 8 + (d & 1);
-    ph[0] = __float2half_rn(x);
-    ph[2] = __float2half_rn(y);
-    ph[4] = __float2half_rn(zf);
+    ph[0] = __float2half_rn(x * sc);
+    ph[2] = __float2half_rn(y * sc);
+    ph[4] = __float2half_rn(zf * sc);
 }
 // the same from a stored point (FP32: cell-relative; FP64: absolute)
 template <typename R>
@@ -489,7 +496,7 @@ __device__ __forceinline__ void store_half_abs(uint4* __restrict__ posh, uint32_
     if constexpr (sizeof(R) == 8)
         o = {(float)(p.x - (double)(cell_x(c) + g.ox) * h), (float)(p.y - (double)(cell_y(c) + g.oy) * h),
              (float)(p.z - (double)(cell_z(c) + g.oz) * h)};
-    store_half(posh, d, o.x, o.y, zframe3(o.z, cell_z(c), (float)h));
+    store_half(posh, d, o.x, o.y, zframe3(o.z, cell_z(c), (float)h), (float)h);
 }
 
 // The boundary points' half-precision copy (they do not move: written once
@@ -505,11 +512,15 @@ __global__ void k_boundary_half(Boundary<R> b, GridView g, double h, uint4* __re
 // Gather of the state that survives a re-sort (x, v, DFSPH k, kv and the
 // last predicted density; the other fields are recomputed after every build).
 // posh (optional): also the half-precision copy of the positions the list
-// build culls with.
-template <typename R>
+// build culls with; support(i): the support radius of particle i's scene.
+struct OneSupport {
+    double h;
+    __device__ __forceinline__ double operator()(uint32_t) const { return h; }
+};
+template <typename R, typename Support>
 __global__ void k_gather_fluid(uint32_t n, const uint32_t* __restrict__ tmp, const uint32_t* __restrict__ key,
                                const uint32_t* __restrict__ starts, Fluid<R> src, Fluid<R> dst,
-                               uint4* __restrict__ posh = nullptr, GridView g = GridView{}, double h = 0.0)
+                               uint4* __restrict__ posh, GridView g, Support support)
 {
     grid_wait();
     const uint32_t p = gtid();
@@ -520,8 +531,8 @@ __global__ void k_gather_fluid(uint32_t n, const uint32_t* __restrict__ tmp, con
     dst.pos[d] = x;
     if (posh) {
         // (FP32: the cell update left z in the modulo-3 frame in w)
-        if constexpr (sizeof(R) == 4) store_half(posh, d, x.x, x.y, x.w);
-        else store_half_abs(posh, d, x, src.cell[i], g, h);
+        if constexpr (sizeof(R) == 4) store_half(posh, d, x.x, x.y, x.w, (float)support(i));
+        else store_half_abs(posh, d, x, src.cell[i], g, support(i));
     }
     dst.vel[d] = src.vel[i];
     dst.kappa[d] = src.kappa[i];

@@ -81,22 +81,37 @@ __device__ __forceinline__ uint32_t cell_code(uint32_t ci, uint32_t cj)
 //
 // The test uses r^2 <= 1.03 h^2: for a pair within h, half-precision values
 // (relative error 2^-11 each; x, y operands within 2.5h, z within 3h)
-// move r^2 by less than 1.7 % of h^2, so every pair the FP32 test accepts
+// move r^2 by less than 1.7 % of h^2, so every pair the exact test accepts
 // is kept; pairs beyond h evaluate to W = 0, grad W = 0 in phase 2 and are
-// dropped there.  Returns the number of accepted candidates (the queue
-// holds the first qcap).
+// dropped there.  Lengths are scaled by a power of two that brings h into
+// [1, 2) (half_scale; exact, so the same bound for any unit of length): the
+// values stay within 6 and their squares within 36, and half precision's
+// subnormal step of 6e-8 is nothing beside them.  Returns the number of
+// accepted candidates (the queue holds the first qcap).
 //
 // reach2: the square of the distance wanted, up to (1.1 h)^2 (candidate lists;
 // the same bounds scale to 1.9 % of h^2 against a slack of 3.6 %, and a true
 // |dz| above 1.9 h may read as little as h: such candidates are dropped by
 // the exact test on the queued ones).
-__device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
-
 //
 // RANK: each queued candidate with the lane whose part of a cell walk by
 // `lanes` lanes it is, above the index's 27 bits: its rank modulo the lanes
 // in its cell (kCellRank, the FP32 walk) or in its column (kColumnRank, FP64).
 enum Rank { kNoRank, kCellRank, kColumnRank };
+
+__device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+
+// The scaled quantities of the half-precision test of one particle.
+struct HalfTest {
+    float x, y, h;  // position in its cell's frame, support radius
+    __half2 zq, h3, thr;
+};
+__device__ __forceinline__ HalfTest half_test(V3<float> xi, int cz, float h, float reach2)
+{
+    const float sc = half_scale(h);
+    return HalfTest{xi.x * sc, xi.y * sc, h * sc, __float2half2_rn(zframe3(xi.z, cz, h) * sc), __float2half2_rn(3.f * h * sc),
+                    __float2half2_rn(reach2 * 1.03f * (sc * sc))};
+}
 
 template <Rank RANK = kNoRank>
 __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t* __restrict__ starts, uint32_t pc,
@@ -109,9 +124,7 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
     const float gym = ofy > 0.f ? ofy * ofy : 0.f, gyp = h - ofy > 0.f ? (h - ofy) * (h - ofy) : 0.f;
     const float gzm = ofz > 0.f ? ofz * ofz : 0.f, gzp = h - ofz > 0.f ? (h - ofz) * (h - ofz) : 0.f;
     const float lim = fmaxf(reach2, h * h) * (float)(1.0 + 1e-5);
-    const __half2 thr = __float2half2_rn(reach2 * 1.03f);
-    const __half2 zq = __float2half2_rn(zframe3(xi.z, cz, h));
-    const __half2 h3 = __float2half2_rn(3.f * h);
+    const HalfTest ht = half_test(xi, cz, h, reach2);
     uint32_t nq = 0;
     // a column's candidate range (empty when trimmed); loaded one column ahead
     auto range = [&](int c, uint32_t* b, uint32_t* e, uint32_t* s1, uint32_t* s2) {
@@ -134,7 +147,7 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
         const int dx = c / 3 - 1, dy = c - (c / 3) * 3 - 1;
         const uint32_t bb = nb, ee = ne, s1 = n1, s2 = n2;
         if (c < 8) range(c + 1, &nb, &ne, &n1, &n2);
-        const __half2 sx = __float2half2_rn(xi.x - (float)dx * h), sy = __float2half2_rn(xi.y - (float)dy * h);
+        const __half2 sx = __float2half2_rn(ht.x - (float)dx * ht.h), sy = __float2half2_rn(ht.y - (float)dy * ht.h);
         // The column's candidates 32 at a time (16 words): the test's
         // acceptance bits are gathered into one word, candidate j0 + b at
         // bit b, and only the accepted candidates (about one in five) are
@@ -146,10 +159,10 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
             auto test = [&](const uint4 w) {
                 const __half2 ddx = __hsub2(sx, as_half2(w.x));
                 const __half2 ddy = __hsub2(sy, as_half2(w.y));
-                const __half2 dz = __habs2(__hsub2(zq, as_half2(w.z)));
-                const __half2 ddz = __hmin2(dz, __hsub2(h3, dz));
+                const __half2 dz = __habs2(__hsub2(ht.zq, as_half2(w.z)));
+                const __half2 ddz = __hmin2(dz, __hsub2(ht.h3, dz));
                 const __half2 r2 = __hfma2(ddz, ddz, __hfma2(ddy, ddy, __hmul2(ddx, ddx)));
-                return __hle2_mask(r2, thr);
+                return __hle2_mask(r2, ht.thr);
             };
             // Two words (four candidates) per iteration: bytes 0 and 2 of
             // each mask (one per half) gathered into one word, then bit 8k+k
@@ -184,7 +197,8 @@ __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t*
 }
 
 // Whether the half-precision cull serves a particle (see cull_half), and its
-// position in its cell's frame.
+// position in its cell's frame.  (h beyond 1e15 either way: h^2 or its FP32
+// gaps leave FP32.)
 template <typename R>
 __device__ __forceinline__ bool half_cull_ok(const GridView& g, uint32_t pc, V3<R> xi, R h, V3<float>* xr)
 {
@@ -193,7 +207,7 @@ __device__ __forceinline__ bool half_cull_ok(const GridView& g, uint32_t pc, V3<
     else *xr = V3<float>{(float)(xi.x - (R)(cx + g.ox) * h), (float)(xi.y - (R)(cy + g.oy) * h),
                          (float)(xi.z - (R)(cz + g.oz) * h)};
     const float hf = (float)h, hh = 0.5f * hf;
-    return cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
+    return hf >= 1e-15f && hf <= 1e15f && cx >= 2 && cy >= 2 && cz >= 2 && cx <= g.nx - 3 && cy <= g.ny - 3 && cz <= g.nz - 3 &&
            fabsf(xr->x - hh) <= hf && fabsf(xr->y - hh) <= hf && fabsf(xr->z - hh) <= hf;
 }
 
@@ -647,9 +661,7 @@ template <int W, Rank RANK = kNoRank>
 __device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W, RANK>& rg, int cz, V3<float> xi, float h, float reach2,
                                                    const uint4* __restrict__ posh, uint32_t* q, uint32_t qcap)
 {
-    const __half2 thr = __float2half2_rn(reach2 * 1.03f);
-    const __half2 zq = __float2half2_rn(zframe3(xi.z, cz, h));
-    const __half2 h3 = __float2half2_rn(3.f * h);
+    const HalfTest ht = half_test(xi, cz, h, reach2);
     const int g0 = (int)(threadIdx.x & 31) & ~(W - 1);
     // the first round of every column's words, all in flight together
     uint4 w0[9];
@@ -668,16 +680,16 @@ __device__ __forceinline__ uint32_t cull_half_wide(int gl, const WideRanges<W, R
         uint32_t s1 = 0u, s2 = 0u;
         if constexpr (RANK) s1 = __shfl_sync(0xffffffffu, rg.m0[c / W], c % W, W);
         if constexpr (RANK == kCellRank) s2 = __shfl_sync(0xffffffffu, rg.m1[c / W], c % W, W);
-        const __half2 sx = __float2half2_rn(xi.x - (float)dx * h), sy = __float2half2_rn(xi.y - (float)dy * h);
+        const __half2 sx = __float2half2_rn(ht.x - (float)dx * ht.h), sy = __float2half2_rn(ht.y - (float)dy * ht.h);
         uint32_t word = (bb >> 1) + gl;
         uint4 w = w0[c];
         // rounds of W words; the warp runs the longest of its groups' columns
         while (__any_sync(0xffffffffu, 2 * (word - gl) < ee)) {
             const __half2 ddx = __hsub2(sx, as_half2(w.x)), ddy = __hsub2(sy, as_half2(w.y));
-            const __half2 dz = __habs2(__hsub2(zq, as_half2(w.z)));
-            const __half2 ddz = __hmin2(dz, __hsub2(h3, dz));
+            const __half2 dz = __habs2(__hsub2(ht.zq, as_half2(w.z)));
+            const __half2 ddz = __hmin2(dz, __hsub2(ht.h3, dz));
             const __half2 r2 = __hfma2(ddz, ddz, __hfma2(ddy, ddy, __hmul2(ddx, ddx)));
-            const unsigned m = __hle2_mask(r2, thr);
+            const unsigned m = __hle2_mask(r2, ht.thr);
             const uint32_t j = 2 * word;
             const bool a0 = (m & 1u) && j >= bb && j < ee;
             const bool a1 = (m & 0x10000u) && j + 1 < ee;

@@ -244,6 +244,13 @@ __global__ void k_pool_bcount(uint32_t N, Boundary<float> b, const uint32_t* __r
     slot[i] = atomicAdd(count + k, 1u);
 }
 
+// The support radius of the scene of particle i (k_gather_fluid).
+struct SceneSupport {
+    const uint32_t* sid;
+    const PoolScene* T;
+    __device__ __forceinline__ float operator()(uint32_t i) const { return T[sid[i]].c.h; }
+};
+
 // The boundary points' half-precision copy for the list build's boundary
 // cull (two points per 16-byte word, {x, y, z in the cell's modulo-3 frame},
 // as the fluid's copy): boundary points do not move, so it is written once
@@ -256,7 +263,7 @@ __global__ void k_pool_boundary_half(uint32_t N, Boundary<float> b, const uint32
     if (d >= N) return;
     const float h = T[bsid[d]].c.h;
     const P4<float> x = b.pos[d];
-    store_half(posh, d, x.x, x.y, zframe3(x.z, cell_z(b.cell[d]), h));
+    store_half(posh, d, x.x, x.y, zframe3(x.z, cell_z(b.cell[d]), h), h);
 }
 
 // AkinciBoundaryModel::computeVolume (AkinciBoundayModel.cpp:11-40) per scene.
@@ -1763,8 +1770,8 @@ private:
         int rc = scan(starts_.p);
         if (rc) return rc;
         run("k_scatter", [&] { launch(k_scatter, blocks(N_, 256), 256, 0, N_, key_.p, slot_.p, starts_.p, tmp_.p, nullptr); });
-        run("k_gather_fluid", [&] { launch(k_gather_fluid<float>, blocks(N_, 256), 256, 0, N_, tmp_.p, key_.p, starts_.p, F(cur_), F(1 - cur_),
-                                                                                          posh_.p, GridView{}, 0.0); });
+        run("k_gather_fluid", [&] { launch(k_gather_fluid<float, SceneSupport>, blocks(N_, 256), 256, 0, N_, tmp_.p, key_.p, starts_.p, F(cur_),
+                                           F(1 - cur_), posh_.p, GridView{}, SceneSupport{sid_.p, table_.p}); });
         SPH_CUDA(cudaGetLastError());
         cur_ = 1 - cur_;
         return SPH_OK;

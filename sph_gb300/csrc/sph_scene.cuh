@@ -1081,8 +1081,8 @@ private:
         int rc = scan(starts_.p);
         if (rc) return rc;
         run("k_scatter", [&] { launch(k_scatter, blocks(n_, 256), 256, 0, n_, key_.p, slot_.p, starts_.p, tmp_.p, a.na); });
-        run("k_gather_fluid", [&] { launch(k_gather_fluid<R>, blocks(n_, 256), 256, 0, n_, tmp_.p, key_.p, starts_.p, fl_[cur_], fl_[1 - cur_],
-                                                                                  posh_.p, gv_, hd_); });
+        run("k_gather_fluid", [&] { launch(k_gather_fluid<R, OneSupport>, blocks(n_, 256), 256, 0, n_, tmp_.p, key_.p, starts_.p, fl_[cur_],
+                                           fl_[1 - cur_], posh_.p, gv_, OneSupport{hd_}); });
         SPH_CUDA(cudaGetLastError());
         cur_ = 1 - cur_;
         return SPH_OK;
