@@ -228,12 +228,22 @@ template <typename T> struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
     ~DevBuf() { if (p) cudaFree(p); }
+    // n counts what p holds: 0 after a failure, so that a buffer kept between
+    // calls is allocated again by the next one (and the error is taken off the
+    // thread's last one, which the next launch check would report).
     cudaError_t alloc(size_t count)
     {
         if (p) cudaFree(p);
         p = nullptr;
-        n = count;
-        return cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T));
+        n = 0;
+        const cudaError_t e = cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T));
+        if (e == cudaSuccess) {
+            n = count;
+        } else {
+            p = nullptr;
+            cudaGetLastError();
+        }
+        return e;
     }
 };
 
@@ -687,10 +697,8 @@ public:
         if (!inited) { fail("not initialised"); return SPH_ERR_INVALID; }
         const unsigned n = active();
         *count_out = n;
-        if (cap_x_.n < 3 * (size_t)n_) {
-            SPH_CUDA(cap_x_.alloc(3 * (size_t)n_));
-            SPH_CUDA(cap_v_.alloc(3 * (size_t)n_));
-        }
+        if (cap_x_.n < 3 * (size_t)n_) SPH_CUDA(cap_x_.alloc(3 * (size_t)n_));
+        if (cap_v_.n < 3 * (size_t)n_) SPH_CUDA(cap_v_.alloc(3 * (size_t)n_));
         if (n) {
             Fluid<R> f = F();
             k_download<R><<<blocks(n, 256), 256, 0, st_>>>(n, f.pos, nullptr, f.id, f.cell, gv_, hd_, 1, cap_x_.p);

@@ -1,0 +1,70 @@
+"""Scenarios of tests/test_cuda_failures_host.py: run in a process of its own with SPH_GB300_LIBRARY naming the library
+linked against the fake CUDA runtime (tests/fake_cudart.cpp).  Prints one JSON line."""
+import ctypes
+import json
+import os
+import sys
+
+import numpy as np
+
+sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+
+import sph_gb300  # noqa: E402
+from scenes import lattice  # noqa: E402
+
+R = 0.02
+FORCES = dict(visc_method=2, visc=0.01, bvisc=0.01, st_method=3, st=0.5, adh_method=4, adh=0.1)
+SOLVERS = {
+    "dfsph": dict(method=2), "dfsph_f64": dict(method=2, precision="f64"), "dfsph_forces": dict(method=2, **FORCES),
+    "dfsph_walks": dict(method=2, neighbor_list_max=0, **FORCES), "wcsph": dict(method=0, visc_method=2, visc=0.01),
+    "wcsph_forces": dict(method=0, **FORCES), "pcisph": dict(method=1, min_it=1, **FORCES),
+}
+
+
+def fake():
+    f = ctypes.CDLL(os.environ["SPH_GB300_LIBRARY"])
+    f.fake_memory.argtypes = [ctypes.c_size_t]
+    f.fake_live_bytes.restype = f.fake_peak_bytes.restype = ctypes.c_size_t
+    return f
+
+
+def scene(n_side=6, **p):
+    s = sph_gb300.Scene(boundary=2, radius=R, **p)
+    s.set_fluid(lattice(R, (2 * R,) * 3, (2 * R + 2 * R * n_side + 1e-9,) * 3))
+    s.add_boundary_points(sph_gb300.sample_box(4 * R, (0, 0, 0), (0.6, 0.6, 0.6)))
+    s.init()
+    return s
+
+
+def failed(call):
+    try:
+        call()
+    except sph_gb300.SPHError:
+        return True
+    return False
+
+
+def downloads(F):
+    """A read whose staging buffer cannot be allocated fails; the next one works."""
+    s = scene(**SOLVERS["dfsph"])
+    P = sph_gb300.Pool(max_particles=1000, max_boundary=10_000, max_keys=100_000, max_scenes=2)
+    P.set_autotune(0)
+    P.set_graph(False)
+    k = P.add_scene(lattice(R, (2 * R,) * 3, (0.3,) * 3), boundary_points=sph_gb300.sample_box(4 * R, (0, 0, 0), (0.6, 0.6, 0.6)),
+                    steps=5, method=2, boundary=2, radius=R, precision="f32")
+    P.step(1)
+    out = {}
+    for name, get in (("scene", s.get), ("pool", lambda f: P.get(k, f))):
+        get("rho")
+        F.fake_fail_malloc(1)  # x needs a larger buffer than rho
+        first = failed(lambda: get("x"))
+        out[name] = [first, failed(lambda: get("x")), failed(lambda: get("rho"))]
+        out[name].append(failed(lambda: (s.step(1) if name == "scene" else P.step(1))))
+    out["null_uses"] = F.fake_null_uses()
+    return out
+
+
+if __name__ == "__main__":
+    F = fake()
+    print(json.dumps({"downloads": downloads}[sys.argv[1]](F)))

@@ -1,0 +1,40 @@
+"""Failing allocations and launches, on the CPU: the library's own objects linked against a fake of the CUDA runtime
+(tests/fake_cudart.cpp) that refuses a chosen one.
+
+* A read whose staging buffer cannot be allocated reports it; later reads allocate again and nothing uses a null buffer."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+from sph_gb300 import buildlib
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA = os.path.dirname(os.path.dirname(buildlib.nvcc()))
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    buildlib.build()
+    objs = [os.path.join(buildlib.OBJDIR, os.path.splitext(u)[0] + ".o") for u in buildlib.UNITS]
+    lib = str(tmp_path_factory.mktemp("fake") / "libsph_fake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(CUDA, "include"), "-o", lib,
+                    os.path.join(HERE, "fake_cudart.cpp"), *objs, "-lpthread", "-ldl"], check=True, capture_output=True, text=True)
+
+    def go(scenario):
+        p = subprocess.run([sys.executable, os.path.join(HERE, "cuda_failures_workload.py"), scenario], capture_output=True,
+                           text=True, timeout=300, env=dict(os.environ, SPH_GB300_LIBRARY=lib))
+        assert p.returncode == 0, p.stderr[-2000:]
+        return json.loads(p.stdout.strip().splitlines()[-1])
+
+    return go
+
+
+def test_failed_download_leaves_no_null_buffer(run):
+    out = run("downloads")
+    assert out["null_uses"] == 0
+    for where in ("scene", "pool"):
+        first, *later = out[where]
+        assert first and not any(later), (where, out[where])
