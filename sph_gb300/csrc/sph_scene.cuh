@@ -1348,6 +1348,7 @@ private:
                 [&](cudaGraphConditionalHandle h) {
                     run("k_dfsph_predict_density_list", [&] { launch(k_dfsph_predict_density_list<R, true>, nb, kBlock, 0, 
                         f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
+                    return launched();
                 },
                 [&](cudaGraphConditionalHandle h) {
                     run("k_dfsph_correct_list", [&] { launch(k_dfsph_correct_list<R, 1>, nb, kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
@@ -1369,11 +1370,13 @@ private:
                     {
                         // computeDensities + computeAlpha + pair lists + the first divergence error
                         auto ph = phase("Neigh search+Densities+Alpha factor");
-                        launch_build_lists<true>(h);
+                        const int brc = launch_build_lists<true>(h);
+                        if (brc) return brc;
                         launch_bh_boundary(0);
                     }
                     // correctDivergenceError DFSPHSolver.cpp:494-590
                     solver.emplace(phases_, "Divergence solver", ls_, capturing_, prof_);
+                    return launched();
                 },
                 [&](cudaGraphConditionalHandle h) {
                     run("k_dfsph_correct_list", [&] { launch(k_dfsph_correct_list<R, 2>, nb, kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
@@ -1434,7 +1437,8 @@ private:
     }
 
     // A solver loop: init(h) launches the kernel that sets the first loop
-    // test, body(h) one iteration whose last kernel sets the next.  Host mode
+    // test and returns its error code, body(h) one iteration whose last kernel
+    // sets the next.  Host mode
     // reads the flag back every few iterations (finished-loop kernels exit at
     // once); capture mode makes it a conditional WHILE node.
     template <typename Init, typename Body> int solve_loop(int loop_id, Init&& init, Body&& body, unsigned minIt, unsigned maxIt)
@@ -1447,8 +1451,8 @@ private:
             SPH_CUDA(cudaStreamGetCaptureInfo(st_, &cs, nullptr, &g, nullptr, nullptr, nullptr));
             cudaGraphConditionalHandle h;
             SPH_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
-            init(h);
-            SPH_CUDA(cudaGetLastError());
+            const int rc = init(h);
+            if (rc) return rc;
             SPH_CUDA(cudaStreamGetCaptureInfo(st_, &cs, nullptr, &g, &deps, nullptr, &ndeps));
             cudaGraphNodeParams p{};
             p.type = cudaGraphNodeTypeConditional;
@@ -1471,21 +1475,28 @@ private:
             SPH_CUDA(cudaStreamEndCapture(st2_, &out));
             return SPH_OK;
         }
-        init((cudaGraphConditionalHandle)0);
-        SPH_CUDA(cudaGetLastError());
-        unsigned launched = 0;
+        const int rc = init((cudaGraphConditionalHandle)0);
+        if (rc) return rc;
+        unsigned done = 0;
         const unsigned first = std::min(std::max(minIt, 1u) + 1u, maxIt);
-        while (launched < maxIt) {
-            unsigned batch = launched == 0 ? first : 2u;
-            batch = std::min(batch, maxIt - launched);
+        while (done < maxIt) {
+            unsigned batch = done == 0 ? first : 2u;
+            batch = std::min(batch, maxIt - done);
             for (unsigned b = 0; b < batch; ++b) body((cudaGraphConditionalHandle)0);
             SPH_CUDA(cudaGetLastError());
-            launched += batch;
+            done += batch;
             SPH_CUDA(cudaMemcpyAsync(&h_sc_->active, &sc_.p->active, sizeof(unsigned), cudaMemcpyDeviceToHost, st_));
             SPH_CUDA(cudaStreamSynchronize(st_));
             chained_ = false;
             if (!h_sc_->active) break;
         }
+        return SPH_OK;
+    }
+
+    // the launches so far succeeded
+    int launched()
+    {
+        SPH_CUDA(cudaGetLastError());
         return SPH_OK;
     }
 
@@ -1549,6 +1560,7 @@ private:
                         run("k_dfsph_predict_density", [&] { launch(k_dfsph_predict_density<R, G, true>, wblocks(), kBlock, 0, 
                             f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h); });
                     });
+                    return launched();
                 },
                 [&](cudaGraphConditionalHandle h) {
                     withG([&](auto gt) {
@@ -1582,6 +1594,7 @@ private:
                         run("k_dfsph_divergence", [&] { launch(k_dfsph_divergence<R, G, true>, wblocks(), kBlock, 0, 
                             f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h); });
                     });
+                    return launched();
                 },
                 [&](cudaGraphConditionalHandle h) {
                     withG([&](auto gt) {
@@ -1695,7 +1708,10 @@ private:
             run("k_pcisph_init", [&] { launch(k_pcisph_init<R>, blocks(n_, 256), 256, 0, f); });
             if (bh_ && nb_) run("k_bh_zero_pressure", [&] { launch(k_bh_zero_pressure<R>, blocks(nb_, 256), 256, 0, B(1)); });
             rc = solve_loop(1,
-                [&](cudaGraphConditionalHandle h) { run("k_pcisph_loop_begin", [&] { launch(k_pcisph_loop_begin, 1, 1, 0, sc_.p, lim_, h); }); },
+                [&](cudaGraphConditionalHandle h) {
+                    run("k_pcisph_loop_begin", [&] { launch(k_pcisph_loop_begin, 1, 1, 0, sc_.p, lim_, h); });
+                    return launched();
+                },
                 [&](cudaGraphConditionalHandle h) {
                     if (cands_)
                     run("k_pcisph_predict", [&] { launch(k_pcisph_predict<R, true>, blocks(n_, 256), 256, 0, f, c_, sc_.p); });

@@ -65,6 +65,24 @@ def downloads(F):
     return out
 
 
+def launches(F):
+    """Each launch of a step fails in turn: {solver: [launches, those whose failure the step did not report]}."""
+    out = {}
+    for name, p in SOLVERS.items():
+        s = scene(**p)
+        n0 = F.fake_launches()
+        s.step(1)
+        n = F.fake_launches() - n0
+        lost = []
+        for k in range(1, n + 1):
+            F.fake_fail_launch(k)
+            if not failed(lambda: s.step(1)):
+                lost.append(k)
+            F.fake_fail_launch(0)
+        out[name] = [n, lost, failed(lambda: s.step(1))]
+    return out
+
+
 if __name__ == "__main__":
     F = fake()
-    print(json.dumps({"downloads": downloads}[sys.argv[1]](F)))
+    print(json.dumps({"downloads": downloads, "launches": launches}[sys.argv[1]](F)))

@@ -1,7 +1,8 @@
 """Failing allocations and launches, on the CPU: the library's own objects linked against a fake of the CUDA runtime
 (tests/fake_cudart.cpp) that refuses a chosen one.
 
-* A read whose staging buffer cannot be allocated reports it; later reads allocate again and nothing uses a null buffer."""
+* A read whose staging buffer cannot be allocated reports it; later reads allocate again and nothing uses a null buffer.
+* A step reports the failure of any of its launches."""
 import json
 import os
 import subprocess
@@ -38,3 +39,8 @@ def test_failed_download_leaves_no_null_buffer(run):
     for where in ("scene", "pool"):
         first, *later = out[where]
         assert first and not any(later), (where, out[where])
+
+
+def test_step_reports_every_failed_launch(run):
+    for solver, (n, lost, later) in run("launches").items():
+        assert n >= 5 and lost == [] and not later, (solver, n, lost, later)
