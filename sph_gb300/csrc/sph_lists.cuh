@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
         xi = xyz(f.pos[i]);
         pc = f.cell[i];
         if constexpr (DIV0) vi = xyz(f.vel[i]);
-        half = half_cull_ok(g, pc, xi, c.h, &xr);
+        half = L.posh && half_cull_ok(g, pc, xi, c.h, &xr);
     }
     const bool bhalf = half && akinci && L.bposh;
     const WideRanges<W> rf = wide_ranges<W>(half, gl, g, cs, pc, xr, hf, (float)c.cull2),

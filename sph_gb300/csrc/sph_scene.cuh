@@ -227,15 +227,19 @@ inline int grid_plan(const sph_scene_desc& d, PointSpan hx, PointSpan hb, bool a
 template <typename T> struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
-    ~DevBuf() { if (p) cudaFree(p); }
+    ~DevBuf() { release(); }
+    void release()
+    {
+        if (p) cudaFree(p);
+        p = nullptr;
+        n = 0;
+    }
     // n counts what p holds: 0 after a failure, so that a buffer kept between
     // calls is allocated again by the next one (and the error is taken off the
     // thread's last one, which the next launch check would report).
     cudaError_t alloc(size_t count)
     {
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
+        release();
         const cudaError_t e = cudaMalloc((void**)&p, std::max<size_t>(count, 1) * sizeof(T));
         if (e == cudaSuccess) {
             n = count;
@@ -369,12 +373,13 @@ public:
             k_gather_boundary<R><<<blocks(nb_, 256), 256, 0, st_>>>(nb_, tmp_.p, key_.p, bstarts_.p, B(0), B(1));
             SPH_CUDA(cudaGetLastError());
             if (akinci_) k_boundary_psi<R><<<blocks(nb_, 128), 128, 0, st_>>>(B(1), gv_, bstarts_.p, c_);
-            if (lists_ || cands_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
             SPH_CUDA(cudaGetLastError());
             SPH_CUDA(cudaStreamSynchronize(st_));
         } else {
             SPH_CUDA(cudaMemsetAsync(bstarts_.p, 0, (nkeys_ + 1) * sizeof(uint32_t), st_));
         }
+        rc = allocate_optional();
+        if (rc) return rc;
         rc = build_grid(false);
         if (rc) return rc;
         if (d.simulation_method == SPH_DFSPH) {
@@ -494,7 +499,7 @@ public:
             k_gather_boundary<R><<<blocks(nb_, 256), 256, 0, st_>>>(nb_, tmp_.p, key_.p, bstarts_.p, B(1), B(0));
             std::swap(bd_[0], bd_[1]);
             if (akinci_) k_boundary_psi<R><<<blocks(nb_, 128), 128, 0, st_>>>(B(1), gv_, bstarts_.p, c_);
-            if (lists_ || cands_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
+            if (bposh_.p) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
             SPH_CUDA(cudaGetLastError());
         } else {
             SPH_CUDA(cudaMemsetAsync(bstarts_.p, 0, (nkeys_ + 1) * sizeof(uint32_t), st_));
@@ -985,37 +990,10 @@ private:
         }
         lists_ = d.simulation_method == SPH_DFSPH && d.neighbor_list_max > 0;
         kmax_ = lists_ ? (uint32_t)d.neighbor_list_max : 0u;
-        // candidate lists, PCISPH and WCSPH, and DFSPH for its non-pressure
-        // forces: Akinci or no boundary (the PCISPH boundary model moves
-        // predicted positions after the prediction), indices below 2^27.  Not
-        // DFSPH in a cube: its clamp moves particles after the grid build whose
-        // candidates (and half-precision positions) the next step's forces
-        // would visit, so those walk the cells.
-        cands_ = d.neighbor_list_max > 0 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask &&
-                 (d.simulation_method != SPH_DFSPH ||
-                  (c_.force_flags != 0 && !c_.has_cube && (G_ > 1 || build_lanes() == 1)));
-        if (cands_) {
-            // one lane: the whole list; G lanes: each twice its even share
-            cslots_ = G_ == 1 ? (uint32_t)d.neighbor_list_max : std::max(1u, 2u * (uint32_t)d.neighbor_list_max / (unsigned)G_);
-            SPH_CUDA(cand_.alloc((size_t)cslots_ * n * G_));
-            SPH_CUDA(candn_.alloc(n * G_));
-            SPH_CUDA(candb_.alloc(n * G_));
-            SPH_CUDA(cudaMemsetAsync(candn_.p, 0, n * G_ * sizeof(uint32_t), st_));
-            SPH_CUDA(cudaMemsetAsync(candb_.p, 0, n * G_ * sizeof(uint32_t), st_));
-        }
         SPH_CUDA(pairs_.alloc(lists_ ? (size_t)kmax_ * n : 1));
         SPH_CUDA(lcount_.alloc(lists_ ? n : 1));
         SPH_CUDA(bgrad_.alloc(lists_ ? n : 1));
         SPH_CUDA(kbuf_.alloc(n));
-        // half-precision positions for the list builds' culls (pairs of
-        // points, the last one whole, and a spare word for the cull), the
-        // fluid's written by every gather, the boundary's once per grid box
-        if (lists_ || cands_) {
-            SPH_CUDA(posh_.alloc(n / 2 + 2));
-            SPH_CUDA(cudaMemsetAsync(posh_.p, 0, (n / 2 + 2) * sizeof(uint4), st_));
-            SPH_CUDA(bposh_.alloc(nb / 2 + 2));
-            SPH_CUDA(cudaMemsetAsync(bposh_.p, 0, (nb / 2 + 2) * sizeof(uint4), st_));
-        }
         SPH_CUDA(cudaMemsetAsync(lcount_.p, 0, lcount_.n * sizeof(uint32_t), st_));
         SPH_CUDA(cudaMemsetAsync(kbuf_.p, 0, n * sizeof(R), st_));
         SPH_CUDA(lstat_.alloc(2));
@@ -1050,6 +1028,50 @@ private:
             b.dp = bh ? bdp_.p : nullptr;
         }
         cur_ = 0;
+        return SPH_OK;
+    }
+
+    // Memory a scene can do without, taken after everything else: where it is
+    // not to be had, the culls run on the positions themselves and the passes
+    // walk the cells.
+    int allocate_optional()
+    {
+        const size_t n = n_, nb = std::max(nb_, 1u);
+        // candidate lists, PCISPH and WCSPH, and DFSPH for its non-pressure
+        // forces: Akinci or no boundary (the PCISPH boundary model moves
+        // predicted positions after the prediction), indices below 2^27.  Not
+        // DFSPH in a cube: its clamp moves particles after the grid build whose
+        // candidates (and half-precision positions) the next step's forces
+        // would visit, so those walk the cells.
+        const bool want = d.neighbor_list_max > 0 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask &&
+                          (d.simulation_method != SPH_DFSPH ||
+                           (c_.force_flags != 0 && !c_.has_cube && (G_ > 1 || build_lanes() == 1)));
+        // half-precision positions for the list builds' culls (pairs of
+        // points, the last one whole, and a spare word for the cull), the
+        // fluid's written by every gather, the boundary's once per grid box
+        bool half = (lists_ || want) && posh_.alloc(n / 2 + 2) == cudaSuccess && bposh_.alloc(nb / 2 + 2) == cudaSuccess;
+        if (half) {
+            SPH_CUDA(cudaMemsetAsync(posh_.p, 0, (n / 2 + 2) * sizeof(uint4), st_));
+            SPH_CUDA(cudaMemsetAsync(bposh_.p, 0, (nb / 2 + 2) * sizeof(uint4), st_));
+            if (nb_) k_boundary_half<R><<<blocks(nb_, 256), 256, 0, st_>>>(B(1), gv_, hd_, bposh_.p);
+            SPH_CUDA(cudaGetLastError());
+        } else {
+            posh_.release();
+            bposh_.release();
+        }
+        // one lane: the whole list; G lanes: each twice its even share
+        const size_t slots = G_ == 1 ? (size_t)d.neighbor_list_max : std::max<size_t>(1, 2 * (size_t)d.neighbor_list_max / (size_t)G_);
+        cands_ = want && half && cand_.alloc(slots * n * G_) == cudaSuccess && candn_.alloc(n * G_) == cudaSuccess &&
+                 candb_.alloc(n * G_) == cudaSuccess;
+        if (cands_) {
+            cslots_ = (uint32_t)slots;
+            SPH_CUDA(cudaMemsetAsync(candn_.p, 0, n * G_ * sizeof(uint32_t), st_));
+            SPH_CUDA(cudaMemsetAsync(candb_.p, 0, n * G_ * sizeof(uint32_t), st_));
+        } else {
+            cand_.release();
+            candn_.release();
+            candb_.release();
+        }
         return SPH_OK;
     }
 

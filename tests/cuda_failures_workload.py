@@ -23,10 +23,7 @@ SOLVERS = {
 
 
 def fake():
-    f = ctypes.CDLL(os.environ["SPH_GB300_LIBRARY"])
-    f.fake_memory.argtypes = [ctypes.c_size_t]
-    f.fake_live_bytes.restype = f.fake_peak_bytes.restype = ctypes.c_size_t
-    return f
+    return ctypes.CDLL(os.environ["SPH_GB300_LIBRARY"])
 
 
 def scene(n_side=6, **p):
@@ -83,6 +80,31 @@ def launches(F):
     return out
 
 
+def allocations(F):
+    """Each allocation of init fails in turn: {solver: [allocations, kernels of the candidate lists' build in a step,
+    [those init did without, such kernels then launched in a step]]}."""
+    out = {}
+    for name, p in SOLVERS.items():
+        def step():
+            k = F.fake_launched(b"k_density_cand")
+            scene(**p).step(1)
+            return F.fake_launched(b"k_density_cand") - k
+
+        m = F.fake_mallocs()
+        lists = step()
+        n = F.fake_mallocs() - m
+        without = []
+        for k in range(1, n + 1):
+            F.fake_fail_malloc(k)
+            try:
+                without.append([k, step()])
+            except sph_gb300.SPHError:
+                pass
+            F.fake_fail_malloc(0)
+        out[name] = [n, lists, without]
+    return out
+
+
 if __name__ == "__main__":
     F = fake()
-    print(json.dumps({"downloads": downloads, "launches": launches}[sys.argv[1]](F)))
+    print(json.dumps({"downloads": downloads, "launches": launches, "allocations": allocations}[sys.argv[1]](F)))

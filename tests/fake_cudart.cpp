@@ -6,8 +6,7 @@
 //
 //   fake_fail_launch(n)   the n-th launch from now on fails (0: none)
 //   fake_fail_malloc(n)   the n-th allocation from now on fails (0: none)
-//   fake_memory(bytes)    allocations beyond this many live bytes fail
-//   fake_launches / fake_live_bytes / fake_peak_bytes
+//   fake_launches() / fake_mallocs()   so far
 //   fake_null_uses()      copies from or to, and downloads into, a null pointer
 //   fake_launched(name)   launches of kernels whose name contains `name`
 #include <cuda_runtime_api.h>
@@ -24,9 +23,7 @@ std::map<const void*, std::string>& names()
     return m;
 }
 std::map<std::string, int> launched;
-std::map<void*, size_t> live;
-size_t live_bytes = 0, peak_bytes = 0, limit_bytes = (size_t)-1;
-int fail_launch = 0, fail_malloc = 0, launches = 0, null_uses = 0;
+int fail_launch = 0, fail_malloc = 0, launches = 0, mallocs = 0, null_uses = 0;
 cudaError_t last = cudaSuccess;
 struct Config {
     dim3 grid, block;
@@ -64,15 +61,8 @@ cudaError_t take(void** p, size_t n)
 extern "C" {
 void fake_fail_launch(int n) { fail_launch = n; }
 void fake_fail_malloc(int n) { fail_malloc = n; }
-void fake_memory(size_t n) { limit_bytes = n ? n : (size_t)-1; }
 int fake_launches() { return launches; }
-size_t fake_live_bytes() { return live_bytes; }
-size_t fake_peak_bytes()
-{
-    const size_t p = peak_bytes;
-    peak_bytes = live_bytes;
-    return p;
-}
+int fake_mallocs() { return mallocs; }
 int fake_null_uses() { return null_uses; }
 int fake_launched(const char* part)
 {
@@ -116,23 +106,13 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void** args, size_t, 
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { return launch(f, args); }
 cudaError_t cudaMalloc(void** p, size_t n)
 {
-    if ((fail_malloc > 0 && --fail_malloc == 0) || live_bytes + n > limit_bytes) return fail(cudaErrorMemoryAllocation);
-    const cudaError_t e = take(p, n);
-    if (e == cudaSuccess) {
-        live[*p] = n;
-        live_bytes += n;
-        if (live_bytes > peak_bytes) peak_bytes = live_bytes;
-    }
-    return e;
+    ++mallocs;
+    if (fail_malloc > 0 && --fail_malloc == 0) return fail(cudaErrorMemoryAllocation);
+    return take(p, n);
 }
 cudaError_t cudaFree(void* p)
 {
-    const auto it = live.find(p);
-    if (it != live.end()) {
-        live_bytes -= it->second;
-        live.erase(it);
-        std::free(p);
-    }
+    std::free(p);
     return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) { return take(p, n); }

@@ -2,7 +2,8 @@
 (tests/fake_cudart.cpp) that refuses a chosen one.
 
 * A read whose staging buffer cannot be allocated reports it; later reads allocate again and nothing uses a null buffer.
-* A step reports the failure of any of its launches."""
+* A step reports the failure of any of its launches.
+* A scene whose candidate lists (or half-precision positions) find no memory runs without them."""
 import json
 import os
 import subprocess
@@ -44,3 +45,12 @@ def test_failed_download_leaves_no_null_buffer(run):
 def test_step_reports_every_failed_launch(run):
     for solver, (n, lost, later) in run("launches").items():
         assert n >= 5 and lost == [] and not later, (solver, n, lost, later)
+
+
+def test_scene_without_memory_for_candidate_lists(run):
+    out = run("allocations")
+    # half-precision positions of fluid and boundary; the lists and their two counts
+    optional = {"dfsph": 2, "dfsph_f64": 2, "dfsph_forces": 5, "dfsph_walks": 0, "wcsph": 5, "wcsph_forces": 5, "pcisph": 5}
+    for solver, (n, lists, without) in out.items():
+        assert lists == (1 if optional[solver] == 5 else 0), solver
+        assert without == [[k, 0] for k in range(n - optional[solver] + 1, n + 1)], (solver, n, without)
