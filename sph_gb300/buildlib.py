@@ -39,7 +39,7 @@ UNITS = {
     "sph_serve.cpp": [],
 }
 HEADERS = ["sph_device.cuh", "sph_kernels.cuh", "sph_lists.cuh", "sph_cand.cuh", "sph_scene.cuh", "sph_scene_base.h", "sph_ctx.h",
-           "sph_phase.cuh"]
+           "sph_phase.cuh", "sph_divide.h"]
 VARIANTS = {"": ([], OBJDIR, LIB),
             "checked": (["-DSPH_BOUNDS_CHECK"], OBJDIR + "_checked", os.path.join(LIBDIR, "libsph_gb300_checked.so"))}
 

@@ -9,6 +9,7 @@
 // tests.
 #pragma once
 
+#include "sph_divide.h"
 #include "sph_lists.cuh"
 
 namespace sph {
@@ -279,23 +280,23 @@ __global__ void __launch_bounds__(kWideBlock) k_density_cand_wide(Fluid<R> f, co
     if (EOS) cand_eos(i, f, c, xi, density);
 }
 
-// x / b for many x and one b with rb = 1 / b rounded: the quotient x rb and one
-// residual correction (Markstein, IBM J. Res. Dev. 34, 1990), which rounds as
-// the division does unless the exact quotient lies within a rounding of rb of
-// the middle between two results; 3 operations instead of about 9, of which
-// FP64 has two lanes per SM.  Quotients that are not finite keep x rb.
-__device__ __forceinline__ double div_by(double x, double b, double rb)
+// u / dt by components, as the divisions round; the rare quotients that
+// `quotient` leaves to the division take it out of line.
+static __device__ __noinline__ V3<double> divide3(V3<double> u, double b) { return V3<double>{u.x / b, u.y / b, u.z / b}; }
+__device__ __forceinline__ V3<double> div3(V3<double> u, const Divisor& d)
 {
-    const double q = __dmul_rn(x, rb);
-    const double r = __fma_rn(__fma_rn(-q, b, x), rb, q);
-    return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : r;
+    V3<double> q;
+    const bool x = quotient(u.x, d, &q.x), y = quotient(u.y, d, &q.y), z = quotient(u.z, d, &q.z);
+    return x && y && z ? q : divide3(u, d.b);
 }
-__device__ __forceinline__ float div_by(float x, float b, float) { return x / b; }
+__device__ __forceinline__ V3<float> div3(V3<float> u, float b) { return u / b; }
+__device__ __forceinline__ Divisor divisor_of(double b) { return divisor(b); }
+__device__ __forceinline__ float divisor_of(float b) { return b; }
 
 // WCSPH with XSPH viscosity (or none of the force plugins' other kinds):
 // pressure force (k_wcsph_pressure_force) and viscosity (k_npforce) from one
 // visit of the candidates, each sum in its own order; the distance and its
-// root are formed once.  us/step: 8,000 particles in FP64 202 -> 143, 90,000
+// root are formed once.  us/step: 8,000 particles in FP64 202 -> 149, 90,000
 // with Akinci walls 103 -> 91.
 template <typename R> struct WcsphFluid { V3<R> p, av; };
 template <typename R> struct WcsphBoundary { V3<R> p, avb; };
@@ -320,7 +321,8 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_forces(Fluid<R> f, const P4<R>
         const R dpi = pi.w;
         const P4<R> vi4 = f.vel[i];
         const V3<R> vi = xyz(vi4);
-        const R rho_i = vi4.w, dt = (R)sc->dt, rdt = (R)1 / dt;
+        const R rho_i = vi4.w;
+        const auto dt = divisor_of((R)sc->dt);
         const uint32_t pc = f.cell[i];
         const bool bvisc = (c.force_flags & F_BVISC) != 0;
         const P4<R>*xk = f.xk, *vel = f.vel;
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_forces(Fluid<R> f, const P4<R>
                 if (!(r2 <= c.cull2)) return;
                 a.p = a.p - (c.mass * (dpi + q.x.w)) * cubic_gradW(c, r, r2);
                 const V3<R> u = ((c.visc * (c.mass / q.v.w)) * (xyz(q.v) - vi)) * cubic_W(c, sqrt(r2));
-                a.av = a.av + V3<R>{div_by(u.x, dt, rdt), div_by(u.y, dt, rdt), div_by(u.z, dt, rdt)};
+                a.av = a.av + div3(u, dt);
             });
         sb.p = sf.p;  // one sum: the boundary's terms follow the fluid's
         if (akinci)
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_forces(Fluid<R> f, const P4<R>
                     a.p = a.p - (pb.w * (dpi * (R)1)) * cubic_gradW(c, r, r2);
                     if (bvisc) {
                         const V3<R> u = ((c.bvisc * (pb.w / rho_i)) * (-vi)) * cubic_W(c, sqrt(r2));
-                        a.avb = a.avb + V3<R>{div_by(u.x, dt, rdt), div_by(u.y, dt, rdt), div_by(u.z, dt, rdt)};
+                        a.avb = a.avb + div3(u, dt);
                     }
                 });
     }
