@@ -245,9 +245,10 @@ template <typename R> struct BuildSums {
     uint32_t cnt;
 };
 
-// A record stored in 16-byte parts.  In build_walk_all the compiler (CUDA 13.0)
-// left out the one 32-byte store of an FP64 record in all but one of its
-// callers' forms: right sums, and lists of whatever the memory held.
+// A record, stored in 16-byte parts.  Of the one 32-byte store of an FP64
+// record the compiler (CUDA 13.0) made nothing in build_walk_all, in all but
+// one of its callers' forms: right sums, and lists of whatever the memory held.
+// No condition for that is known, so every FP64 record is stored this way.
 __device__ __forceinline__ void store_record(P4<float>* d, V3<float> v, uint32_t j) { *d = P4<float>{v.x, v.y, v.z, idx_as(0.f, j)}; }
 __device__ __forceinline__ void store_record(P4<double>* d, V3<double> v, uint32_t j)
 {
@@ -376,7 +377,7 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             } else {
                 sumSq += mg2;
             }
-            if (cnt < L.kmax) L.pairs[(size_t)cnt * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j)};
+            if (cnt < L.kmax) store_record(L.pairs + (size_t)cnt * n + i, mg, j);
             ++cnt;
             if constexpr (DIV0) dv += dot3_div<WHERE>(vi - vj, mg);
         }
@@ -827,7 +828,7 @@ __global__ void __launch_bounds__(kWideBlock, 5) k_build_lists_wide(Fluid<R> f, 
                 const uint32_t b = (__ballot_sync(0xffffffffu, listed) >> g0) & ((1u << W) - 1u);
                 if (listed) {
                     const uint32_t at = cnt + __popc(b & ((1u << gl) - 1u));
-                    if (at < L.kmax) L.pairs[(size_t)at * n + i] = P4<R>{mg.x, mg.y, mg.z, idx_as(R(0), j[t])};
+                    if (at < L.kmax) store_record(L.pairs + (size_t)at * n + i, mg, j[t]);
                 }
                 cnt += __popc(b);
             }
