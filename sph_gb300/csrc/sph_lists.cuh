@@ -304,10 +304,25 @@ template <Rounding WHERE = kOneScene, typename R> __device__ __forceinline__ R d
 }
 
 // The other contraction of a dot product.
-template <typename R> __device__ __forceinline__ R dot3_zyx(V3<R> a, V3<R> b)
+template <Rounding WHERE = kOneScene, typename R> __device__ __forceinline__ R dot3_zyx(V3<R> a, V3<R> b)
 {
-    if constexpr (sizeof(R) == 8) return dot3(a, b);
+    if constexpr (sizeof(R) == 8 || WHERE == kPool) return dot3(a, b);
     else return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+}
+
+// a * b + c and a + b of the one-scene builds: fused in FP32, two roundings in
+// the FP64 parity form (compiled without contraction).
+template <Rounding WHERE = kOneScene, typename R> __device__ __forceinline__ R mul_add(R a, R b, R c)
+{
+    if constexpr (WHERE == kPool) return a * b + c;
+    else if constexpr (sizeof(R) == 8) return __dadd_rn(__dmul_rn(a, b), c);
+    else return __fmaf_rn(a, b, c);
+}
+template <Rounding WHERE = kOneScene, typename R> __device__ __forceinline__ R plain_add(R a, R b)
+{
+    if constexpr (WHERE == kPool) return a + b;
+    else if constexpr (sizeof(R) == 8) return __dadd_rn(a, b);
+    else return __fadd_rn(a, b);
 }
 
 // Forward declarations: the list build's DIV0 form ends with the velocity
@@ -366,16 +381,16 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
         R w;
         V3<R> gw;
         cubic_W_gradW<FAST>(c, r, r2, &w, &gw);
-        density += c.mass * w;
+        density = mul_add<WHERE>(c.mass, w, density);
         const V3<R> mg = c.mass * gw;
-        const R mg2 = dot3(mg, mg);
+        const R mg2 = dot3_div<WHERE>(mg, mg);
         if (mg2 > (R)0) {
-            sumGrad = sumGrad + mg;
+            sumGrad = V3<R>{plain_add<WHERE>(sumGrad.x, mg.x), plain_add<WHERE>(sumGrad.y, mg.y), plain_add<WHERE>(sumGrad.z, mg.z)};
             if constexpr (sizeof(R) == 8) {
                 const R m = sqrt(mg2);
                 sumSq += m * m;
             } else {
-                sumSq += mg2;
+                sumSq = plain_add<WHERE>(sumSq, mg2);
             }
             if (cnt < L.kmax) store_record(L.pairs + (size_t)cnt * n + i, mg, j);
             ++cnt;
@@ -452,8 +467,8 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             R w;
             V3<R> gw;
             cubic_W_gradW<FAST>(c, r, r2, &w, &gw);
-            density += pb.w * w;
-            bg = bg + pb.w * gw;
+            density = mul_add<WHERE>(pb.w, w, density);
+            bg = V3<R>{mul_add<WHERE>(pb.w, gw.x, bg.x), mul_add<WHERE>(pb.w, gw.y, bg.y), mul_add<WHERE>(pb.w, gw.z, bg.z)};
         };
         // The boundary candidates as the fluid ones: culled from the static
         // half-precision copy into the (now free) queue, then evaluated in
@@ -489,7 +504,7 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
             });
         }
     }
-    sumGrad = sumGrad + bg;
+    sumGrad = V3<R>{plain_add<WHERE>(sumGrad.x, bg.x), plain_add<WHERE>(sumGrad.y, bg.y), plain_add<WHERE>(sumGrad.z, bg.z)};
     f.rho[i] = density;
     f.vel[i].w = density;
     R den;
@@ -497,7 +512,7 @@ __device__ __forceinline__ void build_lists_one(uint32_t i, const Fluid<R>& f, c
         const R m = sqrt(dot3(sumGrad, sumGrad));
         den = m * m + sumSq;
     } else {
-        den = dot3(sumGrad, sumGrad) + sumSq;
+        den = dot3_zyx<WHERE>(sumGrad, sumGrad) + sumSq;
     }
     f.alpha[i] = (fabs(den) > c.eps) ? density / den : (R)0;
     L.count[i] = cnt;
@@ -603,13 +618,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_build_lists(Fluid<R> f, const P
 // looks up its columns' ranges, tests its words of a column's candidates, and
 // evaluates its part of the accepted ones; the values go to shared memory and
 // are then summed one after another, each of the sums by a lane of its own,
-// in the list's order and with the rounding of build_lists_one (written out
-// below), so the results are bit-identical to it.
-
-// a * b + c as build_lists_one rounds it: fused in FP32, two roundings in the
-// FP64 parity form (compiled without contraction)
-__device__ __forceinline__ float mul_add(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double mul_add(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+// in the list's order and with the rounding of build_lists_one.  The results
+// are bit-identical to it: the sums' rounding is written out in both; the
+// distances' and the kernel values' contraction is the compiler's, the same in
+// both so far, which test_build_lanes.py checks bit for bit.
 
 constexpr uint32_t kWideBlock = 128, kWideChunk = 32;
 
