@@ -956,10 +956,33 @@ template <typename R> struct PosVelIdx {
 template <typename R> struct NPFluid { V3<R> av, ast; };
 template <typename R> struct NPBoundary { V3<R> avb, aad; };
 
+// Sums whose rounding is written out for the one-scene kernels; the pool's
+// keep the plain expressions, whose contraction is the compiler's.
+enum Rounding { kOneScene, kPool };
+
+// The terms of artificial viscosity with their rounding written out (FP32: the
+// contraction the compiler first chose for the pass over lists), so that every
+// form of the one-scene pass has the same sums.
+template <Rounding WHERE, typename R> __device__ __forceinline__ R art_dot(V3<R> a, V3<R> b)
+{
+    if constexpr (sizeof(R) == 8 || WHERE == kPool) return dot3(a, b);
+    else return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+template <Rounding WHERE, typename R> __device__ __forceinline__ R art_dist(R rl, R h2)
+{
+    if constexpr (sizeof(R) == 8 || WHERE == kPool) return rl * rl + (R)0.01 * h2;
+    else return __fmaf_rn(rl, rl, __fmul_rn(0.01f, h2));
+}
+template <Rounding WHERE, typename R> __device__ __forceinline__ V3<R> add_scaled(V3<R> a, R s, V3<R> g)
+{
+    if constexpr (sizeof(R) == 8 || WHERE == kPool) return a + s * g;
+    else return V3<R>{__fmaf_rn(s, g.x, a.x), __fmaf_rn(s, g.y, a.y), __fmaf_rn(s, g.z, a.z)};
+}
+
 // FL: the scene's force plugins where they are known when compiling (boundary
 // viscosity apart); kAnyForces: from the constants.
 constexpr int kAnyForces = -1;
-template <typename R, int G, bool LISTS = false, int FL = kAnyForces>
+template <typename R, int G, bool LISTS = false, int FL = kAnyForces, Rounding WHERE = kOneScene>
 __device__ __forceinline__ NPForces<R> npforce_sums(uint32_t i, int lane, const Fluid<R>& f,
                                                     const P4<R>* __restrict__ bpos, const GridView& g,
                                                     const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
@@ -995,11 +1018,11 @@ __device__ __forceinline__ NPForces<R> npforce_sums(uint32_t i, int lane, const 
             if (fl & F_STD_VISC)
                 a.av = a.av + ((c.mass * (vj - vi)) / rho_j) * visc_laplW(c, r2);
             if (fl & F_ART_VISC) {
-                const R dotProd = dot3(vi - vj, r);
-                const R sqDist = rl * rl;
                 const R kij = (R)2 * c.density0 / (rho_i + rho_j);
-                a.av = a.av + (kij * (R)10 * (R)0.1 * c.visc * (c.mass / rho_j) * dotProd / (sqDist + (R)0.01 * h2)) *
-                                  cubic_gradW(c, r, r2);
+                a.av = add_scaled<WHERE>(a.av,
+                                         kij * (R)10 * (R)0.1 * c.visc * (c.mass / rho_j) * art_dot<WHERE>(vi - vj, r) /
+                                             art_dist<WHERE>(rl, h2),
+                                         cubic_gradW(c, r, r2));
             }
             if (fl & F_SURFACE_TENSION) {
                 if (rl > (R)0 && rl <= c.h) {
@@ -1025,12 +1048,10 @@ __device__ __forceinline__ NPForces<R> npforce_sums(uint32_t i, int lane, const 
                     a.avb = a.avb + (((c.bvisc * (pb.w / rho_i)) * (-vi)) * cubic_W(c, rl)) / dt;
                 if (fl & F_STD_VISC)
                     a.avb = a.avb + ((pb.w * (-vi)) / rho_i) * visc_laplW(c, r2);
-                if (fl & F_ART_VISC) {
-                    const R dotProd = dot3(vi, r);
-                    const R sqDist = rl * rl;
-                    a.avb = a.avb + ((R)10 * (R)0.1 * c.bvisc * (pb.w / rho_i) * dotProd / (sqDist + (R)0.01 * h2)) *
-                                        cubic_gradW(c, r, r2);
-                }
+                if (fl & F_ART_VISC)
+                    a.avb = add_scaled<WHERE>(
+                        a.avb, (R)10 * (R)0.1 * c.bvisc * (pb.w / rho_i) * art_dot<WHERE>(vi, r) / art_dist<WHERE>(rl, h2),
+                        cubic_gradW(c, r, r2));
             }
             if ((fl & F_ADHESION) && rl > (R)0)
                 a.aad = a.aad - ((c.adh * pb.w * adhesion_W(c, rl)) * r) / rl;

@@ -296,7 +296,6 @@ __device__ __noinline__ BuildSums<R> build_walk_all(uint32_t i, const Fluid<R>& 
 // first), so that the sums of the one-scene build and of its passes agree bit
 // for bit.  The pool's kernels (kPool) keep the plain expression, whose
 // contraction differs from one copy of its unrolled loop to the next.
-enum Rounding { kOneScene, kPool };
 template <Rounding WHERE = kOneScene, typename R> __device__ __forceinline__ R dot3_div(V3<R> a, V3<R> b)
 {
     if constexpr (sizeof(R) == 8 || WHERE == kPool) return dot3(a, b);

@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kBlock) k_pool_npforce(Fluid<float> f, const P
     const PoolScene& sd = T[sid[i]];
     const Consts<float>& c = sd.c;
     if (!sd.running || !(c.force_flags & kPoolForces)) return;
-    const NPForces<float> s = npforce_sums<float, 1>(i, 0, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, c,
+    const NPForces<float> s = npforce_sums<float, 1, false, kAnyForces, kPool>(i, 0, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, c,
                                                      sd.akinci, (float)sd.s.dt);
     npforce_apply(i, f, c, s);
 }

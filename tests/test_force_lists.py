@@ -4,6 +4,7 @@
 * WCSPH with XSPH: the one pass of both forces against the two walks.
 * DFSPH with every force plugin at sizes whose list build has one lane per particle and writes the candidate lists
   itself, with 1 to 8 lanes in the force passes, with lists that hold every candidate and lists that do not.
+* Every set of force plugins: FP32 compiles most of them apart over lists, whose sums stay the walk's.
 * A WCSPH step's phases with lists."""
 import numpy as np
 import pytest
@@ -65,6 +66,28 @@ def test_wcsph_forces_of_one_pass(gpu_lib, precision, n):
     else:
         # 64 terms of p / rho^2 m |grad W| dt, p = k ((rho / rho0)^7 - 1) with k = 1.43e5 and (rho / rho0)^7 <= 4
         assert np.abs(a - w).max() <= 64 * EPS["f32"] * 64 * 2 * 3 * 1.43e5 / 1e6 * 500 * 1e-4
+
+
+VISCOSITY = {"none": {}, "xsph": dict(visc_method=2, visc=0.01, bvisc=0.01), "standard": dict(visc_method=0, visc=0.01, bvisc=0.01),
+             "artificial": dict(visc_method=1, visc=0.01, bvisc=0.01)}
+
+
+@pytest.mark.parametrize("precision,lanes", [("f32", 1), ("f32", 4), ("f64", 1)])
+@pytest.mark.parametrize("visc", list(VISCOSITY))
+@pytest.mark.parametrize("tension", [0, 1])
+@pytest.mark.parametrize("adhesion", [0, 1])
+def test_force_sets(gpu_lib, precision, lanes, visc, tension, adhesion):
+    if visc == "none" and not tension and not adhesion:
+        pytest.skip("no plugin")
+    x, v = block(500)
+    p = dict(method=1, precision=precision, threads_per_particle=lanes, dt=1e-4, min_it=2, max_it=2, eta=0.001, **VISCOSITY[visc])
+    if tension:
+        p.update(st_method=3, st=0.5)
+    if adhesion:
+        p.update(adh_method=4, adh=0.1)
+    a, w = (run(x, v, ("v", "x"), steps=2, neighbor_list_max=k, **p) for k in (64, 0))
+    for g, e in zip(a, w):
+        assert np.array_equal(g, e)
 
 
 def sms():
