@@ -1445,17 +1445,37 @@ private:
                 constexpr int FL = decltype(ft)::value;
                 run("k_npforce", [&] { launch(k_npforce<R, G, LISTS, FL>, wblocks(), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, akinci_, sc_.p, L); });
             };
-            // usual combinations compiled apart: fewer registers and no tests
-            // of the flags in the loop
-            constexpr int XSPH = F_XSPH, STD_ALL = F_STD_VISC | F_SURFACE_TENSION | F_ADHESION, XSPH_ALL = F_XSPH | F_SURFACE_TENSION | F_ADHESION;
-            const int fl = c_.force_flags & ~F_BVISC;
-            if (LISTS && fl == XSPH) go(std::integral_constant<int, LISTS ? XSPH : kAnyForces>{});
-            else if (LISTS && fl == STD_ALL) go(std::integral_constant<int, LISTS ? STD_ALL : kAnyForces>{});
-            else if (LISTS && fl == XSPH_ALL) go(std::integral_constant<int, LISTS ? XSPH_ALL : kAnyForces>{});
+            // FP32 over lists: each set of plugins compiled apart (fewer
+            // registers, no tests of the flags in the loop).  85,000 DFSPH
+            // particles, k_npforce in us, compiled apart / one form: XSPH 43.9 /
+            // 52.8, standard viscosity 40.0 / 48.3, artificial 40.6 /
+            // 49.7, adhesion 15.2 / 17.4, XSPH with surface tension and adhesion
+            // 57.8 / 66.9.
+            // FP64, bound by its arithmetic: within 2 %, one form.
+            if constexpr (LISTS && sizeof(R) == 4) by_force_set(go);
             else go(std::integral_constant<int, kAnyForces>{});
         });
         SPH_CUDA(cudaGetLastError());
         return SPH_OK;
+    }
+
+    // go(the scene's force plugins as a constant, boundary viscosity apart)
+    template <typename Go> void by_force_set(Go&& go)
+    {
+        auto with = [&](auto vt) {
+            constexpr int V = decltype(vt)::value;
+            constexpr int ST = V | F_SURFACE_TENSION, AD = V | F_ADHESION, BOTH = ST | AD;
+            const bool st = c_.force_flags & F_SURFACE_TENSION, ad = c_.force_flags & F_ADHESION;
+            if (st && ad) go(std::integral_constant<int, BOTH>{});
+            else if (st) go(std::integral_constant<int, ST>{});
+            else if (ad) go(std::integral_constant<int, AD>{});
+            else go(std::integral_constant<int, V>{});
+        };
+        // (a scene has one viscosity at most)
+        if (c_.force_flags & F_ART_VISC) with(std::integral_constant<int, F_ART_VISC>{});
+        else if (c_.force_flags & F_XSPH) with(std::integral_constant<int, F_XSPH>{});
+        else if (c_.force_flags & F_STD_VISC) with(std::integral_constant<int, F_STD_VISC>{});
+        else with(std::integral_constant<int, 0>{});
     }
 
     // A solver loop: init(h) launches the kernel that sets the first loop
