@@ -1179,8 +1179,8 @@ private:
     // Several lanes shorten the chain of dependent loads but execute two to
     // three times the instructions, so they pay while their blocks are all
     // resident at once: 8 lanes at 4 blocks of 16 particles per SM, 4 lanes at
-    // 5 blocks of 32.  Build in us (1 / 4 / 8 lanes, FP32, with the ~5 us of an
-    // event pair): 2,000 particles 42.6 / 22.3 / 18.4; 8,000 45.2 / 24.5 / 21.8;
+    // 5 blocks of 32 (in FP64 its shared memory lets 3 reside).  Build in us
+    // (1 / 4 / 8 lanes, FP32, with the ~5 us of an event pair): 2,000 particles 42.6 / 22.3 / 18.4; 8,000 45.2 / 24.5 / 21.8;
     // 13,000 44.3 / 26.5 / 30.4; 24,000 46.0 / 35.7 / 39.4; 30,000 47.7 / 49.8 /
     // 46.6; 40,000 50.1 / 53.6 / 59.2.  FP64: 2,000 177 / 63 / 43; 13,000 195 /
     // 140 / 161; 30,000 309 / 304 / 316.
@@ -1208,14 +1208,21 @@ private:
                         launch(kernel, blocks(n_, kBlock), kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, L, sc_.p, lim_,
                                partials_.p, h, CO());
                     };
-                    // FP64 above five blocks per SM: eight resident blocks (64
-                    // registers, 48 queue entries) instead of seven (72, 64),
-                    // 125,000 particles 1761 -> 1692 us/step; below, the
-                    // registers win.  FP32 keeps seven (125,000 particles would
-                    // gain 249 -> 232, but its sums round differently there and
-                    // the solvers carry that into everything that follows).
+                    // The 64-entry queue (33 KB a block) lets six blocks reside
+                    // on an SM.  FP64 scenes of more blocks than that, up to
+                    // eight per SM, run the form with 48 entries and 64
+                    // registers, whose blocks are then all resident at once:
+                    // 125,000 particles 1007 -> 936 us a build.  Elsewhere the
+                    // first form is as fast or up to 1 % faster (us, first /
+                    // second form: 40,000 414 / 416, 97,280 685 / 689, 105,000
+                    // 802 / 809, 160,000 1178 / 1184, 220,000 1548 / 1559,
+                    // 300,000 2048 / 2059).  FP32 keeps the first form: there
+                    // the second one's distances and kernel values round
+                    // otherwise, which the solvers carry into everything that
+                    // follows.
                     if constexpr (sizeof(R) == 8) {
-                        if ((size_t)n_ > (size_t)sms_ * 5 * kBlock) {
+                        const size_t per_block = (size_t)sms_ * kBlock;
+                        if ((size_t)n_ > 6 * per_block && (size_t)n_ <= 8 * per_block) {
                             one(k_build_lists<R, DIV0, CAND, kBlock, 8, EB, 48>);
                             return;
                         }

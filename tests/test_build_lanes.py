@@ -1,5 +1,5 @@
-"""The list build's forms by size (8, 4 and 1 lanes per particle, and in FP64 one lane with eight blocks per SM) give the
-same bits: a block of particles at the largest size of a form, and with one particle more, far from all others."""
+"""The list build's forms by size (8, 4 and 1 lanes per particle, and in FP64 one lane with eight resident blocks per SM
+where the scene has more than six and no more than eight) give the same bits: a block of particles at the largest size of a form, and with one particle more, far from all others."""
 import numpy as np
 import pytest
 
@@ -11,9 +11,8 @@ pytestmark = pytest.mark.gpu
 R = 0.01
 
 
-@pytest.mark.parametrize("precision", ["f32", "f64"])
+@pytest.mark.parametrize("precision,per_sm", [("f32", 4 * 16), ("f32", 5 * 32), ("f64", 4 * 16), ("f64", 5 * 32), ("f64", 6 * 128), ("f64", 8 * 128)])
 @pytest.mark.parametrize("lists", [64, 24])
-@pytest.mark.parametrize("per_sm", [4 * 16, 5 * 32])
 def test_lanes_give_the_same_bits(gpu_lib, precision, lists, per_sm):
     torch = pytest.importorskip("torch")
     n = torch.cuda.get_device_properties(0).multi_processor_count * per_sm

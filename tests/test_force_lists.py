@@ -100,11 +100,11 @@ def sms():
 @pytest.mark.parametrize("lists", [64, 30])
 @pytest.mark.parametrize("where", ["one", "one_eight_blocks"])
 def test_dfsph_forces_over_lists_of_the_build(gpu_lib, precision, lanes, lists, where):
-    """One particle more than the sizes with several lanes per particle in the build, and (FP64) than those with five
-    blocks per SM."""
+    """One particle more than the sizes with several lanes per particle in the build, and (FP64) than those with six
+    resident blocks per SM."""
     if where == "one_eight_blocks" and (precision == "f32" or lanes in (2, 4)):
         pytest.skip("FP64 only; 1 and 8 lanes")
-    n = sms() * 5 * (32 if where == "one" else 128) + 1
+    n = sms() * (5 * 32 if where == "one" else 6 * 128) + 1
     x, v = block(n)
     p = dict(method=2, precision=precision, threads_per_particle=lanes, dt=1e-3, min_dt=1e-3, max_dt=1e-3, min_it=0, max_it=0,
              min_it_v=0, max_it_v=0, **FORCES)
