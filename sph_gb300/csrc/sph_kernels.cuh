@@ -73,7 +73,8 @@ __device__ __forceinline__ unsigned gtid() { return blockIdx.x * blockDim.x + th
 // descending, error passes and list builds ascending), so that a pass starts
 // on the lists the pass before it read last and finds them in L2 (129 MB).
 // us/step: 250,000 particles DFSPH (106 MB of pair records) 463 -> 452, 490k
-// PCISPH drop 1017 -> 1006, mix of 256 scenes (1.7 GB) 4560 -> 4522.
+// PCISPH drop 1017 -> 1006; the mix of 256 scenes (1.7 GB) gains less than its
+// runs differ.
 __device__ __forceinline__ unsigned gtid_back() { return (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; }
 
 template <int G, typename T> __device__ __forceinline__ T group_sum(T v)
@@ -585,28 +586,29 @@ __global__ void k_boundary_psi(Boundary<R> b, GridView g, const uint32_t* __rest
 }
 
 // ---------------------------------------------------------------------------
-// PCISPH / WCSPH candidate lists.  The reference's
+// Candidate lists (PCISPH, WCSPH, DFSPH's non-pressure forces).  The reference's
 // PCISPH and WCSPH sums run over the particles of the 27 cells found at the
 // start of the step (HashTable::neighborhoodSearch, HashTable.h:136-170), at
 // the current positions (densities, normals, non-pressure forces, pressure
 // accelerations, WCSPH's pressure force) or the predicted ones (PCISPH's
-// predicted densities).  The density pass records, once per step, every
-// fluid candidate of the 27 cells whose current distance is within
-// REACH = h + margin, in the walk's order, with its cell offset; the later
-// passes visit the list instead of the cells.
+// predicted densities).  The density pass (DFSPH: the list build) records,
+// once per step, every fluid and boundary candidate of the 27 cells whose
+// current distance is within h + margin, in the walk's order, with its cell
+// offset; the later passes visit the list instead of the cells.
 // A candidate left out lies beyond h at the current positions, and beyond h
 // at the predicted ones while every predicted displacement stays below
 // margin / 2 (checked per loop iteration; otherwise the predicted-density
 // pass walks the cells): its terms are the ones the walks skip, so the sums
 // are the same, bit for bit.  A list that does not fit its slots is walked.
+//
+// With G lanes per particle each lane has a list of its own.  DFSPH, and
+// PCISPH in FP32: the candidates its share of the cell walk visits (every G-th
+// of a cell's run, in FP64 of a column's), in that order, so its partial sums,
+// and the result, are the walk's bit for bit.  WCSPH, and PCISPH in FP64: the
+// particle's candidates dealt in turn, the same sums re-associated.
+// Layout: idx[(t * n + i) * G + lane], counts [i * G + lane].
 constexpr uint32_t kCandIdxBits = 27;
 constexpr uint32_t kCandIdxMask = (1u << kCandIdxBits) - 1u;
-
-//
-// With G lanes per particle each lane has a list of its own: the candidates
-// its share of the cell walk visits (every G-th of a cell's run), in that
-// order.  So its partial sums, and the result, are the walk's bit for bit.
-// Layout: idx[(t * n + i) * G + lane], counts [i * G + lane].
 struct CandLists {
     const uint32_t* idx = nullptr;   // j | (cell offset code << 27), the fluid candidates and then the boundary's;
                                      // nullptr: no lists

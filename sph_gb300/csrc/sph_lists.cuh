@@ -65,6 +65,22 @@ __device__ __forceinline__ uint32_t cell_code(uint32_t ci, uint32_t cj)
     return (uint32_t)((cell_x(cj) - cell_x(ci) + 1) * 9 + (cell_y(cj) - cell_y(ci) + 1) * 3 + (cell_z(cj) - cell_z(ci) + 1));
 }
 
+enum Rank { kNoRank, kCellRank, kColumnRank };
+
+__device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+
+// The scaled quantities of the half-precision test of one particle.
+struct HalfTest {
+    float x, y, h;  // position in its cell's frame, support radius
+    __half2 zq, h3, thr;
+};
+__device__ __forceinline__ HalfTest half_test(V3<float> xi, int cz, float h, float reach2)
+{
+    const float sc = half_scale(h);
+    return HalfTest{xi.x * sc, xi.y * sc, h * sc, __float2half2_rn(zframe3(xi.z, cz, h) * sc), __float2half2_rn(3.f * h * sc),
+                    __float2half2_rn(reach2 * 1.03f * (sc * sc))};
+}
+
 // Phase 1 of the list build from the half-precision positions: the
 // nine columns of the 27-cell neighbourhood (trimmed as walk() trims them),
 // two candidates per half2 operation, accepted indices queued in walk order.
@@ -97,22 +113,6 @@ __device__ __forceinline__ uint32_t cell_code(uint32_t ci, uint32_t cj)
 // RANK: each queued candidate with the lane whose part of a cell walk by
 // `lanes` lanes it is, above the index's 27 bits: its rank modulo the lanes
 // in its cell (kCellRank, the FP32 walk) or in its column (kColumnRank, FP64).
-enum Rank { kNoRank, kCellRank, kColumnRank };
-
-__device__ __forceinline__ __half2 as_half2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
-
-// The scaled quantities of the half-precision test of one particle.
-struct HalfTest {
-    float x, y, h;  // position in its cell's frame, support radius
-    __half2 zq, h3, thr;
-};
-__device__ __forceinline__ HalfTest half_test(V3<float> xi, int cz, float h, float reach2)
-{
-    const float sc = half_scale(h);
-    return HalfTest{xi.x * sc, xi.y * sc, h * sc, __float2half2_rn(zframe3(xi.z, cz, h) * sc), __float2half2_rn(3.f * h * sc),
-                    __float2half2_rn(reach2 * 1.03f * (sc * sc))};
-}
-
 template <Rank RANK = kNoRank>
 __device__ __forceinline__ uint32_t cull_half(const GridView& g, const uint32_t* __restrict__ starts, uint32_t pc,
                                               V3<float> xi, float h, float reach2, const uint4* __restrict__ posh,

@@ -1894,7 +1894,7 @@ private:
     DevBuf<unsigned long long> lstat_;
     bool lists_ = false;
     uint32_t kmax_ = 0;
-    bool cands_ = false;            // PCISPH candidate lists (CandLists)
+    bool cands_ = false;            // candidate lists (CandLists)
     uint32_t cslots_ = 0;           // list slots per lane
     DevBuf<uint32_t> cand_, candn_, candb_;
     CandLists CL() const
