@@ -408,7 +408,7 @@ typedef struct sph_pool_tuning {
     int build_occupancy;  /* the register budget allows: (128, 896), (128, 1024), (256, 768), (256, 1024) */
     int queue_depth;      /* candidates staged per particle in shared memory by the build: 8..64, multiple of 8 */
     int solver_block;     /* solver passes: threads per block (128 or 256) and threads per SM */
-    int solver_occupancy; /* the register budget allows (1024, 1536 or 2048; the corrections use one) */
+    int solver_occupancy; /* the register budget allows (1024, 1536 or 2048; from 1.2 M particles the corrections use 1024) */
     int scan_width;       /* grid keys per thread of the cell-count scan (sort width): 4, 8 or 16 */
     int source;           /* 0 defaults or set by the caller, 1 tuning cache, 2 measured */
     int steps_left;       /* tuning steps still to run (read only) */

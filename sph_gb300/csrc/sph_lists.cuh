@@ -1088,7 +1088,8 @@ __device__ __forceinline__ void stream_pairs(const Ring<float>& ring, const P4<f
 
 // DFSPH velocity corrections (MODE 0 warm start, 1 density, 2 divergence),
 // as k_dfsph_correct but over the pair lists; kbuf holds this pass's k.
-template <typename R, int MODE>
+// RING: through the ring (FP32), or loaded into registers.
+template <typename R, int MODE, bool RING = sizeof(R) == 4>
 __device__ __forceinline__ V3<R> correct_sum_one(uint32_t i, const Fluid<R>& f, const P4<R>* __restrict__ bpos,
                                                  const GridView& g, const uint32_t* __restrict__ cs,
                                                  const uint32_t* __restrict__ bs, const Consts<R>& c, int akinci,
@@ -1101,7 +1102,7 @@ __device__ __forceinline__ V3<R> correct_sum_one(uint32_t i, const Fluid<R>& f, 
     V3<R> sum = {0, 0, 0};
     if (cnt <= L.kmax) {
         const P4<R>* __restrict__ p = L.pairs + i;
-        if constexpr (sizeof(R) == 4) {
+        if constexpr (RING) {
             stream_pairs(ring, p, n, cnt, n, L.fault, [&](uint32_t j) { return __ldg(kb_ + j); },
                          [&](V3<R> g, R kj) {
                              const R kSum = ki + kj;

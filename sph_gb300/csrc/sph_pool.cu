@@ -468,20 +468,20 @@ __global__ void k_pool_predict_v_warm(Fluid<float> f, const uint32_t* __restrict
     f.kappa[i] = 0.f;
 }
 
-template <int BLOCK, int MINB, int MODE>
+template <int BLOCK, int MINB, int MODE, bool RING>
 __global__ void __launch_bounds__(BLOCK, MINB) k_pool_correct(Fluid<float> f, const P4<float>* __restrict__ bpos,
                                                             const uint32_t* __restrict__ sid, const PoolScene* T,
                                                             const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                             Lists<float> L)
 {
     grid_wait();
-    __shared__ float4 slots[kRingDepth * BLOCK];
+    __shared__ float4 slots[RING ? kRingDepth * BLOCK : 1];
     const uint32_t i = gtid_back();
     if (i >= f.n) return;
     const PoolScene& sd = T[sid[i]];
     if (!sd.running || (MODE != 0 && !sd.loop_active)) return;
-    const V3<float> sum = correct_sum_one<float, MODE>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c,
-                                                       sd.akinci, L, make_ring<float>(slots, BLOCK));
+    const V3<float> sum = correct_sum_one<float, MODE, RING>(i, f, bpos, sd.g, cs + sd.key_base, bs + sd.key_base, sd.c,
+                                                             sd.akinci, L, make_ring<float>(slots, BLOCK));
     correct_apply<float, MODE>(i, f, sd.c, (float)sd.s.dt, sum);
 }
 
@@ -1502,15 +1502,31 @@ private:
         else SPH_BUILD(256, 3);
 #undef SPH_BUILD
     }
-    // (the corrections hold 8 ring slots a thread in shared memory and need
-    // their 64 registers: below that they spill, so 1536 and 2048 threads per
-    // SM select the same kernel)
+    // From kRingParticles on the corrections stream their records through the
+    // ring of sph_lists.cuh, which needs 64 registers (1536 and 2048 threads
+    // per SM then select the same kernel, below that it spills).  Smaller
+    // layouts load them into registers at the occupancy tuned.  us/step at the
+    // best of five shapes, ring / registers: 231,000 particles 352 / 338,
+    // 294,000 403 / 392, 754,000 906 / 877, 922,000 1047 / 1038, 1.53 M 1682 /
+    // 1694, 2.1 M 2258 / 2289, 4.15 M 4221 / 4265.  The same bits either way.
+    static constexpr uint32_t kRingParticles = 1200000u;
     template <int MODE> void launch_correct(Fluid<float> f, const P4<float>* bp, Lists<float> L)
     {
-#define SPH_CORR(BL, MB) \
-    launch(k_pool_correct<BL, MB, MODE>, blocks(N_, BL), BL, 0, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
-        if (tune_.solver_block == 128) SPH_CORR(128, 8);
-        else SPH_CORR(256, 4);
+        const int sb = tune_.solver_block, so = tune_.solver_occ;
+#define SPH_CORR(BL, MB, RING) \
+    launch(k_pool_correct<BL, MB, MODE, RING>, blocks(N_, BL), BL, 0, f, bp, sid_.p, table_.p, starts_.p, bstarts_.p, L)
+        if (N_ >= kRingParticles) {
+            if (sb == 128) SPH_CORR(128, 8, true);
+            else SPH_CORR(256, 4, true);
+        } else if (sb == 128) {
+            if (so == 1536) SPH_CORR(128, 12, false);
+            else if (so == 2048) SPH_CORR(128, 16, false);
+            else SPH_CORR(128, 8, false);
+        } else {
+            if (so == 1536) SPH_CORR(256, 6, false);
+            else if (so == 2048) SPH_CORR(256, 8, false);
+            else SPH_CORR(256, 4, false);
+        }
 #undef SPH_CORR
     }
     template <bool DIV, bool INITIAL> void launch_errors(Fluid<float> f, const P4<float>* bp, Lists<float> L)
