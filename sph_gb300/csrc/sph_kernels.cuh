@@ -843,9 +843,14 @@ template <typename R> struct BoundaryLoad {
     R dp;
 };
 
+// Resident blocks per SM asked for (0: the compiler's choice) by the pressure
+// passes: the unrolled FP32 walks of one lane otherwise take 93 registers
+// (200,000 PCISPH particles without lists: 153 us a pass against 123).
+template <typename R, int G, bool LISTS> constexpr int kWalkBlocks = sizeof(R) == 4 && G == 1 && !LISTS ? 7 : 0;
+
 // WCSPHSolver::computePressureForce WCSPHSolver.cpp:132-188 (xk.w = p/rho^2)
 template <typename R, int G, bool LISTS>
-__global__ void __launch_bounds__(kBlock) k_wcsph_pressure_force(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
+__global__ void __launch_bounds__(kBlock, kWalkBlocks<R, G, LISTS>) k_wcsph_pressure_force(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                  const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                  Consts<R> c, int akinci, const R* __restrict__ bdp,
                                                                  CandLists L)
@@ -1573,7 +1578,7 @@ __global__ void __launch_bounds__(kBlock) k_pcisph_density_pressure(Fluid<R> f, 
 // PCISPHSolver::computePressureAcc PCISPHSolver.cpp:297-358 (Spiky gradient,
 // current positions; xk.w = p/rho^2)
 template <typename R, int G, bool LISTS>
-__global__ void __launch_bounds__(kBlock) k_pcisph_pressure_acc(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
+__global__ void __launch_bounds__(kBlock, kWalkBlocks<R, G, LISTS>) k_pcisph_pressure_acc(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                 const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                 Consts<R> c, int akinci, const DevScalars* __restrict__ sc,
                                                                 const R* __restrict__ bdp, CandLists L)
