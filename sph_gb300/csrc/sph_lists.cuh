@@ -1250,8 +1250,8 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_predict_density_list(Fluid<
 }
 
 // DFSPHSolver::computeDivergenceError over the lists (+ loop control); the
-// step's first one is formed by the list build.
-template <typename R>
+// step's first one (INITIAL) is formed by the list build unless lists are short.
+template <typename R, bool INITIAL>
 __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,
                                                                   const uint32_t* __restrict__ cs, const uint32_t* __restrict__ bs,
                                                                   Consts<R> c, int akinci, DevScalars* sc, LoopLimits lim,
@@ -1261,7 +1261,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f,
     grid_wait();
     __shared__ float4 slots[sizeof(R) == 4 ? kRingDepth * kBlock : 1];
     __shared__ double sh[33];
-    if (!sc->active) return;
+    if (!INITIAL && !sc->active) return;
     const uint32_t i = gtid();
     double err = 0.0;
     if (i < f.count()) {
@@ -1272,7 +1272,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_dfsph_divergence_list(Fluid<R> f,
     }
     double total;
     if (finish_reduction<false>(err, partials, &sc->block_counter, sh, &total) && threadIdx.x == 0)
-        divergence_control<false>(sc, lim, total, f.count(), cond);
+        divergence_control<INITIAL>(sc, lim, total, f.count(), cond);
 }
 
 // The stored lists of the n particles at [base, base + n) of a layout whose

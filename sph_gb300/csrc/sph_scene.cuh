@@ -1043,9 +1043,16 @@ private:
         // DFSPH in a cube: its clamp moves particles after the grid build whose
         // candidates (and half-precision positions) the next step's forces
         // would visit, so those walk the cells.
-        const bool want = d.neighbor_list_max > 0 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask &&
-                          (d.simulation_method != SPH_DFSPH ||
-                           (c_.force_flags != 0 && !c_.has_cube && (G_ > 1 || build_lanes() == 1)));
+        bool want = d.neighbor_list_max > 0 && !bh_ && std::max(n, nb) < (size_t)kCandIdxMask;
+        // PCISPH with several lanes per particle, from the length on at which
+        // most lists fit.  us/step, lists / walks: FP32 (whose lanes' shares are
+        // uneven), 8,000 particles with all forces and 30,000 without: 28 slots
+        // 298 / 263, 313 / 290; 34: 288 / 264, 302 / 291; 40: 270 / 264, 259 /
+        // 292; 64: 149 / 265, 254 / 292.  FP64, 1,000 particles: 16 slots 424 /
+        // 408; 24: 295 / 408; 64: 201 / 407.
+        if (d.simulation_method == SPH_PCISPH) want &= G_ == 1 || d.neighbor_list_max >= (sizeof(R) == 8 ? 24 : 40);
+        if (d.simulation_method == SPH_DFSPH)
+            want &= lists_hold() && c_.force_flags != 0 && !c_.has_cube && (G_ > 1 || build_lanes() == 1);
         // half-precision positions for the list builds' culls (pairs of
         // points, the last one whole, and a spare word for the cull), the
         // fluid's written by every gather, the boundary's once per grid box
@@ -1175,6 +1182,15 @@ private:
         return SPH_OK;
     }
 
+    // DFSPH lists long enough for most particles (a particle at rest has about
+    // 33 neighbours).  Shorter ones overflow nearly everywhere and their
+    // particles walk the cells in every pass: one lane per particle builds them,
+    // without the first error pass, and the forces take the walk.  us/step with
+    // 28 slots, as long lists are built / so: 8,000 particles FP64 5,935 / 5,152,
+    // 80,000 FP32 1,179 / 1,166, with XSPH 1,325 / 1,262 (1,000 FP64 4,400 /
+    // 4,960: left); with 34, 1,595 / 1,758, 361 / 367, 422 / 468.
+    bool lists_hold() const { return d.neighbor_list_max >= 32; }
+
     // Lanes per particle of the list build (results do not depend on it).
     // Several lanes shorten the chain of dependent loads but execute two to
     // three times the instructions, so they pay while their blocks are all
@@ -1186,6 +1202,7 @@ private:
     // 140 / 161; 30,000 309 / 304 / 316.
     int build_lanes() const
     {
+        if (!lists_hold()) return 1;
         if ((size_t)n_ <= (size_t)sms_ * 4 * (kWideBlock / 8)) return 8;
         if ((size_t)n_ <= (size_t)sms_ * 5 * (kWideBlock / 4)) return 4;
         return 1;
@@ -1399,17 +1416,20 @@ private:
                     {
                         // computeDensities + computeAlpha + pair lists + the first divergence error
                         auto ph = phase("Neigh search+Densities+Alpha factor");
-                        const int brc = launch_build_lists<true>(h);
+                        const int brc = lists_hold() ? launch_build_lists<true>(h) : launch_build_lists();
                         if (brc) return brc;
                         launch_bh_boundary(0);
                     }
                     // correctDivergenceError DFSPHSolver.cpp:494-590
                     solver.emplace(phases_, "Divergence solver", ls_, capturing_, prof_);
+                    if (!lists_hold())
+                        run("k_dfsph_divergence_list", [&] { launch(k_dfsph_divergence_list<R, true>, nb, kBlock, 0,
+                            f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
                     return launched();
                 },
                 [&](cudaGraphConditionalHandle h) {
                     run("k_dfsph_correct_list", [&] { launch(k_dfsph_correct_list<R, 2>, nb, kBlock, 0, f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, L); });
-                    run("k_dfsph_divergence_list", [&] { launch(k_dfsph_divergence_list<R>, nb, kBlock, 0, 
+                    run("k_dfsph_divergence_list", [&] { launch(k_dfsph_divergence_list<R, false>, nb, kBlock, 0, 
                         f, bp, gv_, starts_.p, bstarts_.p, c_, hasb_, sc_.p, lim_, partials_.p, h, L); });
                 },
                 lim_.minItV, lim_.maxIt);

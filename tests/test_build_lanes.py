@@ -12,7 +12,7 @@ R = 0.01
 
 
 @pytest.mark.parametrize("precision,per_sm", [("f32", 4 * 16), ("f32", 5 * 32), ("f64", 4 * 16), ("f64", 5 * 32), ("f64", 6 * 128), ("f64", 8 * 128)])
-@pytest.mark.parametrize("lists", [64, 24])
+@pytest.mark.parametrize("lists", [64, 33, 24])
 def test_lanes_give_the_same_bits(gpu_lib, precision, lists, per_sm):
     torch = pytest.importorskip("torch")
     n = torch.cuda.get_device_properties(0).multi_processor_count * per_sm
