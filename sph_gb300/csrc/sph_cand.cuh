@@ -296,7 +296,7 @@ __device__ __forceinline__ float divisor_of(float b) { return b; }
 // WCSPH with XSPH viscosity (or none of the force plugins' other kinds):
 // pressure force (k_wcsph_pressure_force) and viscosity (k_npforce) from one
 // visit of the candidates, each sum in its own order; the distance and its
-// root are formed once.  us/step: 8,000 particles in FP64 202 -> 149, 90,000
+// root are formed once.  us/step: 8,000 particles in FP64 202 -> 148, 90,000
 // with Akinci walls 103 -> 91.
 template <typename R> struct WcsphFluid { V3<R> p, av; };
 template <typename R> struct WcsphBoundary { V3<R> p, avb; };

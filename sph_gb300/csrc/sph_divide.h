@@ -31,33 +31,32 @@ SPH_HD uint64_t bits_of(double v)
     return u;
 #endif
 }
-// |v| between 2^-900 and 2^900 (exponent fields 123 and 1923)
-SPH_HD bool mid_range(uint64_t u) { return ((uint32_t)(u >> 52) & 0x7ffu) - 123u < 1800u; }
-
-// Quotients x / b of many values by one, correctly rounded: x rb (rb = 1 / b
-// rounded) and two residual corrections, of which the first brings it within
-// one unit in the last place and the second rounds it as the division does
+// Quotients x / b of many values by one, correctly rounded: the product of x
+// with 1 / b in two parts, which is within one unit in the last place of the
+// quotient, and one residual correction, which rounds it as the division does
 // (Markstein, IBM J. Res. Dev. 34, 1990, on the final rounding of a quotient):
-// 5 FP64 operations instead of about 9, of which an SM has two lanes.  That
+// 4 FP64 operations instead of about 9, of which an SM has two lanes.  That
 // needs exact residuals and normal numbers: true where *q is the quotient,
-// false where the caller has to divide (operands or quotients outside 2^-900
-// to 2^900, infinities, NaN).
+// false where the caller has to divide (|b| outside 2^-100 to 2^100; |x|
+// outside 2^-800 to 2^800 but zero).
 struct Divisor {
-    double b, rb;
+    double b, hi, lo;  // 1 / b rounded, and what that left out
+    bool ok;
 };
 SPH_HD Divisor divisor(double b)
 {
-    // (a NaN for rb makes every quotient the caller's)
-    return Divisor{b, mid_range(bits_of(b)) ? 1.0 / b : std::nan("")};
+    const bool ok = ((uint32_t)(bits_of(b) >> 52) & 0x7ffu) - 923u < 200u;
+    const double hi = 1.0 / b;
+    return Divisor{b, hi, fma_rn(-hi, b, 1.0) * hi, ok};
 }
 SPH_HD bool quotient(double x, const Divisor& d, double* q)
 {
-    const double q0 = x * d.rb;
-    const double q1 = fma_rn(fma_rn(-q0, d.b, x), d.rb, q0);
-    const double q2 = fma_rn(fma_rn(-q1, d.b, x), d.rb, q1);
-    const bool zero = (bits_of(x) << 1) == 0;  // x rb has its sign
-    *q = zero ? q0 : q2;
-    return zero ? d.rb == d.rb : (mid_range(bits_of(x)) && mid_range(bits_of(q2)));
+    const double q0 = fma_rn(x, d.hi, x * d.lo);
+    const double q1 = fma_rn(fma_rn(-q0, d.b, x), d.hi, q0);
+    *q = q1;
+    // a zero (of either sign) gives a zero
+    const uint64_t u = bits_of(x);
+    return d.ok && (((uint32_t)(u >> 52) & 0x7ffu) - 223u < 1600u || (u << 1) == 0);
 }
 
 }  // namespace sph
