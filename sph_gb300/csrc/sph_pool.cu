@@ -1747,6 +1747,7 @@ private:
         // boundary: sort by (key, id) -- kept scenes are already in order -- and volumes
         if (NB_) {
             k_pool_bcount<<<blocks(NB_, 256), 256, 0, st_>>>(NB_, B(bcur_), bsid_.p, table_.p, key_.p, slot_.p, count_.p);
+            chained_ = false;
             int rc = scan(bstarts_.p);
             if (rc) return rc;
             k_scatter<<<blocks(NB_, 256), 256, 0, st_>>>(NB_, key_.p, slot_.p, bstarts_.p, tmp_.p);
@@ -1762,6 +1763,7 @@ private:
         }
         // fluid grid and lists (DFSPHSolver::init for new scenes; identical
         // recomputation for the kept ones, whose positions have not moved)
+        chained_ = false;
         int rc = build_grid(false);
         if (rc) return rc;
         run("k_pool_build_lists", [&] { launch_build(F(cur_), bpos_[bcur_].p, LS()); });

@@ -367,6 +367,7 @@ public:
             }
             k_cell_count<<<blocks(nb_, 256), 256, 0, st_>>>(nb_, B(0).cell, key_.p, slot_.p, count_.p, gv_);
             if (bh_) k_bh_mark_cells<<<blocks(nb_, 256), 256, 0, st_>>>(nb_, key_.p, cell_epoch_.p);
+            chained_ = false;
             rc = scan(bstarts_.p);
             if (rc) return rc;
             k_scatter<<<blocks(nb_, 256), 256, 0, st_>>>(nb_, key_.p, slot_.p, bstarts_.p, tmp_.p);
@@ -380,6 +381,7 @@ public:
         }
         rc = allocate_optional();
         if (rc) return rc;
+        chained_ = false;
         rc = build_grid(false);
         if (rc) return rc;
         if (d.simulation_method == SPH_DFSPH) {
@@ -493,6 +495,7 @@ public:
                                                                               slot_.p, count_.p, gv_, c_.h, hd_, sc_.p);
             k_cell_count<<<blocks(nb_, 256), 256, 0, st_>>>(nb_, B(1).cell, key_.p, slot_.p, count_.p, gv_);
             SPH_CUDA(cudaGetLastError());
+            chained_ = false;
             rc = scan(bstarts_.p);
             if (rc) return rc;
             k_scatter<<<blocks(nb_, 256), 256, 0, st_>>>(nb_, key_.p, slot_.p, bstarts_.p, tmp_.p);
@@ -505,6 +508,7 @@ public:
             SPH_CUDA(cudaMemsetAsync(bstarts_.p, 0, (nkeys_ + 1) * sizeof(uint32_t), st_));
         }
         SPH_CUDA(cudaMemsetAsync(&sc_.p->escaped, 0, sizeof(unsigned), st_));
+        chained_ = false;
         rc = build_grid(false);
         if (rc) return rc;
         if (d.simulation_method == SPH_DFSPH) {
