@@ -141,9 +141,9 @@ __global__ void __launch_bounds__(kBlock, 7) k_density_cand(Fluid<R> f, const P4
 // The same with W lanes per particle (small scenes), each lane with a list and
 // a partial density of its own.  The lanes share the cull into a common queue.
 // EVEN: the listed candidates are dealt to the lanes in turn (a particle's
-// lists are then all stored or all walked).  Otherwise each takes the candidates of its part
-// of the cell walk (CandLists), so that the FP32 solvers' sums stay the walk's
-// bit for bit: DFSPH's and PCISPH's solves amplify rounding (a change of 1e-7
+// lists are then all stored or all walked).  Otherwise each takes the
+// candidates of its part of the cell walk (CandLists), so that the solvers'
+// sums stay the walk's bit for bit: DFSPH's and PCISPH's solves amplify rounding (a change of 1e-7
 // in the velocities grows to 1e-5 in five steps), WCSPH's and FP64's do not
 // need it, and the lanes' shares are uneven (8,000 WCSPH particles: 36 against
 // 41 us/step, FP64 189 against 279).

@@ -1200,10 +1200,11 @@ private:
     // three times the instructions, so they pay while their blocks are all
     // resident at once: 8 lanes at 4 blocks of 16 particles per SM, 4 lanes at
     // 5 blocks of 32 (in FP64 its shared memory lets 3 reside).  Build in us
-    // (1 / 4 / 8 lanes, FP32, with the ~5 us of an event pair): 2,000 particles 42.6 / 22.3 / 18.4; 8,000 45.2 / 24.5 / 21.8;
-    // 13,000 44.3 / 26.5 / 30.4; 24,000 46.0 / 35.7 / 39.4; 30,000 47.7 / 49.8 /
-    // 46.6; 40,000 50.1 / 53.6 / 59.2.  FP64: 2,000 177 / 63 / 43; 13,000 195 /
-    // 140 / 161; 30,000 309 / 304 / 316.
+    // (1 / 4 / 8 lanes, FP32, with the ~5 us of an event pair): 2,000 particles
+    // 42.6 / 22.3 / 18.4; 8,000 45.2 / 24.5 / 21.8; 13,000 44.3 / 26.5 / 30.4;
+    // 24,000 46.0 / 35.7 / 39.4; 30,000 47.7 / 49.8 / 46.6; 40,000 50.1 / 53.6 /
+    // 59.2.  FP64: 2,000 177 / 63 / 43; 13,000 195 / 140 / 161; 30,000 309 / 304 /
+    // 316.
     int build_lanes() const
     {
         if (!lists_hold()) return 1;
@@ -1479,10 +1480,9 @@ private:
             // FP32 over lists: each set of plugins compiled apart (fewer
             // registers, no tests of the flags in the loop).  85,000 DFSPH
             // particles, k_npforce in us, compiled apart / one form: XSPH 43.9 /
-            // 52.8, standard viscosity 40.0 / 48.3, artificial 40.6 /
-            // 49.7, adhesion 15.2 / 17.4, XSPH with surface tension and adhesion
-            // 57.8 / 66.9.
-            // FP64, bound by its arithmetic: within 2 %, one form.
+            // 52.8, standard viscosity 40.0 / 48.3, artificial 40.6 / 49.7,
+            // adhesion 15.2 / 17.4, XSPH with surface tension and adhesion 57.8 /
+            // 66.9.  FP64, bound by its arithmetic: within 2 %, one form.
             if constexpr (LISTS && sizeof(R) == 4) by_force_set(go);
             else go(std::integral_constant<int, kAnyForces>{});
         });
@@ -1511,9 +1511,9 @@ private:
 
     // A solver loop: init(h) launches the kernel that sets the first loop
     // test and returns its error code, body(h) one iteration whose last kernel
-    // sets the next.  Host mode
-    // reads the flag back every few iterations (finished-loop kernels exit at
-    // once); capture mode makes it a conditional WHILE node.
+    // sets the next.  Host mode reads the flag back every few iterations
+    // (finished-loop kernels exit at once); capture mode makes it a conditional
+    // WHILE node.
     template <typename Init, typename Body> int solve_loop(int loop_id, Init&& init, Body&& body, unsigned minIt, unsigned maxIt)
     {
         if (capturing_) {
@@ -1710,7 +1710,9 @@ private:
         const P4<R>* bp = bd_[1].pos;
         const R* dp = bdp();
         if (cands_ && (c_.force_flags & ~F_BVISC) == F_XSPH) {
-            // both forces from one visit (the host-driven step's timers name them together)
+            // Both forces from one visit, for XSPH alone, the viscosity of the
+            // WCSPH configurations here (k_wcsph_forces has the times); other sets
+            // of plugins take two.  The timers name the phases together.
             auto ph = phase("Pressure force+NPForces");
             withG([&](auto gt) {
                 constexpr int G = decltype(gt)::value;
