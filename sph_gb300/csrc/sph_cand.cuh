@@ -143,10 +143,10 @@ __global__ void __launch_bounds__(kBlock, 7) k_density_cand(Fluid<R> f, const P4
 // EVEN: the listed candidates are dealt to the lanes in turn (a particle's
 // lists are then all stored or all walked).  Otherwise each takes the
 // candidates of its part of the cell walk (CandLists), so that the solvers'
-// sums stay the walk's bit for bit: DFSPH's and PCISPH's solves amplify rounding (a change of 1e-7
-// in the velocities grows to 1e-5 in five steps), WCSPH's and FP64's do not
-// need it, and the lanes' shares are uneven (8,000 WCSPH particles: 36 against
-// 41 us/step, FP64 189 against 279).
+// sums stay the walk's bit for bit: DFSPH's and PCISPH's solves amplify
+// rounding (a change of 1e-7 in the velocities grows to 1e-5 in five steps);
+// WCSPH's, and PCISPH's in FP64, do not need it, and the lanes' shares are
+// uneven (8,000 WCSPH particles: 36 against 41 us/step, FP64 189 against 279).
 // DENS = false: the lists alone (DFSPH's non-pressure forces).
 template <typename R, int W, bool EOS, bool EVEN, bool DENS = true>
 __global__ void __launch_bounds__(kWideBlock) k_density_cand_wide(Fluid<R> f, const P4<R>* __restrict__ bpos, GridView g,

@@ -234,6 +234,11 @@ template <typename T> struct DevBuf {
         p = nullptr;
         n = 0;
     }
+    void swap(DevBuf& o)
+    {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+    }
     // n counts what p holds: 0 after a failure, so that a buffer kept between
     // calls is allocated again by the next one (and the error is taken off the
     // thread's last one, which the next launch check would report).
@@ -439,7 +444,8 @@ public:
     // re-sorted and the DFSPH densities, alpha factors and lists rebuilt at
     // the same positions (same values: sums run in the geometric walk order,
     // which the box does not change), and the step graphs are re-captured.
-    // A box beyond the cell packing's limits stays as it is, and growth stops.
+    // A box beyond the cell packing's limits, or one that there is no memory
+    // for, stays as it is, and growth stops.
     int grow_grid()
     {
         SPH_CUDA(cudaStreamSynchronize(st_));
@@ -477,10 +483,24 @@ public:
             gsteps_[k] = 0;
             for (int q = 0; q < 3; ++q) gshape_[k][q] = 0;
         }
-        rc = use_grid(p);
-        if (rc) return rc;
-        SPH_CUDA(count_.alloc(nkeys_)); SPH_CUDA(starts_.alloc(nkeys_ + 1)); SPH_CUDA(bstarts_.alloc(nkeys_ + 1));
-        SPH_CUDA(tile_sums_.alloc(blocks(nkeys_, kScanTile)));
+        // the new box's memory before anything of the old one goes (without the
+        // candidate lists, if that is what it takes): where there is none, the
+        // box stays as it is
+        DevBuf<uint32_t> count, starts, bstarts, tiles;
+        auto take = [&] {
+            return count.alloc(p.nkeys) == cudaSuccess && starts.alloc(p.nkeys + 1) == cudaSuccess &&
+                   bstarts.alloc(p.nkeys + 1) == cudaSuccess && tiles.alloc(blocks(p.nkeys, kScanTile)) == cudaSuccess;
+        };
+        bool room = take();
+        if (!room && cands_) {
+            drop_candidates();
+            room = take();
+        }
+        if (!room || use_grid(p) != SPH_OK) {
+            grow_ = false;
+            return SPH_OK;
+        }
+        count_.swap(count); starts_.swap(starts); bstarts_.swap(bstarts); tile_sums_.swap(tiles);
         SPH_CUDA(cudaMemsetAsync(count_.p, 0, nkeys_ * sizeof(uint32_t), st_));
         Fluid<R> f = F();
         k_shift_cells<<<blocks(n_, 256), 256, 0, st_>>>(n_, f.na, f.cell, sx, sy, sz);
@@ -952,11 +972,14 @@ private:
     // Installs a planned box: key count, Morton tables, the grid view.
     int use_grid(const GridPlan& p)
     {
+        DevBuf<uint32_t> mx, my;
+        SPH_CUDA(mx.alloc(p.nn[0]));
+        SPH_CUDA(my.alloc(p.nn[1]));
+        SPH_CUDA(cudaMemcpy(mx.p, p.mx.data(), p.nn[0] * 4, cudaMemcpyHostToDevice));
+        SPH_CUDA(cudaMemcpy(my.p, p.my.data(), p.nn[1] * 4, cudaMemcpyHostToDevice));
+        mortx_.swap(mx);
+        morty_.swap(my);
         nkeys_ = (uint32_t)p.nkeys;
-        SPH_CUDA(mortx_.alloc(p.nn[0]));
-        SPH_CUDA(morty_.alloc(p.nn[1]));
-        SPH_CUDA(cudaMemcpy(mortx_.p, p.mx.data(), p.nn[0] * 4, cudaMemcpyHostToDevice));
-        SPH_CUDA(cudaMemcpy(morty_.p, p.my.data(), p.nn[1] * 4, cudaMemcpyHostToDevice));
         gv_.nx = p.nn[0]; gv_.ny = p.nn[1]; gv_.nz = p.nn[2];
         gv_.ox = p.o[0]; gv_.oy = p.o[1]; gv_.oz = p.o[2];
         gv_.mortx = mortx_.p;
@@ -1079,11 +1102,17 @@ private:
             SPH_CUDA(cudaMemsetAsync(candn_.p, 0, n * G_ * sizeof(uint32_t), st_));
             SPH_CUDA(cudaMemsetAsync(candb_.p, 0, n * G_ * sizeof(uint32_t), st_));
         } else {
-            cand_.release();
-            candn_.release();
-            candb_.release();
+            drop_candidates();
         }
         return SPH_OK;
+    }
+    // (no graph of a step may hold them)
+    void drop_candidates()
+    {
+        cands_ = false;
+        cand_.release();
+        candn_.release();
+        candb_.release();
     }
 
     // Exclusive scan of count_ into out (nkeys + 1 entries); zeroes count_.

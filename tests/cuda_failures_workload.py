@@ -105,6 +105,30 @@ def allocations(F):
     return out
 
 
+def growth(F):
+    """A particle leaves the grid box; each allocation of the growth that follows fails in turn: [growths, allocations],
+    then per failure [the step reported it, growths, later steps failed]."""
+    def grown(fail):
+        s = scene(**SOLVERS["dfsph_forces"])
+        F.fake_device_word(1)  # the escape flag, when the step polls it
+        out, m = [], 0
+        for k in range(40):
+            m0 = F.fake_mallocs()
+            if fail:
+                F.fake_fail_malloc(fail)
+            out.append(failed(lambda: s.step(1)))
+            F.fake_fail_malloc(0)
+            m = max(m, F.fake_mallocs() - m0)
+            if F.fake_mallocs() > m0:  # it grew, or tried to
+                break
+        F.fake_device_word(0)
+        later = any(failed(lambda: s.step(1)) for _ in range(3)) or failed(lambda: s.get("x"))
+        return [any(out), s.stats()["grid_growths"], later, m]
+
+    first = grown(0)
+    return {"first": first, "each": [grown(k)[:3] for k in range(1, first[3] + 1)], "null_uses": F.fake_null_uses()}
+
+
 if __name__ == "__main__":
     F = fake()
-    print(json.dumps({"downloads": downloads, "launches": launches, "allocations": allocations}[sys.argv[1]](F)))
+    print(json.dumps({"downloads": downloads, "launches": launches, "allocations": allocations, "growth": growth}[sys.argv[1]](F)))

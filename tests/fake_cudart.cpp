@@ -7,7 +7,8 @@
 //   fake_fail_launch(n)   the n-th launch from now on fails (0: none)
 //   fake_fail_malloc(n)   the n-th allocation from now on fails (0: none)
 //   fake_launches() / fake_mallocs()   so far
-//   fake_null_uses()      copies from or to, and downloads into, a null pointer
+//   fake_device_word(v)   4-byte reads of device memory give v (0: what it holds): the flags a step polls
+//   fake_null_uses()      copies from or to, downloads into, and key scans of a null pointer
 //   fake_launched(name)   launches of kernels whose name contains `name`
 #include <cuda_runtime_api.h>
 
@@ -23,6 +24,7 @@ std::map<const void*, std::string>& names()
     return m;
 }
 std::map<std::string, int> launched;
+unsigned device_word = 0;
 int fail_launch = 0, fail_malloc = 0, launches = 0, mallocs = 0, null_uses = 0;
 cudaError_t last = cudaSuccess;
 struct Config {
@@ -38,7 +40,9 @@ cudaError_t launch(const void* f, void** args)
     const std::string& n = names()[f];
     if (fail_launch > 0 && --fail_launch == 0) return fail(cudaErrorLaunchOutOfResources);
     ++launched[n];
-    // k_download(n, v4, s, id, cell, g, h, kind, out)
+    // k_scan_tiles(nkeys, count, starts, tile_sums); k_download(n, v4, s, id, cell, g, h, kind, out)
+    if (n.find("k_scan_tiles") != std::string::npos)
+        for (int k = 1; k < 4; ++k) null_uses += !*(void**)args[k];
     if (n.find("k_download") != std::string::npos && !*(void**)args[8]) ++null_uses;
     return cudaSuccess;
 }
@@ -61,6 +65,7 @@ cudaError_t take(void** p, size_t n)
 extern "C" {
 void fake_fail_launch(int n) { fail_launch = n; }
 void fake_fail_malloc(int n) { fail_malloc = n; }
+void fake_device_word(unsigned v) { device_word = v; }
 int fake_launches() { return launches; }
 int fake_mallocs() { return mallocs; }
 int fake_null_uses() { return null_uses; }
@@ -122,7 +127,11 @@ cudaError_t cudaFreeHost(void* p)
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { return copy(d, s, n); }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { return copy(d, s, n); }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t)
+{
+    if (device_word && n == 4 && kind == cudaMemcpyDeviceToHost && d && s) return copy(d, &device_word, 4);
+    return copy(d, s, n);
+}
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t)
 {
     if (!d) return copy(d, d, n);

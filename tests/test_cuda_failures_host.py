@@ -3,7 +3,8 @@
 
 * A read whose staging buffer cannot be allocated reports it; later reads allocate again and nothing uses a null buffer.
 * A step reports the failure of any of its launches.
-* A scene whose candidate lists (or half-precision positions) find no memory runs without them."""
+* A scene whose candidate lists (or half-precision positions) find no memory runs without them.
+* A grid box that finds no memory to grow stays as it is."""
 import json
 import os
 import subprocess
@@ -54,3 +55,14 @@ def test_scene_without_memory_for_candidate_lists(run):
     for solver, (n, lists, without) in out.items():
         assert lists == (1 if optional[solver] == 5 else 0), solver
         assert without == [[k, 0] for k in range(n - optional[solver] + 1, n + 1)], (solver, n, without)
+
+
+def test_grid_without_memory_to_grow(run):
+    out = run("growth")
+    failed, growths, later, n = out["first"]
+    assert not failed and growths == 1 and not later and n >= 6
+    assert out["null_uses"] == 0
+    # the first is the staging buffer of the positions' download, whose failure the step reports
+    assert out["each"][0] == [True, 0, False]
+    for failed, growths, later in out["each"][1:]:
+        assert not failed and not later and growths in (0, 1)
